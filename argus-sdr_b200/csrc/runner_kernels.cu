@@ -1277,6 +1277,8 @@ k_wfm_fir(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, cons
     }
 }
 
+constexpr int kPllSeg = 16;  // steps per segment of the parallel solver; the float32 angle restarts as often
+
 struct PllK {
     double alpha, beta;
     float lpa;
@@ -1289,48 +1291,99 @@ struct PllK {
 // ramp phase0 + t*freq0 is exact in Q0.64 turns, so the sin/cos argument needs
 // no float64 range reduction.  The I/Q lowpass states are float32.  The serial
 // loop and the Newton solver both use this step, so they iterate the same map.
+//
+// A trajectory is one chain of dependent operations, so a step costs its
+// latency.  The chain runs through float32 only: the angle above the ramp is
+// the float64 phase at the last pll_begin (the start of a 16-step segment),
+// rounded once, plus the advance since then in float32 -- below 1 rad, of an
+// angle that is rounded to float32 anyway -- while the float64 phase and
+// frequency are carried beside it.  (430 cycles a step through atan2f and the
+// float64 state.)
+struct PllRun {
+    double dphi, df;
+    float I, Q;
+    float base, off, adv;  // the next step's angle above the ramp: base + off + adv
+    float dff;             // df in float32
+};
+
 struct PllEval {
-    double dphi1, df1;
-    float I1, Q1;
     float e;
     float ja, jb, jc, jd;   // phase row: d/dphase, d/dfreq, d/dI, d/dQ
     float ka, kb, kc, kd;   // freq row
     float iphi, qphi;       // I/Q rows' d/dphase (diagonals are 1 - lpa)
 };
 
-// q: the ramp phase phase0 + t*freq0 of step t in Q0.64 turns (callers carry
-// it by adding k.qf per step: the same integer as k.q0 + t*k.qf).
-__device__ __forceinline__ void pll_angle(uint64_t q, double dphi, float &s, float &c) {
-    const float h = (float)(int32_t)(q >> 32) * 4.656612873077393e-10f + (float)(dphi * (1.0 / GPUD_PI));
-    __sincosf(h * 3.14159265358979f, &s, &c);  // |angle| <= pi + |dphi|
+// The phase deviation of an unlocked loop grows to hundreds of radians: it is
+// reduced to one turn in float64 before it is rounded, else the rounding of the
+// angle (4e-6 rad at 50 rad) keeps the parallel solver above its tolerance.
+__device__ __forceinline__ PllRun pll_begin(double dphi, double df, float I, float Q) {
+    const double turns = rint(dphi * (1.0 / (2.0 * GPUD_PI)));
+    return PllRun{dphi, df, I, Q, (float)fma(turns, -2.0 * GPUD_PI, dphi), 0.f, 0.f, (float)df};
 }
 
+__device__ __forceinline__ float pll_rcp(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// atan2 in float32 (within 1.8 ulp; atan2f: 2.0): the quotient t of the smaller
+// by the larger magnitude from an approximate reciprocal and one residual
+// correction, then t + t u P(u), u = t^2, P fitted to atan on [0, 1] by
+// reweighted least squares (relative error 1.7e-8) and evaluated as short
+// chains; octant and signs enter as a factor of t and an offset, both ready
+// before the quotient is.  The scaling keeps the reciprocal's argument normal
+// as I and Q die out (and above zero).
+__device__ __forceinline__ float pll_atan2(float y, float x) {
+    const float ax = fabsf(x), ay = fabsf(y);
+    const float hi = fmaf(fmaxf(ax, ay), 1.8446744e19f, 1e-30f), lo = fminf(ax, ay) * 1.8446744e19f;
+    const bool swap = ay > ax, neg = x < 0.f;
+    // angle of (ax, ay): r or pi/2 - r; of (x, ay): that or pi minus it
+    const float sg = copysignf(1.f, y), st = swap != neg ? -sg : sg;
+    const float oh = swap ? 1.57079637f : neg ? 3.14159274f : 0.f;
+    const float ol = swap ? -4.371139e-8f : neg ? -8.742278e-8f : 0.f;
+    const float sh = sg * oh, sl = sg * ol;
+    const float rc = pll_rcp(hi);
+    float t = lo * rc;
+    t = fmaf(fmaf(-hi, t, lo), rc, t);
+    const float u = t * t, u2 = u * u, u4 = u2 * u2;
+    const float p01 = fmaf(u, 0.19993773f, -0.33333153f), p23 = fmaf(u, 0.10666005f, -0.14211056f);
+    const float p45 = fmaf(u, 0.04321186f, -0.07552214f), p67 = fmaf(u, 0.00292069f, -0.01636793f);
+    const float pp = fmaf(u4, fmaf(u2, p67, p45), fmaf(u2, p23, p01));
+    const float ts = t * st;
+    return (fmaf(ts * u, pp, ts) + sl) + sh;
+}
+
+// q: the ramp phase phase0 + t*freq0 of step t in Q0.64 turns (callers carry
+// it by adding k.qf per step: the same integer as k.q0 + t*k.qf); radians.
+__device__ __forceinline__ float pll_ramp(uint64_t q) { return (float)(int32_t)(q >> 32) * 1.46291808e-9f; }
+
 template <bool kJac>
-__device__ __forceinline__ void pll_step(uint64_t q, double dphi, double df, float I, float Q, float p, const PllK &k,
-                                         PllEval &o) {
+__device__ __forceinline__ void pll_step(uint64_t q, PllRun &s, float p, const PllK &k, PllEval &o) {
     float sn, cs;
-    pll_angle(q, dphi, sn, cs);
-    o.I1 = fmaf(k.lpa, fmaf(p, cs, -I), I);
-    o.Q1 = fmaf(k.lpa, fmaf(p, -sn, -Q), Q);
-    const float e = atan2f(o.Q1, o.I1);
+    __sincosf((pll_ramp(q) + s.base + s.off) + s.adv, &sn, &cs);  // |angle| <= pi + |dphi|
+    s.off += s.adv;
+    const float I1 = fmaf(k.lpa, fmaf(p, cs, -s.I), s.I);
+    const float Q1 = fmaf(k.lpa, fmaf(p, -sn, -s.Q), s.Q);
+    const float e = pll_atan2(Q1, I1);
     o.e = e;
-    double d = df + k.beta * (double)e;
-    bool clamped = false;
-    if (d < k.dfmin) {
-        d = k.dfmin;
-        clamped = true;
-    } else if (d > k.dfmax) {
-        d = k.dfmax;
-        clamped = true;
-    }
-    o.df1 = d;
-    o.dphi1 = dphi + d + k.alpha * (double)e;
+    const float df1 = fminf(fmaxf(fmaf((float)k.beta, e, s.dff), (float)k.dfmin), (float)k.dfmax);
+    s.adv = fmaf((float)k.alpha, e, df1);
+    s.dff = df1;
+    const double ed = (double)e;
+    double d = fma(k.beta, ed, s.df);
+    const bool clamped = d < k.dfmin || d > k.dfmax;
+    d = d < k.dfmin ? k.dfmin : (d > k.dfmax ? k.dfmax : d);
+    s.dphi = fma(k.alpha, ed, s.dphi) + d;
+    s.df = d;
+    s.I = I1;
+    s.Q = Q1;
     if (kJac) {
         // the Jacobian sets the convergence rate only, not the fixed point:
         // an approximate reciprocal is enough
-        const float r2 = fmaf(o.I1, o.I1, o.Q1 * o.Q1);
+        const float r2 = fmaf(I1, I1, Q1 * Q1);
         const float inv = r2 > 0.f ? __fdividef(1.f, r2) : 0.f;
-        const float gI = -o.Q1 * inv, gQ = o.I1 * inv;
+        const float gI = -Q1 * inv, gQ = I1 * inv;
         const float dIphi = -k.lpa * p * sn;  // d/dphase of lpa*p*cos(phase)
         const float dQphi = -k.lpa * p * cs;  // d/dphase of -lpa*p*sin(phase)
         const float ePhi = fmaf(gI, dIphi, gQ * dQphi);
@@ -1371,12 +1424,11 @@ __device__ __forceinline__ double pll_phase_at(const PllK &k, int t, double dphi
     return ph;
 }
 
-// 2*sin(2*phase) of the loop phase, float32 (lr = bpf * that); q is the ramp
-// phase of the same step in Q0.64 turns.
-__device__ __forceinline__ float pll_two_sin2(uint64_t q, double dphi) {
+// Twice the loop phase in half-turns, float32 (lr = bpf * 2 sin(pi h)); q is
+// the ramp phase of the same step in Q0.64 turns.
+__device__ __forceinline__ float pll_twice(uint64_t q, double dphi) {
     const uint64_t q2 = 2 * q;
-    const float h = (float)(int32_t)(q2 >> 32) * 4.656612873077393e-10f + (float)(dphi * (2.0 / GPUD_PI));
-    return 2.0f * sinpif(h);
+    return (float)(int32_t)(q2 >> 32) * 4.656612873077393e-10f + (float)(dphi * (2.0 / GPUD_PI));
 }
 
 // End of one stereoDecodeStateful call: store the loop state, update errAvg
@@ -1459,8 +1511,8 @@ k_pll(const int *__restrict__ list, int count, const SlotBlock *__restrict__ sbt
     }
     __syncthreads();
     const PllK k = pll_consts(cp, s);
-    double dphi = 0.0, df = 0.0, es = 0.0;
-    float I = (float)s.pll_i, Q = (float)s.pll_q;
+    PllRun x = pll_begin(0.0, 0.0, (float)s.pll_i, (float)s.pll_q);
+    double es = 0.0;
     for (int c = 0; c <= nc; ++c) {
         if (warp == 0) {
             if (lane == 0 && c < nc) {
@@ -1471,14 +1523,11 @@ k_pll(const int *__restrict__ list, int count, const SlotBlock *__restrict__ sbt
                 uint64_t qr = k.q0 + (uint64_t)base * k.qf;
                 for (int q = 0; q < len; ++q) {
                     PllEval o;
-                    pll_step<false>(qr, dphi, df, I, Q, sp[q], k, o);
+                    if (q % kPllSeg == 0) x = pll_begin(x.dphi, x.df, x.I, x.Q);
+                    pll_step<false>(qr, x, sp[q], k, o);
                     qr += k.qf;
-                    dphi = o.dphi1;
-                    df = o.df1;
-                    I = o.I1;
-                    Q = o.Q1;
                     es += fabs((double)o.e);
-                    th[q] = pll_two_sin2(qr, dphi);
+                    th[q] = pll_twice(qr, x.dphi);
                 }
             }
         } else {
@@ -1491,7 +1540,7 @@ k_pll(const int *__restrict__ list, int count, const SlotBlock *__restrict__ sbt
                 for (int q = lane; q < len; q += 32) {
                     const double p = (double)sp[q];
                     pp += p * p;
-                    lr[base + q] = bpf[base + q] * th[q];
+                    lr[base + q] = bpf[base + q] * (2.0f * sinpif(th[q]));
                 }
             }
             __syncwarp();
@@ -1510,56 +1559,77 @@ k_pll(const int *__restrict__ list, int count, const SlotBlock *__restrict__ sbt
     }
     __syncthreads();
     if (threadIdx.x != 0) return;
-    pll_finish(s, cp, n, pll_phase_at(k, n, dphi), s.pll_freq + df, (double)I, (double)Q, es, s_red[0]);
+    pll_finish(s, cp, n, pll_phase_at(k, n, x.dphi), s.pll_freq + x.df, (double)x.I, (double)x.Q, es, s_red[0]);
     s.pll_path = 2;
 }
 
 
 // ===========================================================================
-// Pilot PLL, parallel in time: multiple-shooting Newton.
+// Pilot PLL, parallel in time: a coarse model of the loop, then
+// multiple-shooting Newton on the loop itself.
 // ===========================================================================
 // The block's loop trajectory x_t = (phase, freq, I, Q), t = 0..n, obeys
 // x_{t+1} = F(x_t, p_t) with the serial kernel's exact step F.  The block is
-// cut into one segment of S consecutive steps per thread; the unknowns are the
-// segment start states s_g.  Each iteration every thread integrates its
-// segment with F from s_g (the exact nonlinear loop, no linearisation inside
-// the segment), giving the end state E_g(s_g) and the segment Jacobian
-// M_g = J_{t1-1} ... J_{t0}.  Newton's update of the start states,
+// cut into one segment of S = 16 consecutive steps per thread; the unknowns
+// are the segment start states s_g.  Each iteration every thread integrates
+// its segment with F from s_g (the exact nonlinear loop, no linearisation
+// inside the segment), giving the end state E_g(s_g), and Newton's update of
+// the start states,
 //     d_{g+1} = M_g d_g + (E_g(s_g) - s_{g+1}),   d_0 = 0,   s_g <- s_g + d_g,
 // is a linear recurrence over segments, solved by an associative scan over
 // affine maps (4x4 matrix + vector, float32; states and residuals float64 /
 // float32 as in F): warp shuffles, then shared memory across warps, then
 // distributed shared memory across the cluster's CTAs.  The fixed point is the
-// serial trajectory.  From the free-running guess s_g = (phase_0 + t0 freq_0,
-// freq_0, I_0, Q_0) a locked loop converges in 3-5 iterations; acquisition
-// from zero I/Q and noise-driven loops (no pilot) take tens to a hundred, since
-// a segment whose start is exact is exact after one more iteration.  A block
-// not converged after max_iters iterations keeps its consistent prefix and one
-// thread runs the serial loop over the rest.  No trajectory is stored: a last
-// pass integrates each segment from its converged start and writes the
-// outputs.
+// serial trajectory whatever M_g is and wherever the iteration starts: both
+// set the number of iterations only.
+//
+// Where it starts: the loop is slow (50 Hz bandwidth, 200 Hz I/Q lowpass)
+// against a segment, so a segment's effect on the state is known to ~1e-4 rad
+// from four sums over its pilot samples (CoarseSeg), taken once.  The start
+// states come from Newton on that coarse map -- no sweep over samples, one
+// scan each -- and then iterations with F, at first with the coarse map's
+// Jacobian for M_g: two for a locked loop.  Loops that turn against the
+// free-running ramp (acquisition, requests on noise) go on with F's own segment
+// Jacobians.
+//
+// Measured (kernel alone; before: Newton with F's Jacobians from the
+// free-running ramp and scans by shuffles): 40 channels x 32768 steps 78 -> 52
+// us (3-5 -> 2 iterations), one channel of 7680 steps 48 -> 28 us, 154 channels
+// of 8192 steps of which half on noise 360-495 -> 119 us (up to 64 iterations
+// and a serial rest -> 12).  What bounds it: the latency of 16 dependent steps
+// (~250 cycles each) and of a scan (~4500 cycles) per iteration.
+//
+// A block not converged after max_iters iterations keeps its consistent
+// prefix (a segment whose start is exact is exact after one more iteration)
+// and one warp runs the serial loop over the rest.  Blocks longer than one
+// segment per thread of the largest cluster (32768 steps) are solved chunk by
+// chunk, each from the end state of the one before.
 #ifndef GPUD_PLL_CLUSTER
-#define GPUD_PLL_CLUSTER 8  // CTAs per channel at most: segment length max(16, n / (256 * this))
-#endif
-#ifndef GPUD_PLL_JAC_SWEEPS
-#define GPUD_PLL_JAC_SWEEPS 2  // sweeps that evaluate the segment Jacobians before chord steps may start
+#define GPUD_PLL_CLUSTER 8  // CTAs per channel at most
 #endif
 constexpr int kNewtonThreads = 256;
 constexpr int kNewtonMaxCluster = GPUD_PLL_CLUSTER;
-constexpr int kNewtonMinSeg = 16;
-
-// Steps per segment (per thread) for a block of n loop steps.
-__host__ __device__ inline int pll_segment_len(int n) {
-    const int cap = kNewtonMaxCluster * kNewtonThreads;
-    const int s = (n + cap - 1) / cap;
-    return s > kNewtonMinSeg ? s : kNewtonMinSeg;
-}
+constexpr int kPllChunkSteps = kNewtonMaxCluster * kNewtonThreads * kPllSeg;  // steps solved at once
+#ifndef GPUD_PLL_COARSE
+#define GPUD_PLL_COARSE 2  // Newton iterations on the coarse map of a locked loop
+#endif
+#ifndef GPUD_PLL_COARSE_FREE
+#define GPUD_PLL_COARSE_FREE 8  // ... and of one that was not
+#endif
+#ifndef GPUD_PLL_QUASI
+#define GPUD_PLL_QUASI 8  // iterations on the loop that take the coarse map's Jacobian
+#endif
+constexpr int kPllCoarse = GPUD_PLL_COARSE, kPllCoarseFree = GPUD_PLL_COARSE_FREE, kPllQuasi = GPUD_PLL_QUASI;
+static_assert(kPllCoarse > 0 && kPllCoarseFree > 0, "sh.next starts in the coarse iterations");
+constexpr int kPllOnce = 3;       // iterations within which a locked loop converges
+constexpr int kPllJacSweeps = 2;  // then: sweeps that evaluate F's segment Jacobians before chord steps may start
 
 // CTAs per cluster that give every channel of a launch (at most max_n steps)
-// one thread per segment.
+// one thread per segment of a chunk.
 int pll_cluster_for(int max_n) {
-    const int seg = (max_n + pll_segment_len(max_n) - 1) / pll_segment_len(max_n);
-    int c = (seg + kNewtonThreads - 1) / kNewtonThreads;
+    const int steps = max_n < kPllChunkSteps ? max_n : kPllChunkSteps;
+    const int seg = (steps + kPllSeg - 1) / kPllSeg;
+    const int c = (seg + kNewtonThreads - 1) / kNewtonThreads;
     int p = 1;
     while (p < c) p *= 2;
     return p < 1 ? 1 : (p > kNewtonMaxCluster ? kNewtonMaxCluster : p);
@@ -1568,12 +1638,8 @@ int pll_cluster_for(int max_n) {
 // outputs resolve (the float32 sin/cos/atan2 and lowpass states leave a floor
 // near 1e-10 rad and 1e-9 in I/Q).
 constexpr float kTolPhase = 1e-8f, kTolFreq = 1e-12f, kTolIQ = 1e-7f;
+constexpr float kTolAngle = 2.4e-7f;  // half an ulp of an angle of up to 2 pi in float32
 constexpr int kNW = kNewtonThreads / 32;
-
-struct Aff {
-    float a[16];  // row-major, state order (phase, freq, I, Q)
-    float b[4];
-};
 
 // M <- J M, with J's sparsity (phase/freq rows dense, I/Q rows phase + diagonal).
 __device__ __forceinline__ void mat_push(float (&m)[16], const PllEval &o, float om) {
@@ -1587,90 +1653,245 @@ __device__ __forceinline__ void mat_push(float (&m)[16], const PllEval &o, float
     }
 }
 
-// hi o lo (lo applied first)
-__device__ __forceinline__ void aff_compose(Aff &out, const Aff &hi, const Aff &lo) {
-    Aff r;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            r.a[4 * i + j] = fmaf(hi.a[4 * i], lo.a[j],
-                                  fmaf(hi.a[4 * i + 1], lo.a[4 + j],
-                                       fmaf(hi.a[4 * i + 2], lo.a[8 + j], hi.a[4 * i + 3] * lo.a[12 + j])));
-        }
-        r.b[i] = fmaf(hi.a[4 * i], lo.b[0],
-                      fmaf(hi.a[4 * i + 1], lo.b[1], fmaf(hi.a[4 * i + 2], lo.b[2], fmaf(hi.a[4 * i + 3], lo.b[3], hi.b[i]))));
-    }
-    out = r;
-}
-
-__device__ __forceinline__ void aff_shfl_up(Aff &dst, const Aff &src, int d) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) dst.a[i] = __shfl_up_sync(0xffffffffu, src.a[i], d);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) dst.b[i] = __shfl_up_sync(0xffffffffu, src.b[i], d);
-}
-
-__device__ __forceinline__ void aff_identity(Aff &m) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) m.a[i] = (i % 5 == 0) ? 1.f : 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) m.b[i] = 0.f;
-}
-
-__device__ __forceinline__ void aff_load(Aff &m, const float *src) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) m.a[i] = src[i];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) m.b[i] = src[16 + i];
-}
-
-__device__ __forceinline__ void aff_store(float *dst, const Aff &m) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) dst[i] = m.a[i];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) dst[16 + i] = m.b[i];
-}
-
-__device__ __forceinline__ void aff_apply(float out[4], const Aff &m, const float x[4]) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        out[i] = fmaf(m.a[4 * i], x[0], fmaf(m.a[4 * i + 1], x[1], fmaf(m.a[4 * i + 2], x[2], fmaf(m.a[4 * i + 3], x[3], m.b[i]))));
-}
-
 // Segment start state, deviation form (see pll_step).
 struct SegState {
     double dphi, df;
     float I, Q;
 };
 
-// One channel-block per cluster of `gridDim.x / count` CTAs; the block's steps
-// are split into one contiguous segment per thread of the cluster.  With
-// segments of at most kPllStageS steps (blocks of up to 32768 composite
-// samples) each CTA first stages its span of the pilot band in shared memory,
-// transposed (step i of thread j's segment at [i][j], conflict-free), so every
-// Newton sweep reads it from there; the output sweep writes 2 sin(2 phase)
-// back into the same cells and the CTA then writes the L-R products with
-// coalesced stores.
-constexpr int kPllStageS = 16;
+// What the coarse map knows of a segment of m steps with the loop phase held
+// at the free-running ramp theta_i plus a constant: with r = 1 - lpa,
+//     C + jS   = sum_i r^(m-1-i) p_i exp(j theta_i)
+//     C2 + jS2 = sum over the steps of the same sum up to that step,
+// so that I and Q after the segment and their means over it are linear in the
+// state and in the sine and cosine of the constant.
+struct CoarseSeg {
+    float4 c;      // C, S, C2, S2
+    float rm, r1;  // r^m, (r + ... + r^m) / m
+    float m;
+};
 
+// atan2 to 1e-5 rad (the odd polynomial of Abramowitz and Stegun 4.4.49 on
+// the smaller over the larger): the coarse map only sets where Newton starts.
+__device__ __forceinline__ float coarse_atan2(float y, float x) {
+    const float ax = fabsf(x), ay = fabsf(y);
+    const float hi = fmaxf(ax, ay), lo = fminf(ax, ay);
+    const float t = hi > 0.f ? __fdividef(lo, hi) : 0.f;
+    const float u = t * t;
+    float r = fmaf(u, fmaf(u, fmaf(u, fmaf(u, 0.0208351f, -0.0851330f), 0.1801410f), -0.3302995f), 0.9998660f) * t;
+    r = ay > ax ? 1.57079633f - r : r;
+    r = x < 0.f ? 3.14159265f - r : r;
+    return copysignf(r, y);
+}
+
+// The coarse map of one segment from start state x: the map's matrix in a
+// (row-major) and, in float32, the mismatch of the segment's end with the next
+// start nx (the float64 differences are taken first).
+__device__ __forceinline__ float4 coarse_step(const CoarseSeg &c, const PllK &k, const SegState &x, const SegState &nx,
+                                              float (&a)[16]) {
+    const float alpha = (float)k.alpha, beta = (float)k.beta, half = 0.5f * (c.m - 1.f);
+    const float df = (float)x.df;
+    // the phase at the middle of the segment
+    float sn, cs;
+    __sincosf(fmaf(half, fmaf(alpha, coarse_atan2(x.Q, x.I), df), (float)x.dphi), &sn, &cs);
+    const float ri = c.rm * x.I, rq = c.rm * x.Q;
+    const float dI = k.lpa * fmaf(cs, c.c.x, -sn * c.c.y), dQ = -k.lpa * fmaf(sn, c.c.x, cs * c.c.y);
+    const float lm = k.lpa * pll_rcp(c.m);
+    const float mi = lm * fmaf(cs, c.c.z, -sn * c.c.w), mq = -lm * fmaf(sn, c.c.z, cs * c.c.w);
+    const float Im = fmaf(c.r1, x.I, mi), Qm = fmaf(c.r1, x.Q, mq);
+    const float e = coarse_atan2(Qm, Im);
+    const float ka = c.m * alpha, kf = c.m * beta, kp = fmaf(0.5f * (c.m + 1.f), kf, ka);
+    const float f1 = fmaf(kf, e, df);
+    const bool clamped = f1 < (float)k.dfmin || f1 > (float)k.dfmax;
+    const float fc = fminf(fmaxf(f1, (float)k.dfmin), (float)k.dfmax);
+    const float r2 = fmaf(Im, Im, Qm * Qm);
+    const float inv = r2 > 0.f ? pll_rcp(r2) : 0.f;
+    const float gI = -Qm * inv, gQ = Im * inv;
+    const float ePhi = fmaf(gI, mq, -gQ * mi), eI = gI * c.r1, eQ = gQ * c.r1;
+    const float pF = clamped ? 0.f : 1.f, kfe = clamped ? 0.f : kf, kpe = clamped ? ka : kp;
+    a[0] = fmaf(kpe, ePhi, 1.f);
+    a[1] = fmaf(kpe * half, ePhi, pF * c.m);
+    a[2] = kpe * eI;
+    a[3] = kpe * eQ;
+    a[4] = kfe * ePhi;
+    a[5] = fmaf(kfe * half, ePhi, pF);
+    a[6] = kfe * eI;
+    a[7] = kfe * eQ;
+    a[8] = dQ;
+    a[9] = half * dQ;
+    a[10] = c.rm;
+    a[11] = 0.f;
+    a[12] = -dI;
+    a[13] = half * -dI;
+    a[14] = 0.f;
+    a[15] = c.rm;
+    return make_float4((float)(x.dphi - nx.dphi) + fmaf(c.m, clamped ? fc : df, kpe * e),
+                       (float)(x.df - nx.df) + (fc - df), ri + dI - nx.I, rq + dQ - nx.Q);
+}
+
+// An affine map of the state, column by column: four matrix columns (the
+// images of phase, freq, I and Q), then the vector.
+struct AffCols {
+    float4 c[5];
+};
+
+// Columns of a (without its vector) times v, plus w.
+__device__ __forceinline__ float4 aff_mul(const AffCols &a, const float4 &v, const float4 &w) {
+    const float4 c0 = a.c[0], c1 = a.c[1], c2 = a.c[2], c3 = a.c[3];
+    float4 r;
+    r.x = fmaf(c0.x, v.x, fmaf(c1.x, v.y, fmaf(c2.x, v.z, fmaf(c3.x, v.w, w.x))));
+    r.y = fmaf(c0.y, v.x, fmaf(c1.y, v.y, fmaf(c2.y, v.z, fmaf(c3.y, v.w, w.y))));
+    r.z = fmaf(c0.z, v.x, fmaf(c1.z, v.y, fmaf(c2.z, v.z, fmaf(c3.z, v.w, w.z))));
+    r.w = fmaf(c0.w, v.x, fmaf(c1.w, v.y, fmaf(c2.w, v.z, fmaf(c3.w, v.w, w.w))));
+    return r;
+}
+
+__device__ __forceinline__ float4 aff_apply(const AffCols &a, const float4 &v) { return aff_mul(a, v, a.c[4]); }
+
+// Column `col` of the composition of N maps, the first applied first (the next
+// map is loaded while one is applied).
+template <int N>
+__device__ __forceinline__ float4 aff_chain(const AffCols *a, int col) {
+    float4 v = a[0].c[col];
+    AffCols m = a[1];
+#pragma unroll
+    for (int i = 1; i < N; ++i) {
+        const AffCols cur = m;
+        if (i + 1 < N) m = a[i + 1];
+        v = aff_mul(cur, v, col == 4 ? cur.c[4] : make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+    return v;
+}
+
+constexpr int kPllRun = 8;  // segments per run of the scan
+
+struct PllShared {
+    AffCols aff[kNewtonThreads];       // the segments' maps (their matrices kept for chord steps)
+    AffCols run[kNewtonThreads / kPllRun];  // compositions: runs of 8 segments,
+    AffCols warp[kNW];                      // warps,
+    AffCols cta[2][kNewtonMaxCluster];      // and CTAs of the cluster (double-buffered across scans)
+    float4 coarse[kNewtonThreads];     // CoarseSeg::c of every segment
+    float4 dmax[2][kNewtonMaxCluster * kNW];  // every warp's largest corrections (double-buffered)
+    SegState first[kNW];               // each warp's first segment start
+    SegState next;                     // the next CTA's first segment start
+    SegState end;                      // the chunk's end state
+    float seg[kPllSeg][kNewtonThreads + 1];  // staged pilot band, then twice the loop phase
+    double sum[kNewtonMaxCluster * kNW][2];  // every warp's sums over the block (in CTA 0)
+    int badw[kNW];
+    int cbad;
+};
+
+// d at each segment start from the segments' affine maps in sh.aff (each
+// written by its thread): the recurrence over the whole cluster.  The maps are
+// composed upwards column by column -- a lane carries one of the five columns
+// through a run of 8 segments, then through the warp's 4 runs, the CTA's 8
+// warps -- so a composition is 16 multiply-adds in a lane and nothing is
+// shuffled; downwards only the vector d is applied.  pb alternates from scan
+// to scan; one cluster barrier.  (With whole maps per lane and shuffles, 5 + 3
+// + 3 rounds of 20 shuffles and 84 multiply-adds, a scan took 7000 cycles;
+// this one ~2500.)
+template <class Cluster>
+__device__ __forceinline__ float4 pll_scan(Cluster &cl, PllShared &sh, int pb, int crank, int csize) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rn = lane >> 3, col = lane & 7;
+    const AffCols *seg = sh.aff + warp * 32;
+    AffCols *run = sh.run + warp * (32 / kPllRun);
+    __syncwarp();
+    if (col < 5) run[rn].c[col] = aff_chain<kPllRun>(seg + rn * kPllRun, col);
+    __syncwarp();
+    if (lane < 5) sh.warp[warp].c[lane] = aff_chain<32 / kPllRun>(run, lane);
+    __syncthreads();
+    if (csize > 1) {
+        if (warp == 0 && lane < 5) {
+            const float4 v = aff_chain<kNW>(sh.warp, lane);
+            for (int r = crank + 1; r < csize; ++r) cl.map_shared_rank(&sh.cta[pb][crank], r)->c[lane] = v;
+        }
+        cl.sync();  // the CTAs before this one have written their maps here
+    }
+    float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+    for (int r = 0; r < crank; ++r) d = aff_apply(sh.cta[pb][r], d);
+#pragma unroll 2
+    for (int w = 0; w < warp; ++w) d = aff_apply(sh.warp[w], d);
+#pragma unroll
+    for (int r = 0; r < 32 / kPllRun - 1; ++r) {
+        const float4 v = aff_apply(run[r], d);
+        if (r < rn) d = v;
+    }
+    // inside a run d moves from lane to lane, each applying its own map
+    const AffCols own = seg[lane];
+#pragma unroll
+    for (int i = 1; i < kPllRun; ++i) {
+        const float4 v = aff_apply(own, d);
+        const float4 u = make_float4(__shfl_up_sync(0xffffffffu, v.x, 1), __shfl_up_sync(0xffffffffu, v.y, 1),
+                                     __shfl_up_sync(0xffffffffu, v.z, 1), __shfl_up_sync(0xffffffffu, v.w, 1));
+        if (col == i) d = u;
+    }
+    __syncwarp();  // the segments' maps have been read
+    return d;
+}
+
+// The next segment's start state: the next lane's, the next warp's first, or
+// (the CTA's last thread) the next CTA's first.
+__device__ __forceinline__ SegState pll_next_start(const SegState &x0, const PllShared &sh) {
+    SegState nx{__shfl_down_sync(0xffffffffu, x0.dphi, 1), __shfl_down_sync(0xffffffffu, x0.df, 1),
+                __shfl_down_sync(0xffffffffu, x0.I, 1), __shfl_down_sync(0xffffffffu, x0.Q, 1)};
+    const int warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 31) nx = warp < kNW - 1 ? sh.first[warp + 1] : sh.next;
+    return nx;
+}
+
+// A segment's map for the scan: its matrix (row-major a) and the mismatch of
+// its end state x with the next segment's start nx.
+__device__ __forceinline__ void pll_put_matrix(AffCols &m, const float (&a)[16]) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) m.c[c] = make_float4(a[c], a[4 + c], a[8 + c], a[12 + c]);
+}
+
+__device__ __forceinline__ void pll_put_identity(AffCols &m) {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) m.c[c] = make_float4(c == 0, c == 1, c == 2, c == 3);
+}
+
+__device__ __forceinline__ float pll_max(float a, float b) {
+    return __uint_as_float(max(__float_as_uint(a), __float_as_uint(b)));
+}
+
+__device__ __forceinline__ float4 pll_warp_max(const float4 &v) {
+    return make_float4(__uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v.x))),
+                       __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v.y))),
+                       __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v.z))),
+                       __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v.w))));
+}
+
+__device__ __forceinline__ void pll_put_gap(AffCols &m, const SegState &x, const SegState &nx, bool has_next) {
+    m.c[4] = has_next ? make_float4((float)(x.dphi - nx.dphi), (float)(x.df - nx.df), x.I - nx.I, x.Q - nx.Q)
+                      : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// x += d, the frequency kept within `reach` of f0: a step changes it by at most
+// pi beta, so a start t steps on cannot be further off.  (An iterate that
+// overshoots on noise would run into the frequency clamp, where the map forgets
+// its start, and only the consistent prefix would grow, a segment an iteration.)
+__device__ __forceinline__ void pll_move(SegState &x, const float4 &d, double f0, double reach) {
+    x.dphi += (double)d.x;
+    x.df = fmin(fmax(x.df + (double)d.y, f0 - reach), f0 + reach);
+    x.I += d.z;
+    x.Q += d.w;
+}
+
+// One channel-block per cluster of `gridDim.x / count` CTAs.  Each CTA stages
+// its span of the chunk's pilot band in shared memory, transposed (step i of
+// thread j's segment at [i][j], conflict-free), so every sweep reads it from
+// there; the output sweep writes twice the loop phase back into the same cells
+// and the CTA then writes the L-R products with coalesced stores.
 __global__ void __launch_bounds__(kNewtonThreads, 3)
 k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restrict__ sbt,
              const ChanParams *__restrict__ prm, ChanState *__restrict__ st, float *__restrict__ wk, int W,
              int max_iters) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
-    __shared__ float s_tot[kNW][20];     // warp totals
-    __shared__ float s_wex[kNW][20];     // exclusive warp prefix (A, b) within the CTA
-    __shared__ float s_cta[2][20];       // CTA total, double-buffered across iterations
-    __shared__ float s_max[kNW][4];
-    __shared__ float s_cmax[2][4];       // CTA max |d|, double-buffered
-    __shared__ float s_dcta[4];          // d at this CTA's first segment
-    __shared__ SegState s_first[kNW];    // each warp's first segment start (lane 0)
-    __shared__ float s_jac[16][kNewtonThreads];  // each segment's Jacobian, kept for chord steps
-    __shared__ float s_seg[kPllStageS][kNewtonThreads + 1];  // staged pilot band / 2 sin(2 phase)
-    __shared__ double s_sum[kNW][2];
-    __shared__ double s_csum[2];
+    __shared__ PllShared sh;
     const int csize = (int)cl.num_blocks();
     const int crank = (int)cl.block_rank();
     const int idx = blockIdx.x / csize;
@@ -1685,249 +1906,296 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
     float *lr = wk + 4 * W + sb.comp_off;
     const PllK k = pll_consts(cp, s);
     const float om = 1.f - k.lpa;
-    const float I0 = (float)s.pll_i, Q0 = (float)s.pll_q;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // The segment length depends on the channel's own block length only, so a
+    const int tid = (int)threadIdx.x;
+    const int g = crank * kNewtonThreads + tid;
+    // The segmentation depends on the channel's own block length only, so a
     // channel's trajectory (and every rounding in it) is the same whatever
-    // other channels share the launch; the cluster supplies at least
-    // ceil(n / S) threads.
-    const int S = pll_segment_len(n);
-    const int g = crank * kNewtonThreads + (int)threadIdx.x;
-    const int t0 = min(n, g * S), t1 = min(n, t0 + S);
-    const bool has_next = t1 < n;  // the next thread's segment is not empty
-    const bool staged = S <= kPllStageS;  // uniform
-    const int cbase = min(n, crank * kNewtonThreads * S);
-    const int cend = min(n, cbase + kNewtonThreads * S);
-    if (staged) {
-        for (int t = cbase + (int)threadIdx.x; t < cend; t += kNewtonThreads) {
-            const int r = t - cbase;
-            s_seg[r % S][r / S] = __ldg(pil + t);
-        }
-        __syncthreads();
-    }
-    auto pilot = [&](int t) -> float { return staged ? s_seg[t - t0][threadIdx.x] : __ldg(pil + t); };
-    SegState x0{0.0, 0.0, I0, Q0};  // this segment's start: the free-running guess
-    bool converged = false, bad = true;
-    float prev_m0 = 1e30f;  // last iteration's largest phase correction (uniform in the cluster)
-    int iters = 0;
-    for (int it = 0; it < max_iters && !converged; ++it) {
-        iters = it + 1;
-        const int pb = it & 1;
-        // ---- the next segment's start state ------------------------------
-        SegState nx{0.0, 0.0, I0, Q0};
+    // other channels share the launch; the cluster supplies at least one
+    // thread per segment.
+    SegState start{0.0, 0.0, (float)s.pll_i, (float)s.pll_q};  // the chunk's start state
+    bool all_converged = true;
+    bool locked = s.locked != 0;  // the loop of the last block, then whether the last chunk's converged at once
+    int iters = 0, pb = 0;
+    double es = 0.0, pp = 0.0;  // this thread's sums over the block
+    for (int c0 = 0; c0 < n; c0 += kPllChunkSteps) {
+        const int nc = min(n - c0, kPllChunkSteps);
+        const int t0 = c0 + min(nc, g * kPllSeg), t1 = min(c0 + nc, t0 + kPllSeg);
+        const bool has_next = t1 < c0 + nc;  // the next thread's segment is not empty
+        const int nseg = (nc + kPllSeg - 1) / kPllSeg;
+        const int cbase = c0 + min(nc, crank * kNewtonThreads * kPllSeg);
+        const int cend = min(c0 + nc, cbase + kNewtonThreads * kPllSeg);
         {
-            const double a = __shfl_down_sync(0xffffffffu, x0.dphi, 1);
-            const double b = __shfl_down_sync(0xffffffffu, x0.df, 1);
-            const float c = __shfl_down_sync(0xffffffffu, x0.I, 1);
-            const float d = __shfl_down_sync(0xffffffffu, x0.Q, 1);
-            if (it > 0 && has_next) {
-                if (lane < 31)
-                    nx = SegState{a, b, c, d};
-                else if (warp < kNW - 1)
-                    nx = s_first[warp + 1];
-                else
-                    nx = *cl.map_shared_rank(&s_first[0], crank + 1);
+            float v[kPllSeg];
+#pragma unroll
+            for (int i = 0; i < kPllSeg; ++i) {
+                const int t = cbase + tid + i * kNewtonThreads;
+                v[i] = t < cend ? __ldg(pil + t) : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < kPllSeg; ++i) {
+                const int r = tid + i * kNewtonThreads;
+                sh.seg[r % kPllSeg][r / kPllSeg] = v[i];
             }
         }
-        // ---- integrate the segment: end state and Jacobian ----------------
-        // Close to the solution (the last corrections below 1e-2 rad) the
-        // segment Jacobians barely move: they are kept from the last full
-        // evaluation (chord steps), which converge as fast as Newton there.
-        const bool jac = it < GPUD_PLL_JAC_SWEEPS || prev_m0 > 1e-2f;
-        Aff m;
-        aff_identity(m);
-        SegState x = x0;
-        if (t0 < t1) {
+        __syncthreads();
+        // ---- the segment's coarse sums ------------------------------------
+        CoarseSeg co{make_float4(0.f, 0.f, 0.f, 0.f), 1.f, 0.f, (float)(t1 - t0)};
+        {
             uint64_t qr = k.q0 + (uint64_t)t0 * k.qf;
-            if (jac) {
-                for (int t = t0; t < t1; ++t) {
-                    PllEval o;
-                    pll_step<true>(qr, x.dphi, x.df, x.I, x.Q, pilot(t), k, o);
-                    qr += k.qf;
-                    mat_push(m.a, o, om);
-                    x = SegState{o.dphi1, o.df1, o.I1, o.Q1};
-                }
-#pragma unroll
-                for (int i = 0; i < 16; ++i) s_jac[i][threadIdx.x] = m.a[i];
-            } else {
-                for (int t = t0; t < t1; ++t) {
-                    PllEval o;
-                    pll_step<false>(qr, x.dphi, x.df, x.I, x.Q, pilot(t), k, o);
-                    qr += k.qf;
-                    x = SegState{o.dphi1, o.df1, o.I1, o.Q1};
-                }
-#pragma unroll
-                for (int i = 0; i < 16; ++i) m.a[i] = s_jac[i][threadIdx.x];
-            }
-            if (has_next) {
-                m.b[0] = (float)(x.dphi - nx.dphi);
-                m.b[1] = (float)(x.df - nx.df);
-                m.b[2] = x.I - nx.I;
-                m.b[3] = x.Q - nx.Q;
-            }
-        }
-        // ---- scan: d at each segment start -------------------------------
-        Aff inc = m;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            Aff o;
-            aff_shfl_up(o, inc, d);
-            if (lane >= d) aff_compose(inc, inc, o);
-        }
-        Aff exl;  // lanes before this one
-        aff_shfl_up(exl, inc, 1);
-        if (lane == 0) aff_identity(exl);
-        if (lane == 31) aff_store(s_tot[warp], inc);
-        __syncthreads();
-        if (warp == 0) {
-            Aff wv;
-            if (lane < kNW) aff_load(wv, s_tot[lane]);
-            else aff_identity(wv);
-            // only lanes 0..kNW-1 carry warp totals: log2(kNW) rounds
-#pragma unroll
-            for (int d = 1; d < kNW; d <<= 1) {
-                Aff o;
-                aff_shfl_up(o, wv, d);
-                if (lane >= d) aff_compose(wv, wv, o);
-            }
-            Aff ex;
-            aff_shfl_up(ex, wv, 1);
-            if (lane == 0) aff_identity(ex);
-            if (lane < kNW) aff_store(s_wex[lane], ex);
-            if (lane == kNW - 1) aff_store(s_cta[pb], wv);
-        }
-        cl.sync();  // CTA totals of the whole cluster are visible
-        // d at this CTA's first segment: the CTA totals before it, composed by
-        // a scan across warp 0's lanes (lane r holds CTA r's total) and
-        // applied to a zero correction
-        if (warp == 0) {
-            Aff tv;
-            if (lane < crank) aff_load(tv, cl.map_shared_rank(&s_cta[pb][0], lane));
-            else aff_identity(tv);
-#pragma unroll
-            for (int d = 1; d < kNewtonMaxCluster; d <<= 1) {
-                Aff o;
-                aff_shfl_up(o, tv, d);
-                if (lane >= d) aff_compose(tv, tv, o);
-            }
-            const int src = crank > 0 ? crank - 1 : 0;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float v = __shfl_sync(0xffffffffu, tv.b[i], src);
-                if (lane == 0) s_dcta[i] = crank > 0 ? v : 0.f;
-            }
-        }
-        __syncthreads();
-        const float dcta[4] = {s_dcta[0], s_dcta[1], s_dcta[2], s_dcta[3]};
-        float dl[4];
-        {
-            Aff wx;
-            aff_load(wx, s_wex[warp]);
-            float dw[4];
-            aff_apply(dw, wx, dcta);
-            aff_apply(dl, exl, dw);
-        }
-        // ---- update the start state --------------------------------------
-        float mx[4] = {0.f, 0.f, 0.f, 0.f};
-        bad = false;
-        if (t0 < t1) {
-            bad = fabsf(dl[0]) > kTolPhase || fabsf(dl[1]) > kTolFreq || fabsf(dl[2]) > kTolIQ ||
-                  fabsf(dl[3]) > kTolIQ;
-            x0.dphi += (double)dl[0];
-            x0.df += (double)dl[1];
-            x0.I += dl[2];
-            x0.Q += dl[3];
-            mx[0] = fabsf(dl[0]);
-            mx[1] = fabsf(dl[1]);
-            mx[2] = fabsf(dl[2]);
-            mx[3] = fabsf(dl[3]);
-        }
-        if (lane == 0) s_first[warp] = x0;
-        // ---- convergence, agreed by every CTA of the cluster ---------------
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], off));
-        if (lane == 0)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) s_max[warp][i] = mx[i];
-        __syncthreads();
-        if (threadIdx.x < 4) {
-            float v = 0.f;
-            for (int w2 = 0; w2 < kNW; ++w2) v = fmaxf(v, s_max[w2][threadIdx.x]);
-            s_cmax[pb][threadIdx.x] = v;
-        }
-        cl.sync();  // also publishes s_first for the next iteration's reads
-        float m0 = 0.f, m1 = 0.f, m2 = 0.f, m3 = 0.f;
-        for (int r = 0; r < csize; ++r) {
-            const float *rm = cl.map_shared_rank(&s_cmax[pb][0], r);
-            m0 = fmaxf(m0, rm[0]);
-            m1 = fmaxf(m1, rm[1]);
-            m2 = fmaxf(m2, rm[2]);
-            m3 = fmaxf(m3, rm[3]);
-        }
-        converged = (m0 <= kTolPhase && m1 <= kTolFreq && m2 <= kTolIQ && m3 <= kTolIQ);
-        // Accepted one iteration early when the next correction is predicted
-        // below the tolerance: corrections shrinking at least linearly at rate
-        // m0 / prev_m0 leave a next one of m0^2 / prev_m0 (Newton's quadratic
-        // rate leaves less), with the other components already near their floor.
-        if (!converged && it >= 1 && m0 <= 1e-5f && m0 * m0 <= kTolPhase * prev_m0 && m1 <= 1e-10f &&
-            m2 <= 1e-6f && m3 <= 1e-6f)
-            converged = true;
-        prev_m0 = m0;
-    }
-    // ---- not converged: the longest consistent prefix is kept ------------
-    // Segments before the first one whose start still moved by more than the
-    // tolerance form a consistent trajectory from the block start, and that
-    // segment's updated start is its exact start; one thread continues the
-    // serial loop from there to the block end.
-    __shared__ int s_bad[kNW];
-    __shared__ int s_cbad;
-    int gstar = INT_MAX;
-    if (!converged) {
-        int v = bad ? g : INT_MAX;
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, off));
-        if (lane == 0) s_bad[warp] = v;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int c = INT_MAX;
-            for (int w2 = 0; w2 < kNW; ++w2) c = min(c, s_bad[w2]);
-            s_cbad = c;
-        }
-        cl.sync();
-        for (int r = 0; r < csize; ++r) gstar = min(gstar, *cl.map_shared_rank(&s_cbad, r));
-        if (gstar == INT_MAX) gstar = 0;  // cannot happen (not converged means one start moved)
-    }
-    // ---- outputs: each converged segment again from its start --------------
-    double es = 0.0, pp = 0.0;
-    SegState x = x0;
-    if (t0 < t1) {
-        const bool out = g < gstar;
-        uint64_t qr = k.q0 + (uint64_t)t0 * k.qf;
-        for (int t = t0; t < t1; ++t) {
-            const float pt = pilot(t);
-            pp += (double)pt * (double)pt;
-            if (out) {
-                PllEval o;
-                pll_step<false>(qr, x.dphi, x.df, x.I, x.Q, pt, k, o);
+            float C = 0.f, S = 0.f, C2 = 0.f, S2 = 0.f;
+#pragma unroll 4
+            for (int t = t0; t < t1; ++t) {
+                float sn, cs;
+                __sincosf(pll_ramp(qr), &sn, &cs);
                 qr += k.qf;
-                x = SegState{o.dphi1, o.df1, o.I1, o.Q1};
-                es += fabs((double)o.e);
-                const float th = pll_two_sin2(qr, x.dphi);
-                if (staged)
-                    s_seg[t - t0][threadIdx.x] = th;  // this thread's own cell, already read
-                else
-                    lr[t] = bpf[t] * th;
+                const float p = sh.seg[t - t0][tid];
+                C = fmaf(om, C, p * cs);
+                S = fmaf(om, S, p * sn);
+                C2 += C;
+                S2 += S;
+                co.rm *= om;
+                co.r1 += co.rm;
+            }
+            if (t0 < t1) co.r1 = __fdividef(co.r1, co.m);
+            sh.coarse[tid] = make_float4(C, S, C2, S2);
+        }
+        // ---- Newton on the coarse map, from the free-running guess ----------
+        // The next CTA's first start moves by this CTA's maps applied to its
+        // first correction (its own thread adds the same up to float32
+        // rounding), so an iteration takes one cluster barrier.
+        SegState x0{start.dphi + (double)(t0 - c0) * start.df, start.df, start.I, start.Q};
+        const double pi_beta = GPUD_PI * k.beta, reach = (double)(t0 - c0) * pi_beta;
+        if (tid == kNewtonThreads - 1)
+            sh.next = SegState{start.dphi + (double)(t1 - c0) * start.df, start.df, start.I, start.Q};
+        const int ncoarse = locked ? kPllCoarse : kPllCoarseFree;
+        for (int it = 0; it < ncoarse; ++it) {
+            if (lane == 0) sh.first[warp] = x0;
+            __syncthreads();
+            const SegState nx = pll_next_start(x0, sh);
+            float a[16];
+            co.c = sh.coarse[tid];
+            const float4 gap = coarse_step(co, k, x0, nx, a);
+            if (t0 < t1) {
+                pll_put_matrix(sh.aff[tid], a);
+                sh.aff[tid].c[4] = has_next ? gap : make_float4(0.f, 0.f, 0.f, 0.f);
+            } else {
+                pll_put_identity(sh.aff[tid]);
+            }
+            const float4 d = pll_scan(cl, sh, pb, crank, csize);
+            pb ^= 1;
+            if (t0 < t1) pll_move(x0, d, start.df, reach);
+            if (tid == kNewtonThreads - 1 && it + 1 < ncoarse) {
+                SegState y = sh.next;
+                pll_move(y, aff_apply(sh.aff[tid], d), start.df, reach + kPllSeg * pi_beta);
+                sh.next = y;
             }
         }
-    }
-    if (staged) {
-        // the L-R products of this CTA's output segments, coalesced
+        if (g == 0) x0 = start;  // exact
+        __syncthreads();         // the coarse iterations have read sh.first
+        if (lane == 0) sh.first[warp] = x0;
+        if (tid == 0 && crank > 0) *cl.map_shared_rank(&sh.next, crank - 1) = x0;
+        cl.sync();
+        // ---- Newton on the loop -------------------------------------------
+        bool converged = false, bad = true;
+        bool quasi = true;      // the coarse map's Jacobian (uniform in the cluster)
+        int sweeps = 0;         // of F with its own Jacobian
+        float prev_m0 = 1e30f;  // last iteration's largest phase correction (uniform in the cluster)
+        int it = 0;
+        for (; it < max_iters && !converged; ++it) {
+            const SegState nx = pll_next_start(x0, sh);
+            // Close to the solution (the last corrections below 1e-2 rad) the
+            // segment Jacobians barely move: they are kept from the last full
+            // evaluation (chord steps), which converge as fast as Newton there.
+            const bool jac = !quasi && (sweeps < kPllJacSweeps || prev_m0 > 1e-2f);
+            if (t0 < t1) {
+                PllRun x = pll_begin(x0.dphi, x0.df, x0.I, x0.Q);
+                PllEval o;
+                uint64_t qr = k.q0 + (uint64_t)t0 * k.qf;
+                if (jac) {
+                    float a[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) a[i] = i % 5 == 0 ? 1.f : 0.f;
+                    for (int t = t0; t < t1; ++t) {
+                        pll_step<true>(qr, x, sh.seg[t - t0][tid], k, o);
+                        qr += k.qf;
+                        mat_push(a, o, om);
+                    }
+                    pll_put_matrix(sh.aff[tid], a);
+                } else {
+                    float p = sh.seg[0][tid];
+#pragma unroll 2
+                    for (int t = t0; t < t1; ++t) {
+                        const float pn = sh.seg[min(t - t0 + 1, kPllSeg - 1)][tid];  // one step ahead
+                        pll_step<false>(qr, x, p, k, o);
+                        qr += k.qf;
+                        p = pn;
+                    }
+                    if (quasi) {
+                        float a[16];
+                        co.c = sh.coarse[tid];
+                        coarse_step(co, k, x0, nx, a);
+                        pll_put_matrix(sh.aff[tid], a);
+                    }
+                }
+                pll_put_gap(sh.aff[tid], SegState{x.dphi, x.df, x.I, x.Q}, nx, has_next);
+            } else {
+                pll_put_identity(sh.aff[tid]);
+            }
+            if (jac) ++sweeps;
+            const float4 d = pll_scan(cl, sh, pb, crank, csize);
+            // ---- update the start state ------------------------------------
+            float4 mx = make_float4(0.f, 0.f, 0.f, 0.f);
+            bad = false;
+            if (t0 < t1) {
+                mx = make_float4(fabsf(d.x), fabsf(d.y), fabsf(d.z), fabsf(d.w));
+                bad = !(mx.x <= kTolPhase && mx.y <= kTolFreq && mx.z <= kTolIQ && mx.w <= kTolIQ);
+                pll_move(x0, d, start.df, reach);
+            }
+            if (lane == 0) sh.first[warp] = x0;
+            if (tid == 0 && crank > 0) *cl.map_shared_rank(&sh.next, crank - 1) = x0;
+            // ---- convergence, agreed by every CTA of the cluster -----------
+            // (magnitudes compare as their bits, a NaN above all numbers)
+            mx = pll_warp_max(mx);
+            if (lane < csize) cl.map_shared_rank(&sh.dmax[pb][0], lane)[crank * kNW + warp] = mx;
+            cl.sync();  // also publishes the start states for the next iteration's reads
+            mx = lane < csize * kNW ? sh.dmax[pb][lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (lane + 32 < csize * kNW) {
+                const float4 v = sh.dmax[pb][lane + 32];
+                mx = make_float4(pll_max(mx.x, v.x), pll_max(mx.y, v.y), pll_max(mx.z, v.z), pll_max(mx.w, v.w));
+            }
+            mx = pll_warp_max(mx);
+            pb ^= 1;
+            converged = mx.x <= kTolPhase && mx.y <= kTolFreq && mx.z <= kTolIQ && mx.w <= kTolIQ;
+            // Accepted one iteration early when the next correction is predicted
+            // below the tolerance: corrections shrinking at least linearly at rate
+            // m0 / prev_m0 leave a next one of m0^2 / prev_m0 (Newton's quadratic
+            // rate leaves less), with the other components already near their floor.
+            if (!converged && it >= 1 && mx.x <= 1e-5f && mx.x * mx.x <= kTolPhase * prev_m0 && mx.y <= 1e-10f &&
+                mx.z <= 1e-6f && mx.w <= 1e-6f)
+                converged = true;
+            // Or when the corrections no longer shrink and are below the rounding of
+            // a step's angle: unlocked loops, where I and Q pass near zero, stay
+            // there (2e-8 to 2e-7 rad) and would take every iteration allowed.
+            if (!converged && mx.x <= kTolAngle && mx.x > 0.25f * prev_m0 && mx.y <= 1e-10f && mx.z <= 1e-6f &&
+                mx.w <= 1e-6f)
+                converged = true;
+            if (it + 1 >= kPllQuasi) quasi = false;
+            prev_m0 = mx.x;
+        }
+        iters = max(iters, it);
+        // ---- not converged: the longest consistent prefix is kept ----------
+        // Segments before the first one whose start still moved by more than the
+        // tolerance form a consistent trajectory from the chunk start, and that
+        // segment's updated start is its exact start; one warp continues the
+        // serial loop from there to the chunk end.
+        int gstar = INT_MAX;
+        if (!converged) {
+            int v = bad ? g : INT_MAX;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, off));
+            if (lane == 0) sh.badw[warp] = v;
+            __syncthreads();
+            if (tid == 0) {
+                int c = INT_MAX;
+                for (int w2 = 0; w2 < kNW; ++w2) c = min(c, sh.badw[w2]);
+                sh.cbad = c;
+            }
+            cl.sync();
+            for (int r = 0; r < csize; ++r) gstar = min(gstar, *cl.map_shared_rank(&sh.cbad, r));
+            if (gstar == INT_MAX) gstar = 0;  // no start moved past the tolerance in the last iteration
+        }
+        // ---- outputs: each converged segment again from its start ----------
+        PllRun x = pll_begin(x0.dphi, x0.df, x0.I, x0.Q);
+        if (t0 < t1) {
+            for (int t = t0; t < t1; ++t) {
+                const double pt = (double)sh.seg[t - t0][tid];
+                pp += pt * pt;
+            }
+            if (g < gstar) {
+                uint64_t qr = k.q0 + (uint64_t)t0 * k.qf;
+                float p = sh.seg[0][tid];
+#pragma unroll 2
+                for (int t = t0; t < t1; ++t) {
+                    const float pn = sh.seg[min(t - t0 + 1, kPllSeg - 1)][tid];  // one step ahead
+                    PllEval o;
+                    pll_step<false>(qr, x, p, k, o);
+                    qr += k.qf;
+                    es += fabs((double)o.e);
+                    sh.seg[t - t0][tid] = pll_twice(qr, x.dphi);  // this thread's own cell, already read
+                    p = pn;
+                }
+            }
+        }
+        // the L-R products of this CTA's output segments, coalesced, eight
+        // loads in flight per thread
         __syncthreads();
-        for (int t = cbase + (int)threadIdx.x; t < cend; t += kNewtonThreads) {
-            const int r = t - cbase;
-            if (crank * kNewtonThreads + r / S < gstar) lr[t] = bpf[t] * s_seg[r % S][r / S];
+        const int cout = gstar == INT_MAX ? cend : min(cend, c0 + gstar * kPllSeg);
+#pragma unroll
+        for (int h = 0; h < kPllSeg; h += 8) {
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int t = cbase + tid + (h + i) * kNewtonThreads;
+                v[i] = t < cout ? __ldg(bpf + t) : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int r = tid + (h + i) * kNewtonThreads, t = cbase + r;
+                if (t < cout) lr[t] = v[i] * (2.0f * sinpif(sh.seg[r % kPllSeg][r / kPllSeg]));
+            }
+        }
+        // the owner of the chunk's end: the thread holding the last segment, or
+        // the warp of the thread at the first inconsistent segment start
+        const int owner = converged ? nseg - 1 : gstar;
+        if (!converged && (g >> 5) == (owner >> 5)) {
+            // Serial loop from the exact start of segment gstar to the chunk
+            // end, by the owner's whole warp: the lanes load the pilot band and
+            // the L-R band of the next 32 steps (coalesced, one chunk ahead), all
+            // of them evaluate the same recurrence (uniform values, so the loop
+            // never waits on a load), and lane i keeps step i's L-R product for
+            // one coalesced store per 32 steps.
+            const int ol = owner & 31;
+            PllRun xs = pll_begin(__shfl_sync(0xffffffffu, x.dphi, ol), __shfl_sync(0xffffffffu, x.df, ol),
+                                  __shfl_sync(0xffffffffu, x.I, ol), __shfl_sync(0xffffffffu, x.Q, ol));
+            const int ts = __shfl_sync(0xffffffffu, t0, ol), te = c0 + nc;
+            double es_w = __shfl_sync(0xffffffffu, es, ol);
+            uint64_t qr = k.q0 + (uint64_t)ts * k.qf;
+            float pcur = ts + lane < te ? __ldg(pil + ts + lane) : 0.f;
+            float bcur = ts + lane < te ? __ldg(bpf + ts + lane) : 0.f;
+            for (int s0 = ts; s0 < te; s0 += 32) {
+                const int sn = s0 + 32;
+                const float pnext = sn + lane < te ? __ldg(pil + sn + lane) : 0.f;
+                const float bnext = sn + lane < te ? __ldg(bpf + sn + lane) : 0.f;
+                const int cnt = min(32, te - s0);  // uniform in the warp
+                float mine = 0.f;
+#pragma unroll 4
+                for (int i = 0; i < cnt; ++i) {
+                    const float pt = __shfl_sync(0xffffffffu, pcur, i);
+                    PllEval o;
+                    if (i % kPllSeg == 0) xs = pll_begin(xs.dphi, xs.df, xs.I, xs.Q);
+                    pll_step<false>(qr, xs, pt, k, o);
+                    qr += k.qf;
+                    es_w += fabs((double)o.e);
+                    const float th = pll_twice(qr, xs.dphi);
+                    if (lane == i) mine = th;
+                }
+                if (lane < cnt) lr[s0 + lane] = bcur * (2.0f * sinpif(mine));
+                pcur = pnext;
+                bcur = bnext;
+            }
+            if (lane == ol) {
+                x = xs;
+                es = es_w;
+            }
+        }
+        if (g == owner)
+            for (int r = 0; r < csize; ++r) *cl.map_shared_rank(&sh.end, r) = SegState{x.dphi, x.df, x.I, x.Q};
+        all_converged = all_converged && converged;
+        locked = converged && it <= kPllOnce;
+        if (c0 + kPllChunkSteps < n) {
+            cl.sync();  // the end state is everywhere
+            start = sh.end;
         }
     }
 #pragma unroll
@@ -1936,78 +2204,25 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
         pp += __shfl_xor_sync(0xffffffffu, pp, off);
     }
     if (lane == 0) {
-        s_sum[warp][0] = es;
-        s_sum[warp][1] = pp;
+        double *q = cl.map_shared_rank(&sh.sum[0][0], 0) + 2 * (crank * kNW + warp);
+        q[0] = es;
+        q[1] = pp;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    cl.sync();  // CTA 0 has the end state and every warp's sums; no shared memory of another CTA is touched after this
+    if (g != 0) return;
+    double es_all = 0.0, pp_all = 0.0;
+    for (int r = 0; r < csize; ++r) {
         double a = 0, b = 0;
         for (int w2 = 0; w2 < kNW; ++w2) {
-            a += s_sum[w2][0];
-            b += s_sum[w2][1];
+            a += sh.sum[r * kNW + w2][0];
+            b += sh.sum[r * kNW + w2][1];
         }
-        s_csum[0] = a;
-        s_csum[1] = b;
+        es_all += a;
+        pp_all += b;
     }
-    cl.sync();
-    // the owner finishes the block: the thread holding the last segment, or
-    // the thread at the first inconsistent segment start
-    const int owner = converged ? (n - 1) / S : gstar;
-    double es_all = 0.0, pp_all = 0.0;
-    if (g == owner) {
-        for (int r = 0; r < csize; ++r) {
-            const double *rs = cl.map_shared_rank(&s_csum[0], r);
-            es_all += rs[0];
-            pp_all += rs[1];
-        }
-    }
-    cl.sync();  // no shared memory of another CTA is read after this
-    if (converged) {
-        if (g != owner) return;
-        pll_finish(s, cp, n, pll_phase_at(k, n, x.dphi), s.pll_freq + x.df, (double)x.I, (double)x.Q, es_all,
-                   pp_all);
-        s.pll_path = 1;
-        s.pll_iters = iters;
-        return;
-    }
-    // Serial loop from the exact start of segment gstar to the block end, by
-    // the owner's whole warp: the lanes load the pilot band and the L-R band of
-    // the next 32 steps (coalesced, one chunk ahead), all of them evaluate the
-    // same recurrence (uniform values, so the loop never waits on a load), and
-    // lane i keeps step i's L-R product for one coalesced store per chunk.
-    if ((g >> 5) != (owner >> 5)) return;
-    const int ol = owner & 31;
-    SegState xs{__shfl_sync(0xffffffffu, x.dphi, ol), __shfl_sync(0xffffffffu, x.df, ol),
-                __shfl_sync(0xffffffffu, x.I, ol), __shfl_sync(0xffffffffu, x.Q, ol)};
-    const int ts = __shfl_sync(0xffffffffu, t0, ol);
-    double es_w = __shfl_sync(0xffffffffu, es_all, ol);
-    uint64_t qr = k.q0 + (uint64_t)ts * k.qf;
-    float pcur = ts + lane < n ? __ldg(pil + ts + lane) : 0.f;
-    float bcur = ts + lane < n ? bpf[ts + lane] : 0.f;
-    for (int c0 = ts; c0 < n; c0 += 32) {
-        const int cn = c0 + 32;
-        const float pnext = cn + lane < n ? __ldg(pil + cn + lane) : 0.f;
-        const float bnext = cn + lane < n ? bpf[cn + lane] : 0.f;
-        const int cnt = min(32, n - c0);  // uniform in the warp
-        float mine = 0.f;
-#pragma unroll 4
-        for (int i = 0; i < cnt; ++i) {
-            const float pt = __shfl_sync(0xffffffffu, pcur, i);
-            PllEval o;
-            pll_step<false>(qr, xs.dphi, xs.df, xs.I, xs.Q, pt, k, o);
-            qr += k.qf;
-            xs = SegState{o.dphi1, o.df1, o.I1, o.Q1};
-            es_w += fabs((double)o.e);
-            const float th = pll_two_sin2(qr, xs.dphi);
-            if (lane == i) mine = bcur * th;
-        }
-        if (lane < cnt) lr[c0 + lane] = mine;
-        pcur = pnext;
-        bcur = bnext;
-    }
-    if (lane != ol) return;
-    pll_finish(s, cp, n, pll_phase_at(k, n, xs.dphi), s.pll_freq + xs.df, (double)xs.I, (double)xs.Q, es_w, pp_all);
-    s.pll_path = 2;
+    const SegState xe = sh.end;
+    pll_finish(s, cp, n, pll_phase_at(k, n, xe.dphi), s.pll_freq + xe.df, (double)xe.I, (double)xe.Q, es_all, pp_all);
+    s.pll_path = all_converged ? 1 : 2;
     s.pll_iters = iters;
 }
 
