@@ -272,6 +272,97 @@ __global__ void __launch_bounds__(256) lk_poly_accum(PolyArgs a, const float *__
     out[j] = make_float2(ar, ai);
 }
 
+// The same sums from shared memory: a CTA stages the samples of OT consecutive
+// outputs, each once, as polyphase rows Z[p][c] = s(newest_0 + (c-L+1) D - p)
+// (rotated on the way in where asked), so that lane j reads Z[p][j + L-1-k]:
+// consecutive words for consecutive outputs.  One thread keeps one output and
+// adds its taps in the order of lk_poly_accum (bit-identical).  lk_poly_accum
+// waited on one global load a tap (257 taps, 10240 outputs: 40 us; now 10); the
+// 256 threads stage with four loads in flight each, and the chain of
+// multiply-adds of the OT output threads is the bound.  OT = 64 spreads the
+// few outputs of a call over the SMs; calls that fill them anyway take 256 and
+// stage fewer samples twice.
+constexpr int kPolyThreads = 256;
+
+__global__ void __launch_bounds__(kPolyThreads) lk_poly_tile(PolyArgs a, const float *__restrict__ taps, int D, int L,
+                                                             int Lu, int P, int num_taps, int start_idx, int n_out,
+                                                             int OT, int Mp, float2 *__restrict__ out) {
+    extern __shared__ float2 Z[];  // P rows of pitch Mp, then the taps P x Lu
+    float *st = reinterpret_cast<float *>(Z + P * Mp);
+    const int t = threadIdx.x;
+    const int j0 = blockIdx.x * OT, M = OT + Lu - 1;
+    for (int i = t; i < P * Lu; i += kPolyThreads) {
+        const int p = i / Lu, k = i - p * Lu;
+        st[i] = taps[p * L + k];
+    }
+    // sample e = c*D - p + (D-1) of the tile, e = 0 .. M*D-1: index base + e of
+    // the concatenation, which is block sample base + e - H or history
+    const int base = a.H + start_idx + (j0 - Lu + 1) * D - (D - 1);
+    int c = t / D, r = t - (t / D) * D;
+    const int dc = kPolyThreads / D, dr = kPolyThreads - dc * D;
+    constexpr int U = 4;
+    for (int e0 = t; e0 < M * D; e0 += U * kPolyThreads) {
+        float2 v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int e = e0 + u * kPolyThreads, i = base + e, q = i - a.H;
+            v[u] = make_float2(0.f, 0.f);
+            if (e < M * D && i >= 0 && q < a.n_new) v[u] = q >= 0 ? a.newv[q] : a.hist[i];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int e = e0 + u * kPolyThreads, q = base + e - a.H, p = D - 1 - r;
+            if (e < M * D && p < P)
+                Z[p * Mp + c] = a.rotate && q >= 0 ? cmulf(v[u], q64_phasor(a.u0 + (uint64_t)q * a.inc)) : v[u];
+            c += dc;
+            r += dr;
+            if (r >= D) {
+                r -= D;
+                ++c;
+            }
+        }
+    }
+    __syncthreads();
+    const int j = j0 + t;
+    if (t >= OT || j >= n_out) return;
+    float ar = 0.f, ai = 0.f;
+    for (int p = 0; p < P; ++p) {
+        const float2 *z = Z + p * Mp + t + Lu - 1;
+        const float *h = st + p * Lu;
+        const int kn = (num_taps - p + D - 1) / D;  // taps with p + k*D < num_taps
+#pragma unroll 4
+        for (int k = 0; k < kn; ++k) {
+            const float2 v = z[-k];
+            ar = fmaf(h[k], v.x, ar);
+            ai = fmaf(h[k], v.y, ai);
+        }
+    }
+    out[j] = make_float2(ar, ai);
+}
+
+// Outputs of the concatenation a: the tile kernel where its rows fit in shared
+// memory (decimations up to ~800) and most samples of the span meet a tap, the
+// gather kernel beyond.
+static cudaError_t launch_poly(const PolyArgs &a, const float *taps, int D, int L, int num_taps, int start_idx,
+                               int n_out, float2 *out) {
+    const int Lu = (num_taps + D - 1) / D, P = num_taps < D ? num_taps : D;
+    for (int OT : {256, 64, 32}) {
+        if (D > 4 * P) break;  // few taps far apart: most of the span would be walked for nothing
+        if (OT == 256 && n_out < 2 * 148 * 256) continue;
+        const int Mp = (OT + Lu - 1) | 1;
+        const long long smem = (long long)P * Mp * sizeof(float2) + (long long)P * Lu * sizeof(float);
+        if (smem > (OT == 32 ? 220 : 100) * 1024) continue;
+        static std::atomic<uint64_t> optin{0};
+        cudaError_t e = smem_optin_once(optin, (const void *)lk_poly_tile, 220 * 1024);
+        if (e != cudaSuccess) return e;
+        lk_poly_tile<<<(n_out + OT - 1) / OT, kPolyThreads, (size_t)smem>>>(a, taps, D, L, Lu, P, num_taps, start_idx,
+                                                                          n_out, OT, Mp, out);
+        return cudaGetLastError();
+    }
+    lk_poly_accum<<<(n_out + 255) / 256, 256>>>(a, taps, D, L, num_taps, start_idx, n_out, out);
+    return cudaGetLastError();
+}
+
 __global__ void __launch_bounds__(256) lk_history_tail(PolyArgs a, int keep, float2 *__restrict__ dst) {
     int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= keep) return;
@@ -298,10 +389,8 @@ extern "C" GPUD_API int GPUD_CALL gpud_launch_streaming_polyphase_prepare_cuda(
                rad_to_q64(phase_inc)};
     if (out_count > 0) {
         if (!out) return -4;
-        lk_poly_accum<<<(out_count + 255) / 256, 256>>>(a, polyphase_taps, decim, L, num_taps, decim - pc - 1,
-                                                       out_count, (float2 *)out);
+        cudaError_t e = launch_poly(a, polyphase_taps, decim, L, num_taps, decim - pc - 1, out_count, (float2 *)out);
         gpud_count_launch(1);
-        cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return (int)e;
     }
     if (history_out && keep > 0) {
@@ -318,6 +407,12 @@ extern "C" GPUD_API int GPUD_CALL gpud_launch_streaming_polyphase_prepare_cuda(
     if (phase_end_out)
         *phase_end_out = q64_to_rad(rad_to_q64(phase_start) + (uint64_t)n_new * rad_to_q64(phase_inc));
     return 0;
+}
+
+// Whether na samples at a and nb samples at b share no byte.
+static bool poly_apart(const gpud_float2 *a, int na, const gpud_float2 *b, int nb) {
+    const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+    return x + (uintptr_t)na * sizeof(gpud_float2) <= y || y + (uintptr_t)nb * sizeof(gpud_float2) <= x;
 }
 
 extern "C" GPUD_API int GPUD_CALL gpud_launch_streaming_polyphase_stateful_cuda(
@@ -340,41 +435,44 @@ extern "C" GPUD_API int GPUD_CALL gpud_launch_streaming_polyphase_stateful_cuda(
     if (pc >= decim) pc %= decim;
     const double phase_start = *phase_state;
     const uint64_t u0 = rad_to_q64(phase_start), inc = rad_to_q64(phase_inc);
+    const int newH = history_cap > 0 ? (H + n_new < history_cap ? H + n_new : history_cap) : 0;
+    // The samples are rotated as they are read, and a history that lies whole
+    // in the new block is written in place: no shifted copy, no staging.  A
+    // caller whose outputs or history overlap the block gets the separate
+    // steps, in which the block has been read before anything is written.
+    const bool fused = poly_apart(in_new, n_new, out, out_cap) && poly_apart(in_new, n_new, history_state, newH);
     if (n_new > 0) {
         if (!in_new || !shifted_new_tmp) return -13;
-        lk_freq_shift<<<grid_for(n_new, 256), 256>>>((const float2 *)in_new, (float2 *)shifted_new_tmp, n_new, u0,
-                                                     inc);
-        gpud_count_launch(1);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return (int)e;
+        if (!fused) {
+            lk_freq_shift<<<grid_for(n_new, 256), 256>>>((const float2 *)in_new, (float2 *)shifted_new_tmp, n_new, u0,
+                                                         inc);
+            gpud_count_launch(1);
+            cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) return (int)e;
+        }
     }
     const int total = pc + n_new;
     const int out_count = total / decim;
     if (out_count > out_cap) return -14;
-    PolyArgs a{(const float2 *)history_state, H, (const float2 *)shifted_new_tmp, n_new, false, 0, 0};
+    const PolyArgs a{(const float2 *)history_state, H, (const float2 *)(fused ? in_new : shifted_new_tmp), n_new, fused,
+                     u0, inc};
     if (out_count > 0) {
         if (!out) return -15;
-        lk_poly_accum<<<(out_count + 255) / 256, 256>>>(a, polyphase_taps, decim, L, num_taps, decim - pc - 1,
-                                                       out_count, (float2 *)out);
+        cudaError_t e = launch_poly(a, polyphase_taps, decim, L, num_taps, decim - pc - 1, out_count, (float2 *)out);
+        gpud_count_launch(1);
+        if (e != cudaSuccess) return (int)e;
+    }
+    if (newH > 0) {
+        if (!history_state || !history_scratch) return -16;
+        const bool in_place = fused && n_new >= newH;  // no sample of the old history is kept
+        lk_history_tail<<<(newH + 255) / 256, 256>>>(a, newH, (float2 *)(in_place ? history_state : history_scratch));
         gpud_count_launch(1);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return (int)e;
-    }
-    int newH = H;
-    if (history_cap > 0) {
-        newH = H + n_new;
-        if (newH > history_cap) newH = history_cap;
-        if (newH > 0) {
-            if (!history_state || !history_scratch) return -16;
-            lk_history_tail<<<(newH + 255) / 256, 256>>>(a, newH, (float2 *)history_scratch);
-            gpud_count_launch(1);
-            cudaError_t e = cudaGetLastError();
-            if (e != cudaSuccess) return (int)e;
+        if (!in_place) {
             e = cudaMemcpy(history_state, history_scratch, (size_t)newH * sizeof(float2), cudaMemcpyDeviceToDevice);
             if (e != cudaSuccess) return (int)e;
         }
-    } else {
-        newH = 0;
     }
     *history_len_io = newH;
     *phase_count_state = total % decim;
