@@ -10,19 +10,36 @@
 // Every analysis frequency f is a multiple of 10 Hz, so exp(-j 2 pi f i / fs)
 // repeats with period P = fs / gcd(fs, 10) in i.  The discriminator output is
 // folded modulo P once (y[m] = sum of d[m + pP]) and the 201 bins are direct
-// float64 DFT sums of y over [0, P) with twiddles from a table of the P-th
-// roots of unity (exact sincospi arguments): the Goertzel magnitudes without
-// the Goertzel recurrence's error growth, one CTA per (job, bin), and the
-// max / median decision on the device.
+// float64 DFT sums of y over [0, P): the Goertzel magnitudes without the
+// Goertzel recurrence's error growth.
+//
+// y is real, so a window of at least one period folds once more: with
+// s[m] = y[m] + y[P-m] and d[m] = y[m] - y[P-m] the real part of a bin is the
+// sum of s cos and its imaginary part the sum of d sin over m <= P/2.
+//
+// The bins of all stations of one rate are a matrix product, (201 x 2) x P/2
+// twiddles times P/2 x stations samples, and float64 multiply-adds are its bound
+// (40 stations at 312.5 kS/s: 0.25 G, 14 us at the chip's rate).  k_pilot_bins
+// gives every CTA a contiguous share of m for all bins and up to 40 stations:
+// a thread keeps 7 bins x (cos, sin) x SPT stations in registers and reads 7
+// twiddles and SPT samples from shared memory for 14 SPT multiply-adds.  The
+// CTA copies its operands 16 m's ahead with asynchronous copies, the twiddles
+// from a table of the P-th roots of unity (rotating 16 from one sincospi instead
+// was as fast but doubled the error, 6e-15 -> 1e-14); periods beyond the table
+// take a sincospi per term.  (One CTA per station and bin, each thread walking
+// its own run of y: 1045 us.)  k_pilot_decide adds the CTAs' shares in
+// order and takes the max / median decision.
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
 #include <numeric>
+#include <tuple>
 #include <vector>
 
 #include <cuda_runtime.h>
 
 #include "../../include/gpudemod.h"
+#include "gpud_internal.cuh"
 
 extern "C" void gpud_count_launch(int n);
 
@@ -31,16 +48,30 @@ namespace {
 constexpr int kBins = 201;
 constexpr int kPilotThreads = 256;
 constexpr int64_t kMaxTable = 1 << 20;  // roots-of-unity table entries (16 MiB)
+constexpr int kChunk = 16;        // m's per staged chunk
+constexpr int kBinsPT = 7;        // bins per thread: 4 warps x 8 lanes x 7 >= 201
+constexpr int kStGroups = 8;      // station groups of a CTA: 2 warp rows x 4 lane groups
+constexpr int kMaxSpt = 5;        // stations per thread
+constexpr int kMaxSt = kStGroups * kMaxSpt;  // stations per pass
 
 struct PilotJob {
     const float2 *iq;  // first sample of the analysed window
     int32_t nd;        // discriminator samples (window length - 1)
-    int32_t fs;
     int32_t period;    // P = fs / gcd(fs, 10)
-    int32_t folded;    // min(P, nd)
-    int32_t fstep;     // 10 / gcd(fs, 10): table index step per 10 Hz of frequency
-    int32_t table;     // 1: twiddles from the table, 0: sincospi per term
+    int32_t folded;    // terms of a bin: P/2 + 1 pairs (s, d) of a whole period, else the nd samples
+    int32_t paired;
+    int32_t nshare;    // CTAs of its pass
+    int32_t column;    // its column in the pass
+    int32_t ncol;      // columns of the pass
+    int64_t part_off;  // its pass's partial sums
     int64_t y_off;     // offset of this job's folded vector
+};
+
+// Stations of one rate whose bins one launch computes: jobs first..first+count-1.
+struct PilotPass {
+    int first, count, period, folded, paired, fstep, spt;
+    int64_t part_off;  // double2 offset of its partial sums [share][column][bin]
+    int nshare;
 };
 
 // fmDemod (pll.go:170-183): float64 products of the float32 samples, atan2.
@@ -51,15 +82,32 @@ __device__ __forceinline__ double pilot_disc(const float2 *iq, int i) {
     return atan2(num, den);
 }
 
+__device__ __forceinline__ double pilot_folded(const PilotJob &jb, int m) {
+    double acc = 0.0;
+    for (int i = m; i < jb.nd; i += jb.period) acc += pilot_disc(jb.iq, i);
+    return acc;
+}
+
 __global__ void __launch_bounds__(kPilotThreads)
 k_pilot_fold(const PilotJob *__restrict__ jobs, double *__restrict__ y) {
     const PilotJob jb = jobs[blockIdx.y];
     for (int m = blockIdx.x * kPilotThreads + threadIdx.x; m < jb.folded; m += gridDim.x * kPilotThreads) {
-        double acc = 0.0;
-        for (int i = m; i < jb.nd; i += jb.period) acc += pilot_disc(jb.iq, i);
-        y[jb.y_off + m] = acc;
+        const double a = pilot_folded(jb, m);
+        if (!jb.paired) {
+            y[jb.y_off + m] = a;
+        } else {
+            const int o = jb.period - m;
+            const double b = m > 0 && o != m ? pilot_folded(jb, o) : 0.0;
+            reinterpret_cast<double2 *>(y + jb.y_off)[m] = make_double2(a + b, a - b);
+        }
     }
 }
+
+// Shared memory of a CTA, both halves of a double buffer: twiddles | samples.
+struct PilotStage {
+    double2 w[2][kChunk][32 * kBinsPT];
+    double2 y[2][kChunk][kMaxSt];  // (s, d); the first alone where not paired
+};
 
 // tab[a] = exp(j 2 pi a / P), a < P
 __global__ void k_pilot_table(int P, double2 *__restrict__ tab) {
@@ -70,80 +118,182 @@ __global__ void k_pilot_table(int P, double2 *__restrict__ tab) {
     }
 }
 
+// Asynchronous copy of 8 or 16 bytes global -> shared, zeros where !ok.
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void *dst, const void *src, bool ok) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(gpud::smem_u32(dst)), "l"(src), "n"(BYTES),
+                 "r"(ok ? BYTES : 0)
+                 : "memory");
+}
+
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Partial DFT sums of a pass: CTA b takes m in its share of [0, folded), and
+// writes re + j im of every (bin, station) to part[b][station][bin].  While the
+// warps multiply one chunk the copies of the next are under way: one barrier a
+// chunk.
+template <int SPT, bool PAIRED>
 __global__ void __launch_bounds__(kPilotThreads)
-k_pilot_bins(const PilotJob *__restrict__ jobs, const double *__restrict__ y, const double2 *__restrict__ tab,
-             double *__restrict__ mags) {
-    __shared__ double s_re[kPilotThreads / 32], s_im[kPilotThreads / 32];
-    const PilotJob jb = jobs[blockIdx.y];
-    const int bin = blockIdx.x;
-    const int64_t fq = (int64_t)(1800 + bin) * jb.fstep;  // f / gcd(fs, 10), f = 18000 + 10*bin
-    const int P = jb.period;
-    const int per = (jb.folded + kPilotThreads - 1) / kPilotThreads;
-    const int m0 = min(jb.folded, (int)threadIdx.x * per), m1 = min(jb.folded, m0 + per);
-    const double *ym = y + jb.y_off;
-    double re = 0.0, im = 0.0;
-    if (m0 < m1) {
-        int64_t a = (fq * (int64_t)m0) % P;  // index of exp(j 2 pi f m / fs) among the P-th roots
-        for (int m = m0; m < m1; ++m) {
-            double2 w;
-            if (jb.table) {
-                w = tab[a];
-            } else {
-                double s, c;
-                sincospi(2.0 * (double)a / (double)P, &s, &c);
-                w = make_double2(c, s);
+k_pilot_bins(const PilotJob *__restrict__ jobs, int count, int P, int folded, int fstep, const double *__restrict__ y,
+             const double2 *__restrict__ tab, double2 *__restrict__ part) {
+    constexpr int NS = kStGroups * SPT;
+    constexpr int NL = (kChunk * NS + kPilotThreads - 1) / kPilotThreads;  // samples a thread fetches
+    extern __shared__ __align__(16) unsigned char psm[];
+    PilotStage &sm = *reinterpret_cast<PilotStage *>(psm);
+    const int t = (int)threadIdx.x, lane = t & 31, warp = t >> 5;
+    // a warp takes 8 bins x 4 station groups at a time: both operands are
+    // broadcast to the lanes that share them
+    const int bin0 = (warp & 3) * (8 * kBinsPT) + (lane & 7), grp = (warp >> 2) * 4 + (lane >> 3);
+    const int m0 = (int)((int64_t)folded * blockIdx.x / gridDim.x);
+    const int m1 = (int)((int64_t)folded * (blockIdx.x + 1) / gridDim.x);
+    double re[kBinsPT][SPT], im[kBinsPT][SPT];
+#pragma unroll
+    for (int b = 0; b < kBinsPT; ++b)
+#pragma unroll
+        for (int s = 0; s < SPT; ++s) re[b][s] = im[b][s] = 0.0;
+    // thread t's twiddles: bin t; f / gcd(fs, 10) = (1800 + bin) * fstep
+    const int64_t fq = ((int64_t)(1800 + t) * fstep) % P;
+    // its samples of a chunk: consecutive threads on consecutive samples of a station
+    const double *src[NL];
+    int end[NL];
+#pragma unroll
+    for (int u = 0; u < NL; ++u) {
+        const int st = (t + u * kPilotThreads) / kChunk;
+        src[u] = st < count ? y + jobs[st].y_off : y;
+        end[u] = st < count ? min(m1, jobs[st].folded) : 0;
+    }
+    auto stage = [&](int buf, int mc) {
+#pragma unroll
+        for (int u = 0; u < NL; ++u) {
+            const int i = t + u * kPilotThreads, m = mc + i % kChunk;
+            if (i >= kChunk * NS) continue;
+            const int k = min(m, m1 - 1);
+            if (PAIRED)
+                copy_async<16>(&sm.y[buf][i % kChunk][i / kChunk], src[u] + 2 * (int64_t)k, m < end[u]);
+            else
+                copy_async<8>(&sm.y[buf][i % kChunk][i / kChunk], src[u] + k, m < end[u]);
+        }
+        if (t < kBins) {
+            int64_t a = (fq * (int64_t)mc) % P;
+#pragma unroll 4
+            for (int i = 0; i < kChunk; ++i) {
+                if (tab) {
+                    copy_async<16>(&sm.w[buf][i][t], tab + a, true);
+                } else {
+                    double s, c;
+                    sincospi(2.0 * (double)a / (double)P, &s, &c);
+                    sm.w[buf][i][t] = make_double2(c, s);
+                }
+                a += fq;
+                if (a >= P) a -= P;
             }
-            re = fma(ym[m], w.x, re);
-            im = fma(ym[m], w.y, im);
-            a += fq;
-            if (a >= P) a -= P;
         }
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-        re += __shfl_xor_sync(0xffffffffu, re, off);
-        im += __shfl_xor_sync(0xffffffffu, im, off);
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) {
-        s_re[warp] = re;
-        s_im[warp] = im;
-    }
+    };
+    if (m0 < m1) stage(0, m0);
+    copies_wait();
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double r = 0.0, i = 0.0;
-        for (int w = 0; w < kPilotThreads / 32; ++w) {
-            r += s_re[w];
-            i += s_im[w];
+    int buf = 0;
+    for (int mc = m0; mc < m1; mc += kChunk, buf ^= 1) {
+        if (mc + kChunk < m1) stage(buf ^ 1, mc + kChunk);
+        for (int i = 0; i < kChunk; ++i) {  // samples past the share are zero
+            double2 v[SPT];
+#pragma unroll
+            for (int s = 0; s < SPT; ++s) {
+                v[s] = sm.y[buf][i][grp * SPT + s];
+                if (!PAIRED) v[s].y = v[s].x;
+            }
+#pragma unroll
+            for (int b = 0; b < kBinsPT; ++b) {
+                const double2 w = sm.w[buf][i][bin0 + 8 * b];
+#pragma unroll
+                for (int s = 0; s < SPT; ++s) {
+                    re[b][s] = fma(v[s].x, w.x, re[b][s]);
+                    im[b][s] = fma(v[s].y, w.y, im[b][s]);
+                }
+            }
         }
-        mags[(int64_t)blockIdx.y * kBins + bin] = sqrt(r * r + i * i);
+        copies_wait();
+        __syncthreads();
+    }
+    double2 *out = part + (int64_t)blockIdx.x * kBins * count;
+#pragma unroll
+    for (int b = 0; b < kBinsPT; ++b) {
+        const int bin = bin0 + 8 * b;
+#pragma unroll
+        for (int s = 0; s < SPT; ++s) {
+            const int st = grp * SPT + s;
+            if (bin < kBins && st < count) out[st * kBins + bin] = make_double2(re[b][s], im[b][s]);
+        }
     }
 }
 
 // max (first occurrence, as the reference's strict '>' scan from 0) and the
 // median (element 100 of the sorted 201) of each job's magnitudes
-__global__ void __launch_bounds__(kPilotThreads)
-k_pilot_decide(const double *__restrict__ mags, double threshold, gpud_pilot_result *__restrict__ out) {
-    __shared__ double s_m[kBins], s_sorted[kBins];
-    const double *m = mags + (int64_t)blockIdx.x * kBins;
-    for (int i = threadIdx.x; i < kBins; i += kPilotThreads) s_m[i] = m[i];
+// s += v with the rounding error kept in e (Knuth's two-sum): the shares of a
+// bin far below the station's programme are large and cancel.
+__device__ __forceinline__ void add_exact(double &s, double &e, double v) {
+    const double t = s + v, z = t - s;
+    e += (s - (t - z)) + (v - z);
+    s = t;
+}
+
+constexpr int kDecideParts = 4;  // thread groups that add a bin's shares and rank it
+
+__global__ void __launch_bounds__(kDecideParts * kPilotThreads)
+k_pilot_decide(const PilotJob *__restrict__ jobs, const double2 *__restrict__ part, double threshold,
+               gpud_pilot_result *__restrict__ out) {
+    __shared__ double2 s_p[kDecideParts][kBins];
+    __shared__ double s_m[kBins], s_med;
+    __shared__ unsigned long long s_best;
+    __shared__ int s_rank[kBins], s_bin;
+    const PilotJob jb = jobs[blockIdx.x];
+    const int i = threadIdx.x % kPilotThreads, q = threadIdx.x / kPilotThreads;
+    if (threadIdx.x == 0) {
+        s_best = 0ull;
+        s_bin = kBins;
+    }
+    if (i < kBins) {
+        const double2 *p = part + jb.part_off + (int64_t)jb.column * kBins + i;
+        double re = 0.0, im = 0.0, er = 0.0, ei = 0.0;
+#pragma unroll 8
+        for (int k = q; k < jb.nshare; k += kDecideParts) {
+            const double2 v = p[(int64_t)k * kBins * jb.ncol];
+            add_exact(re, er, v.x);
+            add_exact(im, ei, v.y);
+        }
+        s_p[q][i] = make_double2(re + er, im + ei);
+    }
     __syncthreads();
-    for (int i = threadIdx.x; i < kBins; i += kPilotThreads) {
+    if (q == 0 && i < kBins) {
+        double re = 0.0, im = 0.0, er = 0.0, ei = 0.0;
+        for (int k = 0; k < kDecideParts; ++k) {
+            add_exact(re, er, s_p[k][i].x);
+            add_exact(im, ei, s_p[k][i].y);
+        }
+        re += er;
+        im += ei;
+        s_m[i] = sqrt(re * re + im * im);
+        s_rank[i] = 0;
+    }
+    __syncthreads();
+    if (i < kBins) {
+        const double mi = s_m[i];
         int rank = 0;
-        for (int j = 0; j < kBins; ++j) rank += (s_m[j] < s_m[i]) || (s_m[j] == s_m[i] && j < i);
-        s_sorted[rank] = s_m[i];
+        for (int j = q; j < kBins; j += kDecideParts) rank += (s_m[j] < mi) || (s_m[j] == mi && j < i);
+        atomicAdd(&s_rank[i], rank);
+        // magnitudes are not negative: they order as their bits
+        if (q == 0 && mi > 0.0) atomicMax(&s_best, (unsigned long long)__double_as_longlong(mi));
+    }
+    __syncthreads();
+    if (q == 0 && i < kBins) {
+        if (s_rank[i] == kBins / 2) s_med = s_m[i];
+        if (s_m[i] > 0.0 && (unsigned long long)__double_as_longlong(s_m[i]) == s_best) atomicMin(&s_bin, i);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double best = 0.0;
-        int bb = -1;
-        for (int i = 0; i < kBins; ++i)
-            if (s_m[i] > best) {
-                best = s_m[i];
-                bb = i;
-            }
-        const double med = s_sorted[kBins / 2];
+        const double best = __longlong_as_double((long long)s_best), med = s_med;
         gpud_pilot_result r{};
-        r.best_bin = bb < 0 ? 100 : bb;
+        r.best_bin = s_bin == kBins ? 100 : s_bin;
         r.best_hz = 18000.0 + 10.0 * (double)r.best_bin;
         r.median = med;
         r.ratio = med > 0 ? best / med : 0.0;
@@ -152,28 +302,63 @@ k_pilot_decide(const double *__restrict__ mags, double threshold, gpud_pilot_res
     }
 }
 
+template <int SPT, bool PAIRED>
+cudaError_t launch_pilot_bins_as(const PilotPass &ps, cudaStream_t s, const PilotJob *jobs, const double *y,
+                                 const double2 *tab, double2 *part) {
+    static std::atomic<uint64_t> optin{0};
+    cudaError_t e = gpud::smem_optin_once(optin, (const void *)k_pilot_bins<SPT, PAIRED>, (int)sizeof(PilotStage));
+    if (e != cudaSuccess) return e;
+    k_pilot_bins<SPT, PAIRED><<<ps.nshare, kPilotThreads, sizeof(PilotStage), s>>>(
+        jobs + ps.first, ps.count, ps.period, ps.folded, ps.fstep, y, tab, part + ps.part_off);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_pilot_bins(const PilotPass &ps, cudaStream_t s, const PilotJob *jobs, const double *y,
+                              const double2 *tab, double2 *part) {
+    switch (2 * ps.spt + ps.paired) {
+#define GPUD_CASE(N)                                                              \
+    case 2 * N: return launch_pilot_bins_as<N, false>(ps, s, jobs, y, tab, part); \
+    case 2 * N + 1: return launch_pilot_bins_as<N, true>(ps, s, jobs, y, tab, part);
+        GPUD_CASE(1) GPUD_CASE(2) GPUD_CASE(3) GPUD_CASE(4) GPUD_CASE(5)
+#undef GPUD_CASE
+    default: return cudaErrorInvalidValue;
+    }
+}
+
 }  // namespace
 
 struct gpud_pilot {
-    int max_jobs = 0, max_samples = 0;
-    double *d_y = nullptr, *d_mags = nullptr;
-    double2 *d_tab = nullptr;
-    int tab_period = 0;  // period the table currently holds
+    int max_jobs = 0, max_samples = 0, num_sms = 148;
+    double *d_y = nullptr;
+    double2 *d_part = nullptr;  // partial sums: num_sms x 201 per job
+    double2 *d_tab = nullptr;   // roots of unity of the last pass's period
+    int tab_period = 0;
     PilotJob *d_jobs = nullptr;
     gpud_pilot_result *d_res = nullptr;
     std::vector<PilotJob> jobs;
+    std::vector<int> fstep;        // per device job
+    std::vector<PilotPass> passes;
     std::vector<int> job_of;  // job index -> index into the device list (-1: no decision possible)
 };
 
 extern "C" {
+
+// Folded values of a job: P/2 + 1 pairs with P below the window length, or the
+// window's samples; an even number, so that the pairs are aligned.
+static int64_t pilot_row(int max_samples) { return ((int64_t)max_samples + 3) & ~(int64_t)1; }
 
 GPUD_API int GPUD_CALL gpud_pilot_create(int max_jobs, int max_samples, gpud_pilot **out) {
     if (!out || max_jobs <= 0 || max_samples <= 1) return GPUD_E_ARG;
     auto *p = new gpud_pilot();
     p->max_jobs = max_jobs;
     p->max_samples = max_samples;
-    bool ok = cudaMalloc((void **)&p->d_y, sizeof(double) * (size_t)max_jobs * (size_t)max_samples) == cudaSuccess &&
-              cudaMalloc((void **)&p->d_mags, sizeof(double) * (size_t)max_jobs * kBins) == cudaSuccess &&
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
+        p->num_sms = sms;
+    bool ok = cudaMalloc((void **)&p->d_y, sizeof(double) * (size_t)max_jobs * (size_t)pilot_row(max_samples)) == cudaSuccess &&
+              cudaMalloc((void **)&p->d_part, sizeof(double2) * (size_t)max_jobs * kBins * (size_t)p->num_sms) ==
+                  cudaSuccess &&
               cudaMalloc((void **)&p->d_tab, sizeof(double2) * (size_t)kMaxTable) == cudaSuccess &&
               cudaMalloc((void **)&p->d_jobs, sizeof(PilotJob) * (size_t)max_jobs) == cudaSuccess &&
               cudaMalloc((void **)&p->d_res, sizeof(gpud_pilot_result) * (size_t)max_jobs) == cudaSuccess;
@@ -188,7 +373,7 @@ GPUD_API int GPUD_CALL gpud_pilot_create(int max_jobs, int max_samples, gpud_pil
 GPUD_API int GPUD_CALL gpud_pilot_destroy(gpud_pilot *p) {
     if (!p) return 0;
     cudaFree(p->d_y);
-    cudaFree(p->d_mags);
+    cudaFree(p->d_part);
     cudaFree(p->d_tab);
     cudaFree(p->d_jobs);
     cudaFree(p->d_res);
@@ -202,8 +387,8 @@ GPUD_API int GPUD_CALL gpud_pilot_run(gpud_pilot *p, const gpud_pilot_job *jobs,
     if (threshold <= 0) threshold = 4.0;
     cudaStream_t s = (cudaStream_t)stream;
     p->jobs.clear();
+    p->fstep.clear();
     p->job_of.assign((size_t)count, -1);
-    std::vector<int> periods;
     for (int j = 0; j < count; ++j) {
         const gpud_pilot_job &q = jobs[j];
         results[j] = gpud_pilot_result{};
@@ -224,55 +409,86 @@ GPUD_API int GPUD_CALL gpud_pilot_run(gpud_pilot *p, const gpud_pilot_job *jobs,
         const int g = std::gcd(q.sample_rate, 10);
         jb.iq = reinterpret_cast<const float2 *>(q.iq) + start;
         jb.nd = n - 1;
-        jb.fs = q.sample_rate;
         jb.period = q.sample_rate / g;
-        jb.folded = std::min(jb.period, jb.nd);
-        jb.fstep = 10 / g;
-        jb.table = jb.period <= kMaxTable ? 1 : 0;
-        jb.y_off = (int64_t)p->jobs.size() * p->max_samples;
+        jb.paired = jb.nd >= jb.period ? 1 : 0;
+        jb.folded = jb.paired ? jb.period / 2 + 1 : jb.nd;
+        jb.y_off = (int64_t)p->jobs.size() * pilot_row(p->max_samples);
         p->job_of[(size_t)j] = (int)p->jobs.size();
         p->jobs.push_back(jb);
-        if (jb.table) periods.push_back(jb.period);
+        p->fstep.push_back(10 / g);
     }
     const int nj = (int)p->jobs.size();
     if (nj == 0) return 0;
-    // one roots-of-unity table per call: jobs with another period use sincospi
-    int tp = 0;
-    if (!periods.empty()) {
-        std::sort(periods.begin(), periods.end());
-        int best = 0, cnt = 0;
-        for (size_t i = 0; i < periods.size(); ++i) {
-            cnt = (i > 0 && periods[i] == periods[i - 1]) ? cnt + 1 : 1;
-            if (cnt > best) {
-                best = cnt;
-                tp = periods[i];
-            }
-        }
+    // passes: the jobs of one rate (period, step, paired or not), at most kMaxSt
+    // of them at a time, side by side on the device
+    std::vector<int> order((size_t)nj);
+    std::iota(order.begin(), order.end(), 0);
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        const PilotJob &x = p->jobs[(size_t)a], &z = p->jobs[(size_t)b];
+        return std::make_tuple(x.period, p->fstep[(size_t)a], x.paired) <
+               std::make_tuple(z.period, p->fstep[(size_t)b], z.paired);
+    });
+    std::vector<PilotJob> sorted((size_t)nj);
+    std::vector<int> at((size_t)nj);
+    for (int k = 0; k < nj; ++k) {
+        sorted[(size_t)k] = p->jobs[(size_t)order[(size_t)k]];
+        at[(size_t)order[(size_t)k]] = k;
     }
-    for (auto &jb : p->jobs) jb.table = (jb.table && jb.period == tp) ? 1 : 0;
-    if (cudaMemcpyAsync(p->d_jobs, p->jobs.data(), sizeof(PilotJob) * (size_t)nj, cudaMemcpyHostToDevice, s) !=
+    p->passes.clear();
+    int64_t part = 0;
+    for (int k = 0; k < nj;) {
+        PilotPass ps{};
+        ps.first = k;
+        ps.period = sorted[(size_t)k].period;
+        ps.fstep = p->fstep[(size_t)order[(size_t)k]];
+        ps.paired = sorted[(size_t)k].paired;
+        while (k < nj && ps.count < kMaxSt && sorted[(size_t)k].period == ps.period &&
+               sorted[(size_t)k].paired == ps.paired &&
+               p->fstep[(size_t)order[(size_t)k]] == ps.fstep) {
+            ps.folded = std::max(ps.folded, sorted[(size_t)k].folded);
+            ++ps.count;
+            ++k;
+        }
+        ps.spt = (ps.count + kStGroups - 1) / kStGroups;
+        ps.nshare = std::max(1, std::min(p->num_sms, ps.folded / (2 * kChunk)));
+        ps.part_off = part;
+        for (int c = 0; c < ps.count; ++c) {
+            PilotJob &jb = sorted[(size_t)(ps.first + c)];
+            jb.nshare = ps.nshare;
+            jb.column = c;
+            jb.ncol = ps.count;
+            jb.part_off = part;
+        }
+        part += (int64_t)ps.nshare * kBins * ps.count;
+        p->passes.push_back(ps);
+    }
+    if (cudaMemcpyAsync(p->d_jobs, sorted.data(), sizeof(PilotJob) * (size_t)nj, cudaMemcpyHostToDevice, s) !=
         cudaSuccess)
         return GPUD_E_CUDA;
-    if (tp > 0 && tp != p->tab_period) {
-        k_pilot_table<<<(tp + 255) / 256 < 1024 ? (tp + 255) / 256 : 1024, 256, 0, s>>>(tp, p->d_tab);
-        gpud_count_launch(1);
-        p->tab_period = tp;
-    }
     int maxf = 0;
-    for (auto &jb : p->jobs) maxf = std::max(maxf, jb.folded);
+    for (auto &jb : sorted) maxf = std::max(maxf, jb.folded);
     dim3 gf((unsigned)std::min(1024, (maxf + kPilotThreads - 1) / kPilotThreads), (unsigned)nj);
     k_pilot_fold<<<gf, kPilotThreads, 0, s>>>(p->d_jobs, p->d_y);
-    k_pilot_bins<<<dim3(kBins, (unsigned)nj), kPilotThreads, 0, s>>>(p->d_jobs, p->d_y, p->d_tab, p->d_mags);
-    k_pilot_decide<<<nj, kPilotThreads, 0, s>>>(p->d_mags, threshold, p->d_res);
+    for (const PilotPass &ps : p->passes) {
+        const bool table = ps.period <= kMaxTable;
+        if (table && ps.period != p->tab_period) {  // the pass before has read the old one (stream order)
+            k_pilot_table<<<std::min(1024, (ps.period + 255) / 256), 256, 0, s>>>(ps.period, p->d_tab);
+            gpud_count_launch(1);
+            p->tab_period = ps.period;
+        }
+        if (launch_pilot_bins(ps, s, p->d_jobs, p->d_y, table ? p->d_tab : nullptr, p->d_part) != cudaSuccess)
+            return GPUD_E_CUDA;
+    }
+    k_pilot_decide<<<nj, kDecideParts * kPilotThreads, 0, s>>>(p->d_jobs, p->d_part, threshold, p->d_res);
     if (cudaGetLastError() != cudaSuccess) return GPUD_E_CUDA;
-    gpud_count_launch(3);
+    gpud_count_launch(2 + (int)p->passes.size());
     std::vector<gpud_pilot_result> tmp((size_t)nj);
     if (cudaMemcpyAsync(tmp.data(), p->d_res, sizeof(gpud_pilot_result) * (size_t)nj, cudaMemcpyDeviceToHost, s) !=
             cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return GPUD_E_CUDA;
     for (int j = 0; j < count; ++j)
-        if (p->job_of[(size_t)j] >= 0) results[j] = tmp[(size_t)p->job_of[(size_t)j]];
+        if (p->job_of[(size_t)j] >= 0) results[j] = tmp[(size_t)at[(size_t)p->job_of[(size_t)j]]];
     return 0;
 }
 
