@@ -77,6 +77,21 @@ __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
 
+// Two float32 multiply-adds in one instruction, each rounded as fmaf rounds it:
+// c + a*b by component.  The arithmetic rate is the scalar one (71.7 against
+// 71.3 TFLOP/s); the issue slots are half, which is what bounds the FIR kernels
+// (their multiply-adds compete with shared-memory loads for them).
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+    unsigned long long x, y, z, r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a.x), "f"(a.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(b.x), "f"(b.y));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(z) : "f"(c.x), "f"(c.y));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(r));
+    return d;
+}
+
 // ---------------------------------------------------------------------------
 // Per-slot constants
 // ---------------------------------------------------------------------------

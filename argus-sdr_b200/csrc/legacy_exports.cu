@@ -160,10 +160,10 @@ __global__ void __launch_bounds__(kLfThreads) lk_fir(const float2 *__restrict__ 
     __syncthreads();
     // output r of this thread takes tile sample b + r - k under tap k
     const int b = kLfR * t + halo;
-    float ar[kLfR], ai[kLfR];
+    float2 acc[kLfR];
     float2 ring[kLfR];  // ring[(r - k) & 7]: the sample of output r under tap k
 #pragma unroll
-    for (int r = 0; r < kLfR; ++r) ar[r] = ai[r] = 0.f;
+    for (int r = 0; r < kLfR; ++r) acc[r] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int r = 1; r < kLfR; ++r) ring[r] = sx[lf_slot(b + r)];
     int kb = 0;
@@ -174,9 +174,7 @@ __global__ void __launch_bounds__(kLfThreads) lk_fir(const float2 *__restrict__ 
             const float h = st[kb + kk];
 #pragma unroll
             for (int r = 0; r < kLfR; ++r) {
-                const float2 v = ring[(r - kk + kLfR) & 7];
-                ar[r] = fmaf(v.x, h, ar[r]);
-                ai[r] = fmaf(v.y, h, ai[r]);
+                acc[r] = ffma2(ring[(r - kk + kLfR) & 7], make_float2(h, h), acc[r]);
             }
         }
     }
@@ -187,15 +185,13 @@ __global__ void __launch_bounds__(kLfThreads) lk_fir(const float2 *__restrict__ 
         const float h = st[kb + kk];
 #pragma unroll
         for (int r = 0; r < kLfR; ++r) {
-            const float2 v = ring[(r - kk + kLfR) & 7];
-            ar[r] = fmaf(v.x, h, ar[r]);
-            ai[r] = fmaf(v.y, h, ai[r]);
+            acc[r] = ffma2(ring[(r - kk + kLfR) & 7], make_float2(h, h), acc[r]);
         }
     }
     // coalesced stores through the tile's slots (one slot every 8: no conflicts)
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kLfR; ++r) sx[lf_slot(kLfR * t + r)] = make_float2(ar[r], ai[r]);
+    for (int r = 0; r < kLfR; ++r) sx[lf_slot(kLfR * t + r)] = acc[r];
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < kLfR; ++r) {

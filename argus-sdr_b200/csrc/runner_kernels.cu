@@ -150,7 +150,7 @@ int dense_tile() { return kDenseOT; }
 
 // One phase row, L <= 16 taps: lane's R outputs from a window of R+L-1.
 template <int L>
-__device__ __forceinline__ void group_row(const float2 *zrow, const float *hrow, int lane, float *ar, float *ai) {
+__device__ __forceinline__ void group_row(const float2 *zrow, const float *hrow, int lane, float2 *acc) {
     constexpr int R = kDenseR;
     float2 win[R + L - 1];
 #pragma unroll
@@ -164,18 +164,13 @@ __device__ __forceinline__ void group_row(const float2 *zrow, const float *hrow,
 #pragma unroll
     for (int r = 0; r < R; ++r) {
 #pragma unroll
-        for (int u = 0; u < L; ++u) {
-            const float2 z = win[r + L - 1 - u];
-            ar[r] = fmaf(h[u], z.x, ar[r]);
-            ai[r] = fmaf(h[u], z.y, ai[r]);
-        }
+        for (int u = 0; u < L; ++u) acc[r] = ffma2(make_float2(h[u], h[u]), win[r + L - 1 - u], acc[r]);
     }
 }
 
 // One phase row, long arm (Le a multiple of 8 > 16): chunks of 8 taps with a
 // window of R+7 samples that slides 8 columns per chunk (8 new loads).
-__device__ __forceinline__ void group_row_long(const float2 *zrow, const float *hrow, int Le, int lane, float *ar,
-                                               float *ai) {
+__device__ __forceinline__ void group_row_long(const float2 *zrow, const float *hrow, int Le, int lane, float2 *acc) {
     constexpr int R = kDenseR;
     constexpr int W = R + 7;
     float2 win[W];
@@ -193,11 +188,7 @@ __device__ __forceinline__ void group_row_long(const float2 *zrow, const float *
 #pragma unroll
         for (int r = 0; r < R; ++r) {
 #pragma unroll
-            for (int v = 0; v < 8; ++v) {
-                const float2 z = win[r + 7 - v];
-                ar[r] = fmaf(h[v], z.x, ar[r]);
-                ai[r] = fmaf(h[v], z.y, ai[r]);
-            }
+            for (int v = 0; v < 8; ++v) acc[r] = ffma2(make_float2(h[v], h[v]), win[r + 7 - v], acc[r]);
         }
         if (ch + 1 < nc) {
 #pragma unroll
@@ -226,16 +217,16 @@ __device__ __forceinline__ void tile_sum(int rows, const Row &row, float2 *Z, co
     constexpr int R = kDenseR;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if constexpr (!PREC) {
-        float ar[R], ai[R];
+        float2 acc[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) ar[r] = ai[r] = 0.f;
-        for (int pp = warp; pp < rows; pp += 8) row(pp, lane, ar, ai);
+        for (int r = 0; r < R; ++r) acc[r] = make_float2(0.f, 0.f);
+        for (int pp = warp; pp < rows; pp += 8) row(pp, lane, acc);
         __syncthreads();
         float2 *red = Z + warp * kRedStride;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int o = lane * R + r;
-            red[o + (o >> 3)] = make_float2(ar[r], ai[r]);
+            red[o + (o >> 3)] = acc[r];
         }
         __syncthreads();
         for (int o = threadIdx.x; o < kDenseOT; o += kDenseThreads) {
@@ -253,14 +244,14 @@ __device__ __forceinline__ void tile_sum(int rows, const Row &row, float2 *Z, co
 #pragma unroll
         for (int r = 0; r < R; ++r) dr[r] = di[r] = 0.0;
         for (int pp = warp; pp < rows; pp += 8) {
-            float ar[R], ai[R];
+            float2 acc[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r) ar[r] = ai[r] = 0.f;
-            row(pp, lane, ar, ai);
+            for (int r = 0; r < R; ++r) acc[r] = make_float2(0.f, 0.f);
+            row(pp, lane, acc);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                dr[r] += (double)ar[r];
-                di[r] += (double)ai[r];
+                dr[r] += (double)acc[r].x;
+                di[r] += (double)acc[r].y;
             }
         }
         __syncthreads();
@@ -330,7 +321,7 @@ __device__ __forceinline__ void dense_tile(const int2 w, const SlotBlock &sb, co
     }
     __syncthreads();
 
-    auto row = [&](int p, int lane, float *ar, float *ai) { group_row<L>(Z + p * Mp, tsm + p * L, lane, ar, ai); };
+    auto row = [&](int p, int lane, float2 *acc) { group_row<L>(Z + p * Mp, tsm + p * L, lane, acc); };
     float2 *dst = ext + sb.ext_off + j0;
     const int nv = sb.n_out - j0;
     if (cp.precise_sum)
@@ -460,16 +451,16 @@ __device__ __forceinline__ void pipe_tile_sum(int rows, int gw, int lane, int gt
     constexpr int R = kDenseR;
     constexpr int GNT = 32 * GW;
     if constexpr (!PREC) {
-        float ar[R], ai[R];
+        float2 acc[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) ar[r] = ai[r] = 0.f;
-        for (int pp = gw; pp < rows; pp += GW) row(pp, lane, ar, ai);
+        for (int r = 0; r < R; ++r) acc[r] = make_float2(0.f, 0.f);
+        for (int pp = gw; pp < rows; pp += GW) row(pp, lane, acc);
         named_sync(bar, GNT);
         float2 *red = Z + gw * kRedStride;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int o = lane * R + r;
-            red[o + (o >> 3)] = make_float2(ar[r], ai[r]);
+            red[o + (o >> 3)] = acc[r];
         }
         named_sync(bar, GNT);
         for (int o = gt; o < kDenseOT; o += GNT) {
@@ -487,14 +478,14 @@ __device__ __forceinline__ void pipe_tile_sum(int rows, int gw, int lane, int gt
 #pragma unroll
         for (int r = 0; r < R; ++r) dr[r] = di[r] = 0.0;
         for (int pp = gw; pp < rows; pp += GW) {
-            float ar[R], ai[R];
+            float2 acc[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r) ar[r] = ai[r] = 0.f;
-            row(pp, lane, ar, ai);
+            for (int r = 0; r < R; ++r) acc[r] = make_float2(0.f, 0.f);
+            row(pp, lane, acc);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                dr[r] += (double)ar[r];
-                di[r] += (double)ai[r];
+                dr[r] += (double)acc[r].x;
+                di[r] += (double)acc[r].y;
             }
         }
         named_sync(bar, GNT);
@@ -683,7 +674,7 @@ k_extract_dense_pipe(const int2 *__restrict__ work, int ntiles, int pmax, const 
         if (gt == 0) mbar_arrive(empty);  // the raw span, the table and the descriptor may be refilled
 
         const float *hb = tsm + (it & 3) * lo.tstride;
-        auto row = [&](int p, int ln, float *ar, float *ai) { group_row<L>(Z + p * Mp, hb + p * L, ln, ar, ai); };
+        auto row = [&](int p, int ln, float2 *acc) { group_row<L>(Z + p * Mp, hb + p * L, ln, acc); };
         float2 *dst = ext + d.ext_off + d.j0;
         const int nv = d.n_out - d.j0;
         if (d.precise)
@@ -919,16 +910,16 @@ k_extract_group(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt
     const float2 *hist = hist_arena + cp.hist_off + sb.hist_sel * cp.hcap;
     const uint64_t u0 = st[sb.slot].nco_q;
 
-    auto row = [&](int pp, int lane, float *ar, float *ai) {
+    auto row = [&](int pp, int lane, float2 *acc) {
         const float2 *zrow = Z + pp * gt.Mp;
         const float *hrow = tsm + pp * gt.Le;
         switch (L) {
 #define GPUD_ROW(LL) \
-    case LL: group_row<LL>(zrow, hrow, lane, ar, ai); break;
+    case LL: group_row<LL>(zrow, hrow, lane, acc); break;
             GPUD_ROW(1) GPUD_ROW(2) GPUD_ROW(3) GPUD_ROW(4) GPUD_ROW(5) GPUD_ROW(6) GPUD_ROW(7) GPUD_ROW(8)
             GPUD_ROW(9) GPUD_ROW(10) GPUD_ROW(11) GPUD_ROW(12) GPUD_ROW(13) GPUD_ROW(14) GPUD_ROW(15) GPUD_ROW(16)
 #undef GPUD_ROW
-        default: group_row_long(zrow, hrow, gt.Le, lane, ar, ai); break;
+        default: group_row_long(zrow, hrow, gt.Le, lane, acc); break;
         }
     };
     const int nv = sb.n_out - gt.j0;
@@ -974,7 +965,7 @@ __host__ __device__ inline int mod_smem_bytes(int Pc, int L) {
 int mod_smem_bytes_host(int Pc, int L) { return mod_smem_bytes(Pc, L); }
 
 template <int L>
-__device__ __forceinline__ void mod_row(const float2 *zrow, const float2 *hrow, int lane, float *ar, float *ai) {
+__device__ __forceinline__ void mod_row(const float2 *zrow, const float2 *hrow, int lane, float2 *acc) {
     constexpr int R = kDenseR;
     float2 win[R + L - 1];
 #pragma unroll
@@ -990,8 +981,9 @@ __device__ __forceinline__ void mod_row(const float2 *zrow, const float2 *hrow, 
 #pragma unroll
         for (int u = 0; u < L; ++u) {
             const float2 z = win[r + L - 1 - u];
-            ar[r] = fmaf(h[u].x, z.x, fmaf(-h[u].y, z.y, ar[r]));
-            ai[r] = fmaf(h[u].x, z.y, fmaf(h[u].y, z.x, ai[r]));
+            // (packed multiply-adds spill at three CTAs per SM: 1955 -> 2051 us)
+            acc[r].x = fmaf(h[u].x, z.x, fmaf(-h[u].y, z.y, acc[r].x));
+            acc[r].y = fmaf(h[u].x, z.y, fmaf(h[u].y, z.x, acc[r].y));
         }
     }
 }
@@ -1020,14 +1012,14 @@ k_extract_mod(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, 
     const int s0 = D - sb.pc - 1;
     const float2 *hist = hist_arena + cp.hist_off + sb.hist_sel * cp.hcap;
     const int H = sb.hist_len;
-    auto row = [&](int pp, int lane, float *ar, float *ai) {
+    auto row = [&](int pp, int lane, float2 *acc) {
         const float2 *zrow = Z + pp * Mp;
         const float2 *hrow = hc + pp * L;
         switch (L) {
-        case 1: mod_row<1>(zrow, hrow, lane, ar, ai); break;
-        case 2: mod_row<2>(zrow, hrow, lane, ar, ai); break;
-        case 3: mod_row<3>(zrow, hrow, lane, ar, ai); break;
-        default: mod_row<4>(zrow, hrow, lane, ar, ai); break;
+        case 1: mod_row<1>(zrow, hrow, lane, acc); break;
+        case 2: mod_row<2>(zrow, hrow, lane, acc); break;
+        case 3: mod_row<3>(zrow, hrow, lane, acc); break;
+        default: mod_row<4>(zrow, hrow, lane, acc); break;
         }
     };
     const int nv = sb.n_out - j0;
@@ -1236,9 +1228,13 @@ k_wfm_fir(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, cons
     const int t = threadIdx.x;
     // window index of composite sample q0 + 8t + r - k is 8t + r - k + 104
     const int base = 8 * t + kWfmTapsPad;
-    float a[8], b[8], c[8], ring[8];
+    float2 ab[8];  // outputs of the first two filters
+    float c[8], ring[8];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) a[r] = b[r] = c[r] = 0.f;
+    for (int r = 0; r < 8; ++r) {
+        ab[r] = make_float2(0.f, 0.f);
+        c[r] = 0.f;
+    }
 #pragma unroll
     for (int j = 1; j < 8; ++j) ring[j] = win[padi(base + j)];
     for (int kb = 0; kb < kWfmTapsPad; kb += 8) {
@@ -1250,8 +1246,7 @@ k_wfm_fir(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, cons
 #pragma unroll
             for (int r = 0; r < 8; ++r) {
                 const float v = ring[(r - kk + 8) & 7];
-                a[r] = fmaf(h.x, v, a[r]);
-                b[r] = fmaf(h.y, v, b[r]);
+                ab[r] = ffma2(make_float2(h.x, h.y), make_float2(v, v), ab[r]);
                 c[r] = fmaf(h.z, v, c[r]);
             }
         }
@@ -1262,8 +1257,8 @@ k_wfm_fir(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, cons
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         const int i = 8 * t + r, j = i + (i >> 5);
-        s_out[j] = a[r];
-        s_out[kS + j] = b[r];
+        s_out[j] = ab[r].x;
+        s_out[kS + j] = ab[r].y;
         s_out[2 * kS + j] = c[r];
     }
     __syncthreads();
