@@ -39,6 +39,7 @@ int bank_warps() { return kBankThreads / 32; }
 __global__ void __launch_bounds__(256)
 k_bank_pack(const BankGroup *__restrict__ groups, const int *__restrict__ members, const SlotBlock *__restrict__ sbt,
             const ChanParams *__restrict__ prm, const float *__restrict__ taps_arena, float2 *__restrict__ gtab) {
+    dependency_wait();
     const BankGroup b = groups[blockIdx.y];
     const int total = b.T * b.cpad;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -62,6 +63,7 @@ k_extract_bank(const int2 *__restrict__ work, const BankGroup *__restrict__ grou
                const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
                const ChanState *__restrict__ st, const float2 *__restrict__ x, const float2 *__restrict__ gtab,
                float2 *__restrict__ ext) {
+    dependency_wait();
     extern __shared__ float4 bsm[];
     float4 *s_x = bsm;                                  // [kBankJ][kBankKC/2]: (x(n_o-k), x(n_o-k-1))
     float4 *s_g = bsm + kBankJ * (kBankKC / 2);         // [kBankKC/2][kBankLanes]: (g_c[k], g_c[k+1])
@@ -140,8 +142,8 @@ cudaError_t launch_bank_pack(int ngroups, int max_total, cudaStream_t sm, const 
                              const int *members, const SlotBlock *sbt, const ChanParams *prm, const float *taps,
                              float2 *gtab) {
     const int gx = std::min(64, (max_total + 255) / 256);
-    k_bank_pack<<<dim3(gx > 0 ? gx : 1, ngroups), 256, 0, sm>>>(groups, members, sbt, prm, taps, gtab);
-    return cudaGetLastError();
+    return launch_dependent(k_bank_pack, dim3(gx > 0 ? gx : 1, ngroups), 256, 0, sm, groups, members, sbt, prm, taps,
+                            gtab);
 }
 
 cudaError_t launch_extract_bank(int grid, cudaStream_t sm, const int2 *work, const BankGroup *groups,
@@ -150,8 +152,8 @@ cudaError_t launch_extract_bank(int grid, cudaStream_t sm, const int2 *work, con
     static std::atomic<uint64_t> optin{0};
     cudaError_t e = smem_optin_once(optin, (const void *)k_extract_bank, kBankSmem);
     if (e != cudaSuccess) return e;
-    k_extract_bank<<<grid, kBankThreads, kBankSmem, sm>>>(work, groups, members, sbt, prm, st, x, gtab, ext);
-    return cudaGetLastError();
+    return launch_dependent(k_extract_bank, dim3((unsigned)grid), kBankThreads, kBankSmem, sm, work,
+                            groups, members, sbt, prm, st, x, gtab, ext);
 }
 
 }  // namespace gpud

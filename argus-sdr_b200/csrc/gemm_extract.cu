@@ -145,6 +145,7 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 __global__ void __launch_bounds__(256)
 k_gemm_pack(const GemmGroup *__restrict__ groups, const int *__restrict__ members, const SlotBlock *__restrict__ sbt,
             const ChanParams *__restrict__ prm, const float *__restrict__ taps_arena, float *__restrict__ gb) {
+    dependency_wait();
     const GemmGroup g = groups[blockIdx.y];
     const int u = blockIdx.x;
     if (u >= g.L) return;
@@ -188,6 +189,7 @@ k_extract_gemm(const int2 *__restrict__ work, const GemmGroup *__restrict__ grou
                const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
                const ChanState *__restrict__ st, const float2 *__restrict__ x, int n, const float *__restrict__ gb,
                float2 *__restrict__ ext, unsigned *fault) {
+    dependency_wait();
     extern __shared__ __align__(1024) unsigned char gsm[];
     const int2 w = work[blockIdx.x];
     const GemmGroup g = groups[w.x];
@@ -432,8 +434,8 @@ k_extract_gemm(const int2 *__restrict__ work, const GemmGroup *__restrict__ grou
 
 cudaError_t launch_gemm_pack(int ngroups, int max_l, cudaStream_t sm, const GemmGroup *groups, const int *members,
                              const SlotBlock *sbt, const ChanParams *prm, const float *taps, float *gb) {
-    k_gemm_pack<<<dim3(max_l, ngroups, 8), 128, 0, sm>>>(groups, members, sbt, prm, taps, gb);
-    return cudaGetLastError();
+    return launch_dependent(k_gemm_pack, dim3(max_l, ngroups, 8), 128, 0, sm, groups, members, sbt, prm,
+                            taps, gb);
 }
 
 cudaError_t launch_extract_gemm(int grid, int smem, cudaStream_t sm, const int2 *work, const GemmGroup *groups,
@@ -442,8 +444,8 @@ cudaError_t launch_extract_gemm(int grid, int smem, cudaStream_t sm, const int2 
     static std::atomic<uint64_t> optin{0};
     cudaError_t e = smem_optin_once(optin, (const void *)k_extract_gemm, 220 * 1024);
     if (e != cudaSuccess) return e;
-    k_extract_gemm<<<grid, kGemmThreads, smem, sm>>>(work, groups, members, sbt, prm, st, x, n, gb, ext, fault);
-    return cudaGetLastError();
+    return launch_dependent(k_extract_gemm, dim3((unsigned)grid), kGemmThreads, (size_t)smem, sm, work, groups,
+                            members, sbt, prm, st, x, n, gb, ext, fault);
 }
 
 }  // namespace gpud

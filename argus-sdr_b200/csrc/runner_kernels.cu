@@ -340,6 +340,7 @@ k_extract_dense(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt
                 const ChanState *__restrict__ st, const float2 *__restrict__ x, int n,
                 const float2 *__restrict__ hist_arena, const float *__restrict__ taps_arena,
                 float2 *__restrict__ ext) {
+    dependency_wait();
     extern __shared__ float4 smem4[];
     const int2 w = work[blockIdx.x];
     const SlotBlock sb = sbt[w.x];
@@ -354,6 +355,7 @@ k_extract_dense_any(const int2 *__restrict__ work, const SlotBlock *__restrict__
                     const ChanParams *__restrict__ prm, const ChanState *__restrict__ st,
                     const float2 *__restrict__ x, int n, const float2 *__restrict__ hist_arena,
                     const float *__restrict__ taps_arena, float2 *__restrict__ ext) {
+    dependency_wait();
     extern __shared__ float4 smem4[];
     const int2 w = work[blockIdx.x];
     const SlotBlock sb = sbt[w.x];
@@ -516,6 +518,7 @@ k_extract_dense_pipe(const int2 *__restrict__ work, int ntiles, int pmax, const 
                      const ChanParams *__restrict__ prm, const ChanState *__restrict__ st,
                      const float2 *__restrict__ x, int n, const float2 *__restrict__ hist_arena,
                      const float *__restrict__ taps_arena, float2 *__restrict__ ext, unsigned *fault) {
+    dependency_wait();
     constexpr int GW = kPipeCW / NG;  // warps per consumer group
     constexpr int GNT = 32 * GW;      // threads per consumer group
     extern __shared__ __align__(128) unsigned char psm[];
@@ -705,6 +708,7 @@ k_extract_wide(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt,
                const ChanState *__restrict__ st, const float2 *__restrict__ x, int n,
                const float2 *__restrict__ hist_arena, const float *__restrict__ taps_arena,
                float2 *__restrict__ ext) {
+    dependency_wait();
     extern __shared__ float4 smemw4[];
     const int2 w = work[blockIdx.x];
     const SlotBlock sb = sbt[w.x];
@@ -890,6 +894,7 @@ k_extract_group(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt
                 const ChanState *__restrict__ st, const float2 *__restrict__ x, int n,
                 const float2 *__restrict__ hist_arena, const float *__restrict__ taps_arena,
                 float2 *__restrict__ ext) {
+    dependency_wait();
     extern __shared__ float4 smemg4[];
     const int2 w = work[blockIdx.x];
     const SlotBlock sb = sbt[w.x];
@@ -993,6 +998,7 @@ k_extract_mod(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, 
               const ChanState *__restrict__ st, const float2 *__restrict__ x, int n,
               const float2 *__restrict__ hist_arena, const float *__restrict__ taps_arena,
               float2 *__restrict__ ext) {
+    dependency_wait();
     extern __shared__ float4 smemm4[];
     const int2 w = work[blockIdx.x];
     const SlotBlock sb = sbt[w.x];
@@ -1084,6 +1090,7 @@ constexpr int kDecOT = 256;
 __global__ void __launch_bounds__(kDecOT)
 k_decim2(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
          const double *__restrict__ d1taps, const float2 *__restrict__ d1hist, float2 *__restrict__ ext) {
+    dependency_wait();
     const int2 w = work[blockIdx.x];
     const SlotBlock sb = sbt[w.x];
     const int j = w.y * kDecOT + (int)threadIdx.x;
@@ -1112,6 +1119,7 @@ __global__ void __launch_bounds__(256)
 k_demod(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
         const ChanState *__restrict__ st, const float2 *__restrict__ ext, float *__restrict__ comp,
         float *__restrict__ audio) {
+    dependency_wait();
     const int2 w = work[blockIdx.x];
     const SlotBlock sb = sbt[w.x];
     const ChanParams &cp = prm[sb.slot];
@@ -1150,6 +1158,7 @@ k_demod(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const 
 __global__ void __launch_bounds__(256)
 k_am(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const float2 *__restrict__ ext,
      float *__restrict__ audio) {
+    dependency_wait();
     __shared__ double red[256];
     const SlotBlock sb = sbt[work[blockIdx.x].x];
     const float2 *iq = ext + sb.dem_off;
@@ -1212,6 +1221,7 @@ __device__ __forceinline__ void stage_window(float *win, const float *__restrict
 __global__ void __launch_bounds__(kFirThreads)
 k_wfm_fir(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
           const WfmTaps *__restrict__ taps, float *__restrict__ wk, int W, const float *__restrict__ comp_dl) {
+    dependency_wait();
     __shared__ float win[padi(kFirOT + kWfmTapsPad) + 8];
     __shared__ float4 tp[kWfmTapsPad];
     __shared__ float s_out[3 * (kFirOT + kFirOT / 32)];
@@ -1484,6 +1494,7 @@ constexpr int kPllChunk = 2048;
 __global__ void __launch_bounds__(64)
 k_pll(const int *__restrict__ list, int count, const SlotBlock *__restrict__ sbt,
       const ChanParams *__restrict__ prm, ChanState *__restrict__ st, float *__restrict__ wk, int W) {
+    dependency_wait();
     __shared__ float s_pil[2][kPllChunk];
     __shared__ float s_th[2][kPllChunk];
     __shared__ double s_red[32];
@@ -1884,6 +1895,7 @@ __global__ void __launch_bounds__(kNewtonThreads, 3)
 k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restrict__ sbt,
              const ChanParams *__restrict__ prm, ChanState *__restrict__ st, float *__restrict__ wk, int W,
              int max_iters) {
+    dependency_wait();
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     __shared__ PllShared sh;
@@ -2226,6 +2238,7 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
 __global__ void __launch_bounds__(256)
 k_comp_power(const int *__restrict__ list, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
              ChanState *__restrict__ st, const float *__restrict__ wk) {
+    dependency_wait();
     __shared__ double red[256];
     const SlotBlock sb = sbt[list[blockIdx.x]];
     const ChanParams &cp = prm[sb.slot];
@@ -2249,6 +2262,7 @@ k_comp_power(const int *__restrict__ list, const SlotBlock *__restrict__ sbt, co
 __global__ void __launch_bounds__(256)
 k_free_stereo(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
               const BinadeTable *__restrict__ tabs38, float *__restrict__ wk, int W) {
+    dependency_wait();
     const int2 w = work[blockIdx.x];
     const SlotBlock sb = sbt[w.x];
     const ChanParams &cp = prm[sb.slot];
@@ -2267,6 +2281,7 @@ __global__ void __launch_bounds__(kFirThreads)
 k_wfm_out(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
           const ChanState *__restrict__ st, const WfmTaps *__restrict__ taps, const float *__restrict__ wk, int W,
           const float *__restrict__ lr_dl, const float *__restrict__ audio_dl, float *__restrict__ audio) {
+    dependency_wait();
     __shared__ float win[padi(kFirOT + kWfmTapsPad) + 8];
     __shared__ float tp[kWfmTapsPad];
     __shared__ float s_out[kFirOT + kFirOT / 32];
@@ -2373,6 +2388,7 @@ __global__ void __launch_bounds__(kRdsThreads)
 k_rds(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
       const ChanState *__restrict__ st, const WfmTaps *__restrict__ taps, const BinadeTable *__restrict__ tabs,
       const float *__restrict__ wk, const float2 *__restrict__ rds_dl, float2 *__restrict__ rds_out) {
+    dependency_wait();
     extern __shared__ float2 cpl[];
     const int2 w = work[blockIdx.x];
     const SlotBlock sb = sbt[w.x];
@@ -2459,6 +2475,7 @@ k_post_front(const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ p
              const float2 *__restrict__ ext, const float *__restrict__ wk, float *__restrict__ comp_dl,
              float2 *__restrict__ rds_dl, const BinadeTable *__restrict__ tabs, float2 *__restrict__ d1hist,
              DevResult *__restrict__ res) {
+    dependency_wait();
     const SlotBlock sb = sbt[blockIdx.x];
     const ChanParams &cp = prm[sb.slot];
     ChanState &s = st[sb.slot];
@@ -2521,6 +2538,7 @@ k_post_front(const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ p
 __global__ void __launch_bounds__(128)
 k_post_extract(const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm, ChanState *__restrict__ st,
                const float2 *__restrict__ x, int n, float2 *__restrict__ hist_arena, DevResult *__restrict__ res) {
+    dependency_wait();
     const SlotBlock sb = sbt[blockIdx.x];
     const ChanParams &cp = prm[sb.slot];
     ChanState &s = st[sb.slot];
@@ -2547,6 +2565,7 @@ __global__ void __launch_bounds__(128)
 k_post_back(const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm, ChanState *__restrict__ st,
             const float *__restrict__ wk, int W, float *__restrict__ lr_dl, float *__restrict__ audio_dl,
             DevResult *__restrict__ res) {
+    dependency_wait();
     const SlotBlock sb = sbt[blockIdx.x];
     const ChanParams &cp = prm[sb.slot];
     ChanState &s = st[sb.slot];
@@ -2600,6 +2619,7 @@ __global__ void __launch_bounds__(kAudThreads)
 k_audio48_rs(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
              const RsBank *__restrict__ banks, const AudState *__restrict__ aud, const float *__restrict__ audio,
              float *__restrict__ rs_out) {
+    dependency_wait();
     extern __shared__ double s_aud[];  // bank (L*K doubles) | inputs 2 x kAudWin floats
     const int2 w = work[blockIdx.x];
     const SlotBlock sb = sbt[w.x];
@@ -2697,6 +2717,7 @@ __global__ void __launch_bounds__(kAudOutThreads)
 k_audio48_out(const int *__restrict__ list, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
               const RsBank *__restrict__ banks, AudState *__restrict__ aud, const float *__restrict__ audio,
               const float *__restrict__ rs_out, int16_t *__restrict__ pcm) {
+    dependency_wait();
     constexpr int kWarps = kAudOutThreads / 32;
     __shared__ double s_wa[kWarps], s_wb[2][kWarps];  // warp totals, then exclusive warp prefixes
     extern __shared__ float s_rs[];  // the channel's resampled block (when it fits), then its output samples
@@ -2844,8 +2865,8 @@ static cudaError_t launch_dense_L(int grid, int smem, cudaStream_t sm, const int
     static std::atomic<uint64_t> optin{0};
     cudaError_t e = smem_optin_once(optin, (const void *)k_extract_dense<L>, 220 * 1024);
     if (e != cudaSuccess) return e;
-    k_extract_dense<L><<<grid, kDenseThreads, smem, sm>>>(work, sbt, prm, st, x, n, hist, taps, ext);
-    return cudaGetLastError();
+    return launch_dependent(k_extract_dense<L>, dim3((unsigned)grid), kDenseThreads, (size_t)smem, sm, work, sbt,
+                            prm, st, x, n, hist, taps, ext);
 }
 
 cudaError_t launch_extract_dense_any(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
@@ -2854,8 +2875,8 @@ cudaError_t launch_extract_dense_any(int grid, int smem, cudaStream_t sm, const 
     static std::atomic<uint64_t> optin{0};
     cudaError_t e = smem_optin_once(optin, (const void *)k_extract_dense_any, 220 * 1024);
     if (e != cudaSuccess) return e;
-    k_extract_dense_any<<<grid, kDenseThreads, smem, sm>>>(work, sbt, prm, st, x, n, hist, taps, ext);
-    return cudaGetLastError();
+    return launch_dependent(k_extract_dense_any, dim3((unsigned)grid), kDenseThreads, (size_t)smem, sm, work, sbt,
+                            prm, st, x, n, hist, taps, ext);
 }
 
 cudaError_t launch_extract_dense(int L, int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
@@ -2881,9 +2902,8 @@ static cudaError_t launch_dense_pipe_LG(int ntiles, int grid, int pmax, cudaStre
     cudaError_t e = smem_optin_once(optin, (const void *)k_extract_dense_pipe<L, NG>, 220 * 1024);
     if (e != cudaSuccess) return e;
     const int smem = pipe_layout(pmax, L, NG).bytes;
-    k_extract_dense_pipe<L, NG><<<grid, kPipeThreads, smem, sm>>>(work, ntiles, pmax, sbt, prm, st, x, n, hist,
-                                                                  taps, ext, fault);
-    return cudaGetLastError();
+    return launch_dependent(k_extract_dense_pipe<L, NG>, dim3((unsigned)grid), kPipeThreads, (size_t)smem, sm,
+                            work, ntiles, pmax, sbt, prm, st, x, n, hist, taps, ext, fault);
 }
 
 // Consumer groups of the pipelined dense form for a class whose channels have
@@ -2924,8 +2944,8 @@ cudaError_t launch_extract_wide(int grid, int smem, cudaStream_t sm, const int2 
     static std::atomic<uint64_t> optin{0};
     cudaError_t e = smem_optin_once(optin, (const void *)k_extract_wide, 64 * 1024);
     if (e != cudaSuccess) return e;
-    k_extract_wide<<<grid, 256, smem, sm>>>(work, sbt, prm, st, x, n, hist, taps, ext);
-    return cudaGetLastError();
+    return launch_dependent(k_extract_wide, dim3((unsigned)grid), 256, (size_t)smem, sm, work, sbt, prm, st, x, n,
+                            hist, taps, ext);
 }
 
 cudaError_t launch_extract_group(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
@@ -2934,8 +2954,8 @@ cudaError_t launch_extract_group(int grid, int smem, cudaStream_t sm, const int2
     static std::atomic<uint64_t> optin{0};
     cudaError_t e = smem_optin_once(optin, (const void *)k_extract_group, 220 * 1024);
     if (e != cudaSuccess) return e;
-    k_extract_group<<<grid, kDenseThreads, smem, sm>>>(work, sbt, prm, st, x, n, hist, taps, ext);
-    return cudaGetLastError();
+    return launch_dependent(k_extract_group, dim3((unsigned)grid), kDenseThreads, (size_t)smem, sm, work, sbt, prm,
+                            st, x, n, hist, taps, ext);
 }
 
 cudaError_t launch_extract_mod(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
@@ -2944,20 +2964,18 @@ cudaError_t launch_extract_mod(int grid, int smem, cudaStream_t sm, const int2 *
     static std::atomic<uint64_t> optin{0};
     cudaError_t e = smem_optin_once(optin, (const void *)k_extract_mod, 220 * 1024);
     if (e != cudaSuccess) return e;
-    k_extract_mod<<<grid, kDenseThreads, smem, sm>>>(work, sbt, prm, st, x, n, hist, taps, ext);
-    return cudaGetLastError();
+    return launch_dependent(k_extract_mod, dim3((unsigned)grid), kDenseThreads, (size_t)smem, sm, work, sbt, prm,
+                            st, x, n, hist, taps, ext);
 }
 
 cudaError_t launch_comp_power(int count, cudaStream_t sm, const int *list, const SlotBlock *sbt,
                               const ChanParams *prm, ChanState *st, const float *wk) {
-    k_comp_power<<<count, 256, 0, sm>>>(list, sbt, prm, st, wk);
-    return cudaGetLastError();
+    return launch_dependent(k_comp_power, dim3((unsigned)count), 256, 0, sm, list, sbt, prm, st, wk);
 }
 
 cudaError_t launch_free_stereo(int grid, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
                                const ChanParams *prm, const BinadeTable *tabs38, float *wk, int W) {
-    k_free_stereo<<<grid, 256, 0, sm>>>(work, sbt, prm, tabs38, wk, W);
-    return cudaGetLastError();
+    return launch_dependent(k_free_stereo, dim3((unsigned)grid), 256, 0, sm, work, sbt, prm, tabs38, wk, W);
 }
 
 // Second decimation of the one-shot segment demod (recorder/cpu_audio.go:
@@ -2988,26 +3006,24 @@ cudaError_t launch_seg_aa(cudaStream_t sm, const float *in, int C, const double 
 
 cudaError_t launch_demod(int grid, cudaStream_t sm, const int2 *work, const SlotBlock *sbt, const ChanParams *prm,
                          const ChanState *st, const float2 *ext, float *comp, float *audio) {
-    k_demod<<<grid, 256, 0, sm>>>(work, sbt, prm, st, ext, comp, audio);
-    return cudaGetLastError();
+    return launch_dependent(k_demod, dim3((unsigned)grid), 256, 0, sm, work, sbt, prm, st, ext, comp,
+                            audio);
 }
 
 cudaError_t launch_am(int grid, cudaStream_t sm, const int2 *work, const SlotBlock *sbt, const float2 *ext,
                       float *audio) {
-    k_am<<<grid, 256, 0, sm>>>(work, sbt, ext, audio);
-    return cudaGetLastError();
+    return launch_dependent(k_am, dim3((unsigned)grid), 256, 0, sm, work, sbt, ext, audio);
 }
 
 cudaError_t launch_wfm_fir(int grid, cudaStream_t sm, const int2 *work, const SlotBlock *sbt, const ChanParams *prm,
                            const WfmTaps *taps, float *wk, int W, const float *comp_dl) {
-    k_wfm_fir<<<grid, kFirThreads, 0, sm>>>(work, sbt, prm, taps, wk, W, comp_dl);
-    return cudaGetLastError();
+    return launch_dependent(k_wfm_fir, dim3((unsigned)grid), kFirThreads, 0, sm, work, sbt, prm, taps, wk,
+                            W, comp_dl);
 }
 
 cudaError_t launch_pll(int count, cudaStream_t sm, const int *list, const SlotBlock *sbt, const ChanParams *prm,
                        ChanState *st, float *wk, int W) {
-    k_pll<<<count, 64, 0, sm>>>(list, count, sbt, prm, st, wk, W);
-    return cudaGetLastError();
+    return launch_dependent(k_pll, dim3((unsigned)count), 64, 0, sm, list, count, sbt, prm, st, wk, W);
 }
 
 cudaError_t launch_pll_newton(int count, int cluster, cudaStream_t sm, const int *list, const SlotBlock *sbt,
@@ -3017,13 +3033,15 @@ cudaError_t launch_pll_newton(int count, int cluster, cudaStream_t sm, const int
     cfg.blockDim = dim3(kNewtonThreads, 1, 1);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = sm;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)cluster;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, k_pll_newton, list, count, sbt, prm, st, wk, W, max_iters);
 }
 
@@ -3032,21 +3050,21 @@ int pll_newton_threads() { return kNewtonThreads; }
 cudaError_t launch_wfm_out(int grid, cudaStream_t sm, const int2 *work, const SlotBlock *sbt, const ChanParams *prm,
                            const ChanState *st, const WfmTaps *taps, const float *wk, int W, const float *lr_dl,
                            const float *audio_dl, float *audio) {
-    k_wfm_out<<<grid, kFirThreads, 0, sm>>>(work, sbt, prm, st, taps, wk, W, lr_dl, audio_dl, audio);
-    return cudaGetLastError();
+    return launch_dependent(k_wfm_out, dim3((unsigned)grid), kFirThreads, 0, sm, work, sbt, prm, st, taps,
+                            wk, W, lr_dl, audio_dl, audio);
 }
 
 cudaError_t launch_rds(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
                        const ChanParams *prm, const ChanState *st, const WfmTaps *taps, const BinadeTable *tabs,
                        const float *wk, const float2 *rds_dl, float2 *rds_out) {
-    k_rds<<<grid, kRdsThreads, smem, sm>>>(work, sbt, prm, st, taps, tabs, wk, rds_dl, rds_out);
-    return cudaGetLastError();
+    return launch_dependent(k_rds, dim3((unsigned)grid), kRdsThreads, (size_t)smem, sm, work, sbt, prm, st, taps,
+                            tabs, wk, rds_dl, rds_out);
 }
 
 cudaError_t launch_decim2(int grid, cudaStream_t sm, const int2 *work, const SlotBlock *sbt, const ChanParams *prm,
                           const double *d1taps, const float2 *d1hist, float2 *ext) {
-    k_decim2<<<grid, kDecOT, 0, sm>>>(work, sbt, prm, d1taps, d1hist, ext);
-    return cudaGetLastError();
+    return launch_dependent(k_decim2, dim3((unsigned)grid), kDecOT, 0, sm, work, sbt, prm, d1taps, d1hist,
+                            ext);
 }
 
 int decim2_tile() { return kDecOT; }
@@ -3054,8 +3072,8 @@ int decim2_tile() { return kDecOT; }
 cudaError_t launch_post_front(int grid, cudaStream_t sm, const SlotBlock *sbt, const ChanParams *prm, ChanState *st,
                               const float2 *ext, const float *wk, float *comp_dl, float2 *rds_dl,
                               const BinadeTable *tabs, float2 *d1hist, DevResult *res) {
-    k_post_front<<<grid, 128, 0, sm>>>(sbt, prm, st, ext, wk, comp_dl, rds_dl, tabs, d1hist, res);
-    return cudaGetLastError();
+    return launch_dependent(k_post_front, dim3((unsigned)grid), 128, 0, sm, sbt, prm, st, ext, wk, comp_dl,
+                            rds_dl, tabs, d1hist, res);
 }
 
 cudaError_t launch_audio48(int grid_rs, int count, cudaStream_t sm, const int2 *work, const int *list,
@@ -3065,26 +3083,29 @@ cudaError_t launch_audio48(int grid_rs, int count, cudaStream_t sm, const int2 *
     static std::atomic<uint64_t> optin{0};  // 64 KiB of dynamic shared memory needs the opt-in
     cudaError_t e = smem_optin_once(optin, (const void *)k_audio48_rs, smem);
     if (e != cudaSuccess) return e;
-    if (grid_rs > 0) k_audio48_rs<<<grid_rs, kAudThreads, smem, sm>>>(work, sbt, prm, banks, aud, audio, rs_buf);
+    if (grid_rs > 0)
+        e = launch_dependent(k_audio48_rs, dim3((unsigned)grid_rs), kAudThreads, (size_t)smem, sm, work, sbt, prm, banks,
+                             aud, audio, rs_buf);
+    if (e != cudaSuccess) return e;
     static std::atomic<uint64_t> optin_out{0};
     e = smem_optin_once(optin_out, (const void *)k_audio48_out, kAudOutStage * 4);
     if (e != cudaSuccess) return e;
-    k_audio48_out<<<count, kAudOutThreads, kAudOutStage * 4, sm>>>(list, sbt, prm, banks, aud, audio, rs_buf, pcm);
-    return cudaGetLastError();
+    return launch_dependent(k_audio48_out, dim3((unsigned)count), kAudOutThreads, kAudOutStage * 4, sm,
+                            list, sbt, prm, banks, aud, audio, rs_buf, pcm);
 }
 
 int audio48_tile() { return kAudOT; }
 
 cudaError_t launch_post_extract(int grid, cudaStream_t sm, const SlotBlock *sbt, const ChanParams *prm, ChanState *st,
                                 const float2 *x, int n, float2 *hist, DevResult *res) {
-    k_post_extract<<<grid, 128, 0, sm>>>(sbt, prm, st, x, n, hist, res);
-    return cudaGetLastError();
+    return launch_dependent(k_post_extract, dim3((unsigned)grid), 128, 0, sm, sbt, prm, st, x, n, hist,
+                            res);
 }
 
 cudaError_t launch_post_back(int grid, cudaStream_t sm, const SlotBlock *sbt, const ChanParams *prm, ChanState *st,
                              const float *wk, int W, float *lr_dl, float *audio_dl, DevResult *res) {
-    k_post_back<<<grid, 128, 0, sm>>>(sbt, prm, st, wk, W, lr_dl, audio_dl, res);
-    return cudaGetLastError();
+    return launch_dependent(k_post_back, dim3((unsigned)grid), 128, 0, sm, sbt, prm, st, wk, W, lr_dl,
+                            audio_dl, res);
 }
 
 int rds_smem_bytes(int dr) {
