@@ -1510,19 +1510,31 @@ static int enqueue_block(gpud_runner *r, Frame &f, const Frame *prev, BlockPlan 
         CK(launch_wfm_fir((int)pl.w_fir.size(), f.s, d_w + o_fir, d_sb, r->d_prm, wt, f.d_wk, W, r->d_comp_dl));
         nl++;
     }
+    // The RDS baseband and the front half's state carry read nothing the back
+    // half writes: with a pilot loop in the block, whose few CTAs leave most of
+    // the GPU free, they run beside it on the side stream, and the frame stream
+    // joins them before the outputs are copied (one station 123 -> 111 us a
+    // block, FM band 309 -> 291, 512 serving channels 585 -> 561).  Not while
+    // stages are timed: then every kernel has its interval.
+    const bool fork = !pl.pll_list.empty() && f.s2 && !r->profiling;
+    cudaStream_t fs = fork ? f.s2 : f.s;
+    if (fork) {
+        CK(cudaEventRecord(f.ev_fork, f.s));
+        CK(cudaStreamWaitEvent(f.s2, f.ev_fork, 0));
+    }
     if (!pl.w_rds.empty()) {
         prof_mark(r, f, "rds");
-        CK(launch_rds((int)pl.w_rds.size(), pl.rds_smem, f.s, d_w + o_rds, d_sb, r->d_prm, r->d_st, wt, r->d_tabs,
+        CK(launch_rds((int)pl.w_rds.size(), pl.rds_smem, fs, d_w + o_rds, d_sb, r->d_prm, r->d_st, wt, r->d_tabs,
                       f.d_wk, r->d_rds_dl, d_rds));
         nl++;
     }
     if (!pl.sbs.empty()) {
         prof_mark(r, f, "post_front");
-        CK(launch_post_front((int)pl.sbs.size(), f.s, d_sb, r->d_prm, r->d_st, d_ext, f.d_wk, r->d_comp_dl,
+        CK(launch_post_front((int)pl.sbs.size(), fs, d_sb, r->d_prm, r->d_st, d_ext, f.d_wk, r->d_comp_dl,
                              r->d_rds_dl, r->d_tabs, r->d_d1hist, d_res));
         nl++;
     }
-    CK(cudaEventRecord(f.ev_front, f.s));
+    CK(cudaEventRecord(f.ev_front, fs));
     // ---- back half: after the previous block's back half ----
     if (prev) {
         prof_mark(r, f, "wait_prev_back");
@@ -1573,6 +1585,7 @@ static int enqueue_block(gpud_runner *r, Frame &f, const Frame *prev, BlockPlan 
         nl++;
     }
     CK(cudaEventRecord(f.ev_back, f.s));
+    if (fork) CK(cudaStreamWaitEvent(f.s, f.ev_front, 0));
     prof_mark(r, f, "d2h");
     r->launches += (uint64_t)nl;
     gpud_count_launch(nl);
