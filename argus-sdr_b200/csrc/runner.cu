@@ -21,6 +21,7 @@
 #include <cstring>
 #include <map>
 #include <tuple>
+#include <type_traits>
 #include <mutex>
 #include <string>
 #include <time.h>
@@ -315,7 +316,7 @@ struct Frame {
     char *d_desc = nullptr, *h_desc = nullptr;
     size_t desc_cap = 0;
     char *d_out = nullptr, *h_out = nullptr;
-    size_t out_cap = 0;
+    size_t out_cap = 0, hout_cap = 0;
     char *h_stage = nullptr;
     size_t stage_cap = 0;
     float *d_wk = nullptr;
@@ -348,6 +349,10 @@ struct Frame {
 using namespace gpud;
 
 struct gpud_runner {
+    // a runner that lives for one block (the one-shot entry points): one frame,
+    // no input ring, no pinned staging, host memory for what is copied back only
+    bool one_shot = false;
+    char *d_slab = nullptr;  // the persistent arenas below, one allocation
     int fs = 0, max_block = 0, max_ch = 0, max_taps = 0;
     uint64_t budget = 0, used = 0;
     int schedule = GPUD_SCHED_BATCHED;
@@ -1158,15 +1163,24 @@ static int ensure_frame(gpud_runner *r, Frame &f, const BlockPlan &pl) {
     size_t res = align256(pl.sbs.size() * sizeof(DevResult));
     size_t need = res + align256((size_t)pl.tot_pcm * 2) + align256((size_t)pl.tot_audio * 4) +
                   align256((size_t)pl.tot_rds * 8) + align256((size_t)pl.tot_ext * 8);
-    if (need > f.out_cap) {
+    // the host mirror: the same layout, which a one-shot runner (no emitted IQ)
+    // cuts behind the audio that is copied back
+    size_t hneed = need;
+    if (r->one_shot && pl.tot_emit_ext == 0)
+        hneed = !r->host_outputs ? res
+                                 : res + align256((size_t)pl.tot_pcm * 2) + align256((size_t)pl.tot_rds * 8) +
+                                       align256((size_t)pl.tot_audio_host * 4);
+    if (need > f.out_cap || hneed > f.hout_cap) {
         cudaFree(f.d_out);
         if (f.h_out) cudaFreeHost(f.h_out);
         f.d_out = nullptr;
         f.h_out = nullptr;
-        size_t cap = need * 5 / 4 + 4096;
+        f.out_cap = f.hout_cap = 0;
+        size_t cap = need * 5 / 4 + 4096, hcap = hneed * 5 / 4 + 4096;
         CK(cudaMalloc((void **)&f.d_out, cap));
-        CK(cudaMallocHost((void **)&f.h_out, cap));
+        CK(cudaMallocHost((void **)&f.h_out, hcap));
         f.out_cap = cap;
+        f.hout_cap = hcap;
         r->graph_rebuilds++;
     }
     size_t nw = 0;
@@ -1254,7 +1268,11 @@ static int stage_input(gpud_runner *r, Frame &f, const gpud_float2 *iq, int n, i
     bool pinned = cudaPointerGetAttributes(&at, iq) == cudaSuccess && at.type == cudaMemoryTypeHost;
     cudaGetLastError();
     const void *src = iq;
-    if (!pinned) {
+    if (r->one_shot) {
+        // straight from the caller's memory: the copy stages pageable memory
+        // itself, and page-locking as much for one block costs ten times the copy
+        CK(dalloc(&f.d_block, (size_t)n));
+    } else if (!pinned) {
         std::memcpy(f.h_in, iq, (size_t)n * sizeof(float2));
         src = f.h_in;
     }
@@ -1639,7 +1657,7 @@ static int submit_batched(gpud_runner *r, const gpud_float2 *iq, int n, int on_d
     // a block in pinned host memory starts its copy into the input ring now,
     // before this submit waits for a free frame
     int ring = -1;
-    if (!on_device && n > 0 && iq && host_pinned(iq)) {
+    if (!r->one_shot && !on_device && n > 0 && iq && host_pinned(iq)) {
         ring = r->ring_next;
         r->ring_next = (ring + 1) % kInRing;
         CK(cudaStreamWaitEvent(r->in_s, r->ring_free[ring], 0));  // its previous block's readers are done
@@ -1778,7 +1796,7 @@ static int run_plain(gpud_runner *r, const gpud_float2 *iq, int n, int on_device
         advance_mirrors(r, one, n, &a1);
         after.push_back(a1[0]);
     }
-    if (gathered.size() > f.out_cap) return set_err(r, GPUD_E_CUDA, "plain gather overflow");
+    if (gathered.size() > f.hout_cap) return set_err(r, GPUD_E_CUDA, "plain gather overflow");
     std::memcpy(f.h_out, gathered.data(), gathered.size());
     f.off_res = 0;
     f.off_pcm = p_off;
@@ -1814,12 +1832,13 @@ static int run_block(gpud_runner *r, const gpud_float2 *iq, int n, int on_device
 
 extern "C" {
 
-GPUD_API int GPUD_CALL gpud_runner_create(int sample_rate, int max_block, int max_channels, int max_taps,
-                                          uint64_t device_mem_budget, gpud_runner **out) {
+static int create_runner(int sample_rate, int max_block, int max_channels, int max_taps, uint64_t device_mem_budget,
+                         bool one_shot, gpud_runner **out) {
     if (!out || sample_rate <= 0 || max_block <= 0 || max_channels <= 0 || max_channels > 4096 || max_taps <= 0 ||
         max_taps > 4096)
         return GPUD_E_ARG;
     auto *r = new gpud_runner();
+    r->one_shot = one_shot;
     r->fs = sample_rate;
     r->max_block = max_block;
     r->max_ch = max_channels;
@@ -1857,35 +1876,54 @@ GPUD_API int GPUD_CALL gpud_runner_create(int sample_rate, int max_block, int ma
         CKC(cudaEventCreateWithFlags(&f.ev_done, cudaEventDisableTiming));
         CKC(cudaEventCreate(&f.ev0));
         CKC(cudaEventCreate(&f.ev1));
+        if (one_shot) break;  // the only frame; its block buffer comes with the block
         CKC(dalloc(&f.d_block, (size_t)max_block));
         CKC(cudaMallocHost((void **)&f.h_in, (size_t)max_block * sizeof(float2)));
     }
-    CKC(cudaStreamCreateWithFlags(&r->in_s, cudaStreamNonBlocking));
-    for (int i = 0; i < kInRing; ++i) {
-        CKC(dalloc(&r->d_ring[i], (size_t)max_block));
-        CKC(cudaEventCreate(&r->ring_t0[i]));
-        CKC(cudaEventCreate(&r->ring_copied[i]));
-        CKC(cudaEventCreateWithFlags(&r->ring_free[i], cudaEventDisableTiming));
+    if (!one_shot) {
+        CKC(cudaStreamCreateWithFlags(&r->in_s, cudaStreamNonBlocking));
+        for (int i = 0; i < kInRing; ++i) {
+            CKC(dalloc(&r->d_ring[i], (size_t)max_block));
+            CKC(cudaEventCreate(&r->ring_t0[i]));
+            CKC(cudaEventCreate(&r->ring_copied[i]));
+            CKC(cudaEventCreateWithFlags(&r->ring_free[i], cudaEventDisableTiming));
+        }
     }
-    size_t M = (size_t)max_channels;
-    CKC(dalloc(&r->d_prm, M));
-    CKC(dalloc(&r->d_st, M));
-    CKC(dalloc(&r->d_taps, M * 2 * (size_t)r->tapcap));
-    CKC(dalloc(&r->d_hist, M * 2 * (size_t)max_taps));
-    CKC(dalloc(&r->d_comp_dl, M * kWfmHist));
-    CKC(dalloc(&r->d_lr_dl, M * kWfmHist));
-    CKC(dalloc(&r->d_audio_dl, M * kAudioDlStrideH));
-    CKC(dalloc(&r->d_rds_dl, M * kWfmHist));
-    CKC(dalloc(&r->d_wtaps, (size_t)kMaxWfmClasses));
-    CKC(dalloc(&r->d_tabs, (size_t)kMaxWfmClasses * 2));  // RDS 57 kHz tables, then 38 kHz tables
-    CKC(dalloc(&r->d_aud, M));
-    CKC(dalloc(&r->d_d1taps, M * kD1Taps));
-    CKC(dalloc(&r->d_d1hist, M * kWfmHist));
-    CKC(dalloc(&r->d_banks, (size_t)kMaxRsClasses));
+    const size_t M = (size_t)max_channels;
+    // first pass: the size of every arena; second: their places in the slab
+    size_t total = 0;
+    auto arena = [&](auto *&p, size_t count) {
+        const size_t bytes = align256(std::max<size_t>(count, 1) * sizeof(*p));
+        if (r->d_slab) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(r->d_slab + total);
+        total += bytes;
+    };
+    for (int pass = 0; pass < 2; ++pass) {
+        total = 0;
+        arena(r->d_prm, M);
+        arena(r->d_st, M);
+        arena(r->d_taps, M * 2 * (size_t)r->tapcap);
+        arena(r->d_hist, M * 2 * (size_t)max_taps);
+        arena(r->d_comp_dl, M * kWfmHist);
+        arena(r->d_lr_dl, M * kWfmHist);
+        arena(r->d_audio_dl, M * kAudioDlStrideH);
+        arena(r->d_rds_dl, M * kWfmHist);
+        arena(r->d_wtaps, (size_t)kMaxWfmClasses);
+        arena(r->d_tabs, (size_t)kMaxWfmClasses * 2);  // RDS 57 kHz tables, then 38 kHz tables
+        arena(r->d_aud, M);
+        arena(r->d_d1taps, M * kD1Taps);
+        arena(r->d_d1hist, M * kWfmHist);
+        arena(r->d_banks, (size_t)kMaxRsClasses);
+        if (!pass) CKC(cudaMalloc((void **)&r->d_slab, total));
+    }
 #undef CKC
     r->used = slot_state_bytes(r) * M + (uint64_t)max_block * 8 * (kFrames + kInRing) + sizeof(RsBank) * kMaxRsClasses;
     *out = r;
     return 0;
+}
+
+GPUD_API int GPUD_CALL gpud_runner_create(int sample_rate, int max_block, int max_channels, int max_taps,
+                                          uint64_t device_mem_budget, gpud_runner **out) {
+    return create_runner(sample_rate, max_block, max_channels, max_taps, device_mem_budget, false, out);
 }
 
 GPUD_API int GPUD_CALL gpud_runner_destroy(gpud_runner *r) {
@@ -1926,20 +1964,7 @@ GPUD_API int GPUD_CALL gpud_runner_destroy(gpud_runner *r) {
         if (f.s) cudaStreamDestroy(f.s);
     }
     if (r->h_fault) cudaFreeHost(r->h_fault);
-    cudaFree(r->d_prm);
-    cudaFree(r->d_st);
-    cudaFree(r->d_taps);
-    cudaFree(r->d_hist);
-    cudaFree(r->d_comp_dl);
-    cudaFree(r->d_lr_dl);
-    cudaFree(r->d_audio_dl);
-    cudaFree(r->d_rds_dl);
-    cudaFree(r->d_wtaps);
-    cudaFree(r->d_tabs);
-    cudaFree(r->d_aud);
-    cudaFree(r->d_d1taps);
-    cudaFree(r->d_d1hist);
-    cudaFree(r->d_banks);
+    cudaFree(r->d_slab);
     for (double *a : r->rs_arms) cudaFree(a);
     if (r->stream) cudaStreamDestroy(r->stream);
     if (r->admin) cudaStreamDestroy(r->admin);
@@ -2607,7 +2632,7 @@ GPUD_API int GPUD_CALL gpud_wfm_batch_audio(const gpud_float2 *iq, int n, int iq
     res->demod_rate = rate;
     if ((n + d1 - 1) / d1 < 2) return 0;  // fewer than two decimated samples: no audio
     gpud_runner *r = nullptr;
-    int rc = gpud_runner_create(sample_rate, n, 1, 101, 0, &r);
+    int rc = create_runner(sample_rate, n, 1, 101, 0, true, &r);
     if (rc) return rc;
     gpud_channel_spec sp{};
     sp.signal_id = 1;
@@ -2679,7 +2704,7 @@ GPUD_API int GPUD_CALL gpud_demod_audio_segment(int mode, const gpud_float2 *iq,
     res->demod_rate = rate;
     res->out_rate = rate;
     gpud_runner *r = nullptr;
-    int rc = gpud_runner_create(sample_rate, n, 1, 101, 0, &r);
+    int rc = create_runner(sample_rate, n, 1, 101, 0, true, &r);
     if (rc) return rc;
     gpud_channel_spec sp{};
     sp.signal_id = 1;
