@@ -103,6 +103,7 @@ cudaError_t launch_audio48(int grid_rs, int count, cudaStream_t sm, const int2 *
                            const SlotBlock *sbt, const ChanParams *prm, const RsBank *banks, AudState *aud,
                            const float *audio, float *rs_buf, int16_t *pcm);
 int audio48_tile();
+cudaError_t launch_rs_bank(cudaStream_t sm, int L, int M, int K, double *arm);
 int rds_smem_bytes(int dr);
 int rds_tile();
 int dense_smem_bytes_host(int P, int L);
@@ -497,19 +498,6 @@ static uint64_t slot_state_bytes(const gpud_runner *r) {
            (kWfmHist * 3 + kAudioDlStrideH) * 8 + sizeof(AudState) + kD1Taps * 8 + kWfmHist * 8;
 }
 
-// NewResampler (dsp/resample.go:45-93, 256-295): L/M from the gcd, odd
-// prototype of L*32(+1) taps, windowed sinc fc = 0.90/max(L, M), Kaiser
-// beta 6 (bessel0 series), gain L, split into L arms of K taps.
-static double rs_bessel0(double x) {
-    double sum = 1.0, term = 1.0;
-    for (int k = 1; k < 30; k++) {
-        term *= (x / (2 * (double)k)) * (x / (2 * (double)k));
-        sum += term;
-        if (term < 1e-12 * sum) break;
-    }
-    return sum;
-}
-
 static int rs_gcd(int a, int b) {
     while (b != 0) {
         int t = a % b;
@@ -521,30 +509,15 @@ static int rs_gcd(int a, int b) {
 
 constexpr int kRsMaxArms = 1 << 17;  // any 48 kHz ratio from an integer rate up to 6 GS/s
 
-static bool build_rs_bank(int in_rate, int out_rate, RsBank *bk, std::vector<double> &arms) {
+// NewResampler's geometry (dsp/resample.go:45-60): L/M from the gcd, an odd
+// prototype of L*32(+1) taps split into L arms of K taps.
+static bool rs_geometry(int in_rate, int out_rate, RsBank *bk) {
     std::memset(bk, 0, sizeof *bk);
     const int g = rs_gcd(in_rate, out_rate);
     const int l = out_rate / g, m = in_rate / g;
     if (l > kRsMaxArms) return false;
-    int plen = l * 32;
-    if (plen % 2 == 0) plen++;
-    const int k = (plen + l - 1) / l;
+    const int plen = (l * 32) | 1, k = (plen + l - 1) / l;
     if (k > kRsTaps) return false;
-    arms.assign((size_t)l * k, 0.0);
-    const double fc = 0.90 / (double)std::max(l, m);
-    const double mid = (double)(plen - 1) / 2.0, b0 = rs_bessel0(6.0);
-    for (int p = 0; p < l; ++p)
-        for (int t = 0; t < k; ++t) {
-            const int n = p + t * l;
-            double v = 0.0;
-            if (n < plen) {
-                const double x = (double)n - mid;
-                const double sn = std::fabs(x) < 1e-12 ? 2 * GPUD_PI * fc : std::sin(2 * GPUD_PI * fc * x) / x;
-                const double xx = x / mid;
-                v = sn * (rs_bessel0(6.0 * std::sqrt(1 - xx * xx)) / b0) * (double)l;
-            }
-            arms[(size_t)p * k + t] = v;
-        }
     bk->L = l;
     bk->M = m;
     bk->K = k;
@@ -556,16 +529,15 @@ static int rs_class_for(gpud_runner *r, int rate) {
         if (r->rs_rate[i] == rate) return (int)i;
     if ((int)r->rs_rate.size() >= kMaxRsClasses) return -1;
     RsBank bk;
-    std::vector<double> arms;
-    if (!build_rs_bank(rate, 48000, &bk, arms)) return -1;
+    if (!rs_geometry(rate, 48000, &bk)) return -1;
     const int id = (int)r->rs_rate.size();
     double *d_arm = nullptr;
-    if (cudaMalloc((void **)&d_arm, arms.size() * sizeof(double)) != cudaSuccess) return -1;
+    if (cudaMalloc((void **)&d_arm, (size_t)bk.L * (size_t)bk.K * sizeof(double)) != cudaSuccess) return -1;
     r->rs_arms.push_back(d_arm);
     bk.arm = d_arm;
     // a new bank id is not referenced by any block in flight
-    if (cudaMemcpyAsync(d_arm, arms.data(), arms.size() * sizeof(double), cudaMemcpyHostToDevice, r->admin) !=
-            cudaSuccess ||
+    gpud_count_launch(1);
+    if (launch_rs_bank(r->admin, bk.L, bk.M, bk.K, d_arm) != cudaSuccess ||
         cudaMemcpyAsync(r->d_banks + id, &bk, sizeof(RsBank), cudaMemcpyHostToDevice, r->admin) != cudaSuccess)
         return -1;
     if (cudaStreamSynchronize(r->admin) != cudaSuccess) return -1;

@@ -3096,6 +3096,41 @@ cudaError_t launch_audio48(int grid_rs, int count, cudaStream_t sm, const int2 *
 
 int audio48_tile() { return kAudOT; }
 
+// Arms of a resampler bank (NewResampler, dsp/resample.go:45-93, 256-295):
+// windowed sinc fc = 0.90/max(L, M), Kaiser beta 6 by the reference's Bessel
+// series, gain L; arm[p*K + t] = prototype tap p + t*L.  One thread per tap: a
+// rate that shares no factor with 48 kHz has up to 48000 arms of 33 taps, which
+// took the host longer than the rest of an event's demod together.
+__device__ __forceinline__ double rs_bessel0(double x) {
+    double sum = 1.0, term = 1.0;
+    for (int k = 1; k < 30; k++) {
+        const double q = __ddiv_rn(x, 2.0 * (double)k);
+        term = __dmul_rn(term, __dmul_rn(q, q));
+        sum = __dadd_rn(sum, term);
+        if (term < __dmul_rn(1e-12, sum)) break;
+    }
+    return sum;
+}
+
+__global__ void __launch_bounds__(256) k_rs_bank(int L, int M, int K, double *__restrict__ arm) {
+    const int i = blockIdx.x * blockDim.x + (int)threadIdx.x;
+    if (i >= L * K) return;
+    const int plen = (L * 32) | 1, p = i / K, n = p + (i - p * K) * L;
+    double v = 0.0;
+    if (n < plen) {
+        const double fc = 0.90 / (double)max(L, M), mid = (double)(plen - 1) / 2.0, x = (double)n - mid;
+        const double sn = fabs(x) < 1e-12 ? 2 * GPUD_PI * fc : sin(2 * GPUD_PI * fc * x) / x;
+        const double xx = x / mid;
+        v = sn * (rs_bessel0(6.0 * sqrt(__dsub_rn(1.0, __dmul_rn(xx, xx)))) / rs_bessel0(6.0)) * (double)L;
+    }
+    arm[i] = v;
+}
+
+cudaError_t launch_rs_bank(cudaStream_t sm, int L, int M, int K, double *arm) {
+    k_rs_bank<<<(L * K + 255) / 256, 256, 0, sm>>>(L, M, K, arm);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_post_extract(int grid, cudaStream_t sm, const SlotBlock *sbt, const ChanParams *prm, ChanState *st,
                                 const float2 *x, int n, float2 *hist, DevResult *res) {
     return launch_dependent(k_post_extract, dim3((unsigned)grid), 128, 0, sm, sbt, prm, st, x, n, hist,
