@@ -234,8 +234,8 @@ struct BankGroup {
     int32_t n_out;   // outputs of every member this block
     int32_t jt0;     // first output of the bank tiles (earlier ones: the warp-per-output kernel)
     int32_t mem_off;
-    int32_t g_off;   // float2 offset of the packed modulated taps (T x cpad) in the frame's buffer
-    int32_t r;       // outputs per lane of a work item (1, 2 or 4): 8r outputs per item
+    int32_t g_off;   // float2 offset of the packed modulated taps (T rounded to even, x cpad) in the frame's buffer
+    int32_t r;       // outputs per lane of a full 32-channel item (1, 2 or 4): 8r outputs per item
 };
 
 // Rational polyphase resampler bank (dsp/resample.go:45-93) for one input rate.

@@ -60,6 +60,7 @@ cudaError_t launch_extract_bank(int grid, cudaStream_t sm, const int2 *work, con
                                 const int *members, const SlotBlock *sbt, const ChanParams *prm, const ChanState *st,
                                 const float2 *x, const float2 *gtab, float2 *ext);
 int bank_lanes();
+int64_t bank_pack_entries(int T, int cpad);
 int bank_warps();
 size_t gemm_pack_bytes_host(int D, int L, int N);
 cudaError_t launch_extract_wide(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
@@ -918,9 +919,11 @@ static std::vector<char> plan_gemm_groups(gpud_runner *r, BlockPlan &pl) {
 // form a bank when there are at least kBankMinChannels of them.  A bank takes
 // every output from jt0 on: the first output whose window lies inside the
 // block; the warp-per-output kernel keeps the outputs before it (they reach
-// into the carried history).  A bank's work items hold 8r outputs, r = 4
-// unless the bank then gives fewer than two items per SM.  Returns the first
-// banked output of every row (-1: not banked).
+// into the carried history).  A work item holds 8r outputs: r = 4, which loads
+// least per multiply-add, unless the block's banks together then give fewer
+// items than there are SMs (r = 2, 1: 120 channels 44 us with r = 4, 53 with r
+// halved per bank until each had two items per SM).  Returns the first banked
+// output of every row (-1: not banked).
 static std::vector<int> plan_bank_groups(gpud_runner *r, BlockPlan &pl, const std::vector<char> &grouped) {
     pl.banks.clear();
     pl.bmembers.clear();
@@ -956,20 +959,27 @@ static std::vector<int> plan_bank_groups(gpud_runner *r, BlockPlan &pl, const st
         b.jt0 = jb;
         b.mem_off = (int)pl.bmembers.size();
         b.g_off = (int)pl.bank_g;
-        const int nch = b.cpad / bank_lanes();
-        b.r = 4;
-        while (b.r > 1 && (int64_t)(n_out - jb + 8 * b.r - 1) / (8 * b.r) * nch < 2 * r->num_sms) b.r >>= 1;
-        pl.bank_g += ((int64_t)T * b.cpad + 63) & ~63;
-        pl.bank_max_total = std::max(pl.bank_max_total, T * b.cpad);
-        const int bi = (int)pl.banks.size();
+        pl.bank_g += (bank_pack_entries(T, b.cpad) + 63) & ~63;
+        pl.bank_max_total = std::max(pl.bank_max_total, (int)bank_pack_entries(T, b.cpad));
         for (int row : rows) {
             pl.bmembers.push_back(row);
             first[(size_t)row] = jb;
         }
-        const int tile = bank_warps() * b.r;
-        for (int t = 0; jb + t * tile < n_out; ++t)
-            for (int c = 0; c < nch; ++c) pl.w_bank.push_back(make_int2(bi, t * nch + c));
         pl.banks.push_back(b);
+    }
+    auto items = [&](const BankGroup &b, int rr) {
+        return (int64_t)((b.n_out - b.jt0 + bank_warps() * rr - 1) / (bank_warps() * rr)) * (b.cpad / bank_lanes());
+    };
+    int rr = 4;
+    for (; rr > 1; rr >>= 1) {
+        int64_t total = 0;
+        for (const BankGroup &b : pl.banks) total += items(b, rr);
+        if (total >= r->num_sms) break;
+    }
+    for (int bi = 0; bi < (int)pl.banks.size(); ++bi) {
+        BankGroup &b = pl.banks[(size_t)bi];
+        b.r = rr;
+        for (int64_t k = 0, n = items(b, rr); k < n; ++k) pl.w_bank.push_back(make_int2(bi, (int)k));
     }
     return first;
 }
