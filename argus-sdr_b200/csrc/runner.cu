@@ -100,10 +100,10 @@ cudaError_t launch_decim2(int grid, cudaStream_t sm, const int2 *work, const Slo
 int decim2_tile();
 cudaError_t launch_post_back(int grid, cudaStream_t sm, const SlotBlock *sbt, const ChanParams *prm, ChanState *st,
                              const float *wk, int W, float *lr_dl, float *audio_dl, DevResult *res);
-cudaError_t launch_audio48(int grid_rs, int count, cudaStream_t sm, const int2 *work, const int *list,
+cudaError_t launch_audio48(int grid_rs, int rs_smem, int count, cudaStream_t sm, const int2 *work, const int *list,
                            const SlotBlock *sbt, const ChanParams *prm, const RsBank *banks, AudState *aud,
                            const float *audio, float *rs_buf, int16_t *pcm);
-int audio48_tile();
+void audio48_tile(int L, int M, int C, int *outputs, int *smem);
 cudaError_t launch_rs_bank(cudaStream_t sm, int L, int M, int K, double *arm);
 int rds_smem_bytes(int dr);
 int rds_tile();
@@ -290,6 +290,7 @@ struct BlockPlan {
     bool batch_stereo = false;  // a GPUD_CH_BATCH_STEREO channel has composite this block
     std::vector<int> aud_list;  // entries with a 48 kHz back end and input this block
     std::vector<int2> w_aud;    // (entry, tile) of the 48 kHz resampler
+    int aud_smem = 0;
     std::vector<int2> w_dec;    // (entry, tile) of the pre-demod decimator
     int64_t tot_ext = 0, tot_emit_ext = 0, tot_comp = 0, tot_audio = 0, tot_audio_host = 0, tot_rds = 0,
             tot_pcm = 0;
@@ -1019,6 +1020,7 @@ static void finish_plan(gpud_runner *r, BlockPlan &pl) {
         }
     pl.aud_list.clear();
     pl.w_aud.clear();
+    pl.aud_smem = 0;
     pl.w_dec.clear();
     for (int i = 0; i < (int)pl.sbs.size(); ++i) {
         SlotBlock &sb = pl.sbs[(size_t)i];
@@ -1032,7 +1034,10 @@ static void finish_plan(gpud_runner *r, BlockPlan &pl) {
         pcm += ((int64_t)sb.rs_nout * s.aud_ch * ((s.spec.flags & GPUD_CH_PCM_F32) ? 2 : 1) + 7) & ~7;
         if (sb.rs_frames > 0) {
             pl.aud_list.push_back(i);
-            for (int t = 0; t * audio48_tile() < sb.rs_nout; ++t) pl.w_aud.push_back(make_int2(i, t));
+            int ot, sm;
+            audio48_tile(s.rs_L, s.rs_M, s.aud_ch, &ot, &sm);
+            for (int t = 0; t * ot < sb.rs_nout; ++t) pl.w_aud.push_back(make_int2(i, t));
+            pl.aud_smem = std::max(pl.aud_smem, sm);
         }
     }
     pl.tot_comp = comp;
@@ -1574,7 +1579,7 @@ static int enqueue_block(gpud_runner *r, Frame &f, const Frame *prev, BlockPlan 
     }
     if (!pl.aud_list.empty()) {
         prof_mark(r, f, "audio48k");
-        CK(launch_audio48((int)pl.w_aud.size(), (int)pl.aud_list.size(), f.s, d_w + o_waud, d_aud_list, d_sb,
+        CK(launch_audio48((int)pl.w_aud.size(), pl.aud_smem, (int)pl.aud_list.size(), f.s, d_w + o_waud, d_aud_list, d_sb,
                           r->d_prm, r->d_banks, r->d_aud, d_audio, f.d_rs, d_pcm));
         nl += pl.w_aud.empty() ? 1 : 2;
     }

@@ -2610,42 +2610,117 @@ k_post_back(const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ pr
 // from its start -- then the WFM gain 0.35 and s16le: int16(clip(s * 32767)),
 // truncating; it also carries the delay lines and the de-emphasis state.
 constexpr int kAudThreads = 256;
-constexpr int kAudOT = 256;  // resampled frames per CTA in k_audio48_rs
+constexpr int kAudOT = 256;       // resampled frames per CTA where each thread takes one
+constexpr int kAudWin = 2600;     // most staged input frames of a tile
+constexpr int kAudBank = 4096;    // most staged bank coefficients (doubles)
+constexpr int kAudLive = 160;     // fewest busy threads of a tile with several outputs per thread
 
-constexpr int kAudWin = 2048;     // staged input frames per channel and CTA (256 outputs at M/L <= 7.8)
-constexpr int kAudBank = 4096;    // staged bank coefficients (doubles)
+// Tile of one resampler ratio: outputs o, o+L, o+2L, o+3L stand at one phase, so
+// a thread takes r = 4 of them and reads each of its arm's coefficients once,
+// unless the tile's input window then leaves too few threads busy (M/L above
+// about 3: 40 stereo channels at 312.5 kHz 14.0 us with r = 1, 16.4 with 2,
+// 24.5 with 4 and 96 threads).  r = 0: arms or window too large for shared
+// memory (one output per thread from global memory).
+struct AudTile {
+    int r, ot, smem;
+};
+__host__ __device__ inline int aud_window(int ot, int L, int M, int K) {
+    return (int)((int64_t)(ot - 1) * M / L) + K + 2;
+}
+__host__ __device__ inline AudTile aud_tile(int L, int M, int K, int C) {
+    if (L == M || (int64_t)L * K > kAudBank) return {0, kAudOT, 0};
+    for (int r = 4; r >= 1; r -= 3) {
+        // one output per thread: whole warps; four: whole blocks of 4L
+        const int unit = r > 1 ? r * L : 32;
+        int ot = kAudThreads * r / unit * unit;
+        while (ot > 0 && aud_window(ot, L, M, K) > kAudWin) ot -= unit;
+        if (ot < kAudLive * r) continue;
+        return {r, ot, (((L * K + 1) & ~1) + C * aud_window(ot, L, M, K)) * 8};
+    }
+    return {0, kAudOT, 0};
+}
 
+// R outputs of a staged tile, C channels: the products and sums of one output
+// in its arm's order.
+template <int R, int C>
+__device__ __forceinline__ void aud_dot(const double *arm, const float *x, int M, int K, double (&acc)[R][C]) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int c = 0; c < C; ++c) acc[r][c] = 0.0;
+#pragma unroll 11
+    for (int k = 0; k < K; ++k) {
+        const double h = arm[k];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float *p = x + (r * M - k) * C;
+            if constexpr (C == 2) {
+                const float2 v = *reinterpret_cast<const float2 *>(p);
+                acc[r][0] = __dadd_rn(acc[r][0], __dmul_rn((double)v.x, h));
+                acc[r][1] = __dadd_rn(acc[r][1], __dmul_rn((double)v.y, h));
+            } else {
+                acc[r][0] = __dadd_rn(acc[r][0], __dmul_rn((double)*p, h));
+            }
+        }
+    }
+}
+
+template <int R, int C>
+__device__ __forceinline__ void aud_outputs(const SlotBlock &sb, int oa, int ob, int ot, const double *s_bank,
+                                            const float *s_in, int ph0, int L, int M, int K,
+                                            float *__restrict__ rs_out) {
+    // thread i: phase slot i % L of block i / L, outputs oa + (i/L)*R*L + i%L + r*L
+    const int i = (int)threadIdx.x, o0 = oa + (R > 1 ? (i / L) * (R * L) + i % L : i);
+    if (i * R >= ot || o0 >= ob) return;
+    const unsigned t = (unsigned)ph0 + (unsigned)(o0 - oa) * (unsigned)M, cc = t / (unsigned)L;
+    double acc[R][C];
+    aud_dot<R, C>(s_bank + (int)(t - cc * (unsigned)L) * K, s_in + ((int)cc + K - 1) * C, M, K, acc);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int o = o0 + r * L;
+        if (o >= ob) break;
+        float *dst = rs_out + sb.pcm_off + o * C;
+        dst[0] = (float)acc[r][0];
+        if constexpr (C == 2) dst[1] = (float)acc[r][1];
+    }
+}
+
+// Bound by its latencies (the channel's tables, then the arms and the window into
+// shared memory, then the chains of 33 sums): four outputs per thread stage the
+// arms a quarter as often, load a coefficient once for four products, keep four
+// chains in flight and fit 120 narrow channels in about one wave of CTAs.
+// Measured, one output per thread before and now: 120 mono channels 20.9 ->
+// 12.8 us, 512 channels of all modes 26.0 -> 20.5, 40 stereo ones (r = 1) 14.0
+// both.  (A window staged in float64 spares 33 conversions per output but strides
+// of M/L doubles conflict in the banks: 40 stereo channels 21.7 us.)
 __global__ void __launch_bounds__(kAudThreads)
 k_audio48_rs(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
              const RsBank *__restrict__ banks, const AudState *__restrict__ aud, const float *__restrict__ audio,
              float *__restrict__ rs_out) {
     dependency_wait();
-    extern __shared__ double s_aud[];  // bank (L*K doubles) | inputs 2 x kAudWin floats
+    extern __shared__ __align__(16) double s_aud[];  // arms (L*K, rounded to even) | window (win x C)
     const int2 w = work[blockIdx.x];
     const SlotBlock sb = sbt[w.x];
-    const int oa = w.y * kAudOT, ob = min(sb.rs_nout, oa + kAudOT);  // this CTA's outputs
-    if (oa >= ob) return;
     const ChanParams &cp = prm[sb.slot];
     const AudState &as = aud[sb.slot];
-    const RsBank &bk = banks[cp.rs_bank];
+    const RsBank bk = banks[cp.rs_bank];
     const int C = cp.aud_ch, L = bk.L, M = bk.M, K = bk.K;
+    const AudTile at = aud_tile(L, M, K, C);
+    const int oa = w.y * at.ot, ob = min(sb.rs_nout, oa + at.ot);  // this CTA's outputs
+    if (oa >= ob) return;
     const float *in = audio + sb.audio_off;
     if (L == M) {
         for (int o = oa + (int)threadIdx.x; o < ob; o += kAudThreads)
             for (int c = 0; c < C; ++c) rs_out[sb.pcm_off + o * C + c] = in[o * C + c];
         return;
     }
-    // consumed-input window of the tile: [lo, hi]
-    const int64_t lo = ((int64_t)sb.rs_t0 + (int64_t)oa * M) / L - K;
-    const int64_t hi = ((int64_t)sb.rs_t0 + (int64_t)(ob - 1) * M) / L - 1;
-    const int win = (int)(hi - lo + 1);
-    const bool staged = win <= kAudWin && L * K <= kAudBank;
-    double *s_bank = s_aud;
-    float *s_in = reinterpret_cast<float *>(s_aud + kAudBank);
-    if (staged) {
-        // eight loads in flight per thread: the staging, not the 33-tap dot
-        // products, sets this kernel's time
-        constexpr int U = 8;
+    if (at.r) {
+        // inputs consumed before the tile's first output, and its phase
+        const int64_t Ta = (int64_t)sb.rs_t0 + (int64_t)oa * M, ca = Ta / L;
+        const int ph0 = (int)(Ta - ca * L);
+        const int win = (int)(((int64_t)ph0 + (int64_t)(ob - 1 - oa) * M) / L) + K;  // from input ca - K on
+        float *s_in = reinterpret_cast<float *>(s_aud + ((L * K + 1) & ~1));
+        constexpr int U = 8;  // loads in flight per thread
         const int nb = L * K;
         for (int i0 = threadIdx.x; i0 < nb; i0 += U * kAudThreads) {
             double v[U];
@@ -2657,51 +2732,51 @@ k_audio48_rs(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, c
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int i = i0 + u * kAudThreads;
-                if (i < nb) s_bank[i] = v[u];
+                if (i < nb) s_aud[i] = v[u];
             }
         }
-        for (int c = 0; c < C; ++c) {
-            for (int i0 = threadIdx.x; i0 < win; i0 += U * kAudThreads) {
-                float v[U];
+        const int64_t g0 = (ca - K) * C;  // element e of the window is in[g0 + e], or carried
+        for (int i0 = threadIdx.x; i0 < win * C; i0 += U * kAudThreads) {
+            float v[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int i = i0 + u * kAudThreads;
-                    const int64_t g = lo + i;
-                    v[u] = i < win ? (g >= 0 ? in[g * C + c] : as.dl[c][-1 - g]) : 0.f;
-                }
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + u * kAudThreads;
+                const int64_t g = g0 + i;
+                v[u] = 0.f;
+                if (i < win * C) v[u] = g >= 0 ? in[g] : C == 2 ? as.dl[i & 1][-1 - (g >> 1)] : as.dl[0][-1 - g];
+            }
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int i = i0 + u * kAudThreads;
-                    if (i < win) s_in[c * kAudWin + i] = v[u];
-                }
+            for (int u = 0; u < U; ++u) {
+                const int i = i0 + u * kAudThreads;
+                if (i < win * C) s_in[i] = v[u];
             }
         }
         __syncthreads();
+#define GPUD_AUD(R)                                                                                  \
+    if (C == 2) aud_outputs<R, 2>(sb, oa, ob, at.ot, s_aud, s_in, ph0, L, M, K, rs_out);             \
+    else aud_outputs<R, 1>(sb, oa, ob, at.ot, s_aud, s_in, ph0, L, M, K, rs_out);
+        if (at.r == 4) {
+            GPUD_AUD(4)
+        } else {
+            GPUD_AUD(1)
+        }
+#undef GPUD_AUD
+        return;
     }
     for (int o = oa + (int)threadIdx.x; o < ob; o += kAudThreads) {
         const int64_t T = (int64_t)sb.rs_t0 + (int64_t)o * M;
         const int64_t cc = T / L;  // T >= 0
         const int ph = (int)(T - cc * L);
         double acc0 = 0.0, acc1 = 0.0;
-        if (staged) {
-            const double *arm = s_bank + ph * K;
-            const float *x0 = s_in + (cc - 1 - lo), *x1 = s_in + kAudWin + (cc - 1 - lo);
-            for (int k = 0; k < K; ++k) {
-                const double h = arm[k];
-                acc0 = __dadd_rn(acc0, __dmul_rn((double)x0[-k], h));
-                if (C == 2) acc1 = __dadd_rn(acc1, __dmul_rn((double)x1[-k], h));
-            }
-        } else {
-            const double *arm = bk.arm + ph * K;
-            for (int k = 0; k < K; ++k) {
-                const int64_t i = cc - 1 - k;
-                const double h = arm[k];
-                const float v0 = i >= 0 ? in[i * C] : as.dl[0][-1 - i];
-                acc0 = __dadd_rn(acc0, __dmul_rn((double)v0, h));
-                if (C == 2) {
-                    const float v1 = i >= 0 ? in[i * 2 + 1] : as.dl[1][-1 - i];
-                    acc1 = __dadd_rn(acc1, __dmul_rn((double)v1, h));
-                }
+        const double *arm = bk.arm + ph * K;
+        for (int k = 0; k < K; ++k) {
+            const int64_t i = cc - 1 - k;
+            const double h = arm[k];
+            const float v0 = i >= 0 ? in[i * C] : as.dl[0][-1 - i];
+            acc0 = __dadd_rn(acc0, __dmul_rn((double)v0, h));
+            if (C == 2) {
+                const float v1 = i >= 0 ? in[i * 2 + 1] : as.dl[1][-1 - i];
+                acc1 = __dadd_rn(acc1, __dmul_rn((double)v1, h));
             }
         }
         float *dst = rs_out + sb.pcm_off + o * C;
@@ -3076,15 +3151,14 @@ cudaError_t launch_post_front(int grid, cudaStream_t sm, const SlotBlock *sbt, c
                             rds_dl, tabs, d1hist, res);
 }
 
-cudaError_t launch_audio48(int grid_rs, int count, cudaStream_t sm, const int2 *work, const int *list,
+cudaError_t launch_audio48(int grid_rs, int rs_smem, int count, cudaStream_t sm, const int2 *work, const int *list,
                            const SlotBlock *sbt, const ChanParams *prm, const RsBank *banks, AudState *aud,
                            const float *audio, float *rs_buf, int16_t *pcm) {
-    const int smem = kAudBank * 8 + 2 * kAudWin * 4;
-    static std::atomic<uint64_t> optin{0};  // 64 KiB of dynamic shared memory needs the opt-in
-    cudaError_t e = smem_optin_once(optin, (const void *)k_audio48_rs, smem);
+    static std::atomic<uint64_t> optin{0};  // more than 48 KiB of dynamic shared memory needs the opt-in
+    cudaError_t e = smem_optin_once(optin, (const void *)k_audio48_rs, (kAudBank + 2 * kAudWin) * 8);
     if (e != cudaSuccess) return e;
     if (grid_rs > 0)
-        e = launch_dependent(k_audio48_rs, dim3((unsigned)grid_rs), kAudThreads, (size_t)smem, sm, work, sbt, prm, banks,
+        e = launch_dependent(k_audio48_rs, dim3((unsigned)grid_rs), kAudThreads, (size_t)rs_smem, sm, work, sbt, prm, banks,
                              aud, audio, rs_buf);
     if (e != cudaSuccess) return e;
     static std::atomic<uint64_t> optin_out{0};
@@ -3094,7 +3168,11 @@ cudaError_t launch_audio48(int grid_rs, int count, cudaStream_t sm, const int2 *
                             list, sbt, prm, banks, aud, audio, rs_buf, pcm);
 }
 
-int audio48_tile() { return kAudOT; }
+void audio48_tile(int L, int M, int C, int *outputs, int *smem) {
+    const AudTile t = aud_tile(L, M, kRsTaps, C);
+    *outputs = t.ot;
+    *smem = t.smem;
+}
 
 // Arms of a resampler bank (NewResampler, dsp/resample.go:45-93, 256-295):
 // windowed sinc fc = 0.90/max(L, M), Kaiser beta 6 by the reference's Bessel
