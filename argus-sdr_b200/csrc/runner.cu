@@ -113,6 +113,8 @@ int dense_tile();
 int wide_smem_bytes_host(int T);
 int group_smem_bytes_host(int Pc, int L);
 int mod_smem_bytes_host(int Pc, int L);
+int mod_launch_bytes_host(int P, int Pc, int L);
+int mod_item(int tile, int tiles);
 cudaError_t launch_extract_group(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
                                  const ChanParams *prm, const ChanState *st, const float2 *x, int n,
                                  const float2 *hist, const float *taps, float2 *ext);
@@ -1066,6 +1068,17 @@ static void finish_plan(gpud_runner *r, BlockPlan &pl) {
     pl.rds_smem = 0;
     std::vector<char> grouped = plan_gemm_groups(r, pl);
     const std::vector<int> banked = plan_bank_groups(r, pl, grouped);
+    // Tiles per work item of the modulated form: the item builds its channel's
+    // T modulated taps once, so with few phases (little to do per tile) it takes
+    // several, unless the block has too few tiles to keep every SM at work.
+    int64_t mod_total = 0;
+    for (int i = 0; i < (int)pl.sbs.size(); ++i)
+        if (r->slots[(size_t)pl.sbs[(size_t)i].slot].ext_kind == 3 && banked[(size_t)i] < 0)
+            mod_total += (pl.sbs[(size_t)i].n_out + dense_tile() - 1) / dense_tile();
+    std::vector<int> mod_rows;
+    auto mod_tiles = [&](const Slot &s) {
+        return mod_total < 16 * (int64_t)r->num_sms ? 1 : std::min(8, std::max(1, 256 / s.P));
+    };
     for (int i = 0; i < (int)pl.sbs.size(); ++i) {
         const SlotBlock &sb = pl.sbs[(size_t)i];
         Slot &s = r->slots[(size_t)sb.slot];
@@ -1084,12 +1097,13 @@ static void finish_plan(gpud_runner *r, BlockPlan &pl) {
                 pl.dense_smem[s.L] = std::max(pl.dense_smem[s.L], dense_smem_bytes_host(s.P, s.L));
                 pl.dense_pmax[s.L] = std::max(pl.dense_pmax[s.L], s.P);
             } else if (s.ext_kind == 2 || s.ext_kind == 3) {
-                auto &wl = s.ext_kind == 2 ? pl.w_group : pl.w_mod;
-                for (int t = 0; t * dense_tile() < sb.n_out; ++t) wl.push_back(make_int2(i, t));
-                if (s.ext_kind == 2)
+                if (s.ext_kind == 2) {
+                    for (int t = 0; t * dense_tile() < sb.n_out; ++t) pl.w_group.push_back(make_int2(i, t));
                     pl.group_smem = std::max(pl.group_smem, group_smem_bytes_host(s.pg, s.L));
-                else
-                    pl.mod_smem = std::max(pl.mod_smem, mod_smem_bytes_host(s.pg, s.L));
+                } else {
+                    mod_rows.push_back(i);
+                    pl.mod_smem = std::max(pl.mod_smem, mod_launch_bytes_host(s.P, s.pg, s.L));
+                }
             } else {
                 for (int t = 0; t * kWideTile < sb.n_out; ++t) pl.w_wide.push_back(make_int2(i, t));
                 pl.wide_smem = std::max(pl.wide_smem, wide_smem_bytes_host(s.T));
@@ -1127,7 +1141,18 @@ static void finish_plan(gpud_runner *r, BlockPlan &pl) {
         });
     };
     longest_first(pl.w_group);
-    longest_first(pl.w_mod);
+    // the modulated form's rows by code path (the CTAs of an SM share its
+    // instruction cache), the longest first
+    auto mod_key = [&](int row) {
+        const Slot &s = r->slots[(size_t)pl.sbs[(size_t)row].slot];
+        return std::make_tuple(-s.L, precise_sum(s.spec), -(int64_t)s.P);
+    };
+    std::stable_sort(mod_rows.begin(), mod_rows.end(), [&](int a, int b) { return mod_key(a) < mod_key(b); });
+    for (int row : mod_rows) {
+        const int nt = (pl.sbs[(size_t)row].n_out + dense_tile() - 1) / dense_tile();
+        const int k = mod_tiles(r->slots[(size_t)pl.sbs[(size_t)row].slot]);
+        for (int t = 0; t < nt; t += k) pl.w_mod.push_back(make_int2(row, mod_item(t, std::min(k, nt - t))));
+    }
 }
 
 static int ensure_frame(gpud_runner *r, Frame &f, const BlockPlan &pl) {

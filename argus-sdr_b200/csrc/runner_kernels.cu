@@ -960,40 +960,257 @@ k_extract_group(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt
 // taps hc[p + uD] = h[p + uD] exp(-j (p + uD) inc) of its phases, and every
 // output takes one rotation exp(j phi(n_j)) at the end:
 //     y_j = exp(j phi(n_j)) * sum_k hc[k] x(n_j - k).
+//
+// A warp works on 32 of its tile's outputs by itself: lane w + 8g runs chain w
+// (the phases pp = w, w+8, ... of a group) of the outputs 8g .. 8g+7, with the
+// R + L - 1 samples of a phase in a register window, and the eight chains of an
+// output are added in order at the end of each group.  Raw samples need no work
+// on their way, so the window of a warp's outputs comes into its own piece of
+// shared memory by asynchronous copies, kModKC phases at a time, each column a
+// contiguous run: 16 bytes per copy where all columns start at one parity (D
+// even), else 8.  Eight columns are followed by a pad of 64 bytes, so the window
+// loads of two output groups fall on the two halves of the banks.  Nothing waits
+// for another warp but the taps, which are built once per work item.
+// Bound by instruction issue (multiply-adds 42 % of the instructions, staging
+// addresses and window loads the rest; 16 warps per SM).  1344 such channels of
+// 64..768 taps among 2048: 1954 us with a tile's samples staged by the whole CTA
+// through registers, 1288 now.  Chunks of 16 with the next one in flight: 1643
+// (per-chunk work weighs more than the latency that 16 warps hide); rows of a
+// chunk unrolled by four: 1435, by two: 1344 (instruction cache).
+constexpr int kModKC = 32;                 // phases per staged chunk
+constexpr int kModPitch = kModKC + 2;      // column stride (float2): even, room for a copy that starts one early
+constexpr int kModR = 8;                   // outputs per lane
+constexpr int kModBuf = 34 * kModPitch + (34 >> 3) * 8 + kModPitch;  // 32 + L - 1 <= 35 columns
+constexpr int kModWarps = kDenseThreads / 32;
+constexpr int kModRed = 33;                // row stride of the chains' sums
+static_assert(kModBuf % 2 == 0 && kModBuf >= 2 * kModWarps * kModRed, "16-byte copies; float64 sums of eight chains");
+constexpr int kModTileBits = 24, kModTileMask = (1 << kModTileBits) - 1;  // work item: (entry, first tile | tiles)
+constexpr int kModTaps = 2048;             // modulated taps held at a time: all of them for most channels
 
-__host__ __device__ inline int mod_smem_bytes(int Pc, int L) {
+// Dynamic shared memory that sizes a channel's phase groups (they order its
+// sums, so this is kept as it was when a group was staged whole).
+int mod_smem_bytes_host(int Pc, int L) {
     int z = (Pc * dense_row_stride(L) * 8 + 15) & ~15;
     if (z < kRedBytes) z = kRedBytes;
     return z + Pc * L * 8 + 16;
 }
 
-int mod_smem_bytes_host(int Pc, int L) { return mod_smem_bytes(Pc, L); }
+int mod_item(int tile, int tiles) { return tile | tiles << kModTileBits; }
 
-template <int L>
-__device__ __forceinline__ void mod_row(const float2 *zrow, const float2 *hrow, int lane, float2 *acc) {
-    constexpr int R = kDenseR;
-    float2 win[R + L - 1];
+// What a launch needs: two chunks per warp and the modulated taps of as many
+// groups as kModTaps holds (at least one group's).
+int mod_launch_bytes_host(int P, int Pc, int L) {
+    return kModWarps * kModBuf * 8 + std::max(Pc * L, std::min(P * L, kModTaps)) * 8;
+}
+
+template <int BYTES>
+__device__ __forceinline__ void copy_async(float2 *dst, const float2 *src) {
+    if constexpr (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+template <int L, bool PREC>
+__device__ __forceinline__ void mod_tile(const int2 w, const SlotBlock &sb, const ChanParams &cp,
+                                         const ChanState *__restrict__ st, const float2 *__restrict__ x, int n,
+                                         const float2 *__restrict__ hist_arena, const float *__restrict__ taps_arena,
+                                         float2 *__restrict__ ext, float2 *smem) {
+    constexpr int R = kModR;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int chain = lane & 7, og = lane >> 3;
+    const int D = cp.decim, P = cp.nphase, pg = sb.pg, ng = sb.ng;
+    const uint64_t u0 = st[sb.slot].nco_q;
+    const uint64_t inc = cp.inc_q;
+    const float *tg = taps_arena + cp.taps_off;
+    const float2 *hist = hist_arena + cp.hist_off + sb.hist_sel * cp.hcap;
+    const int H = sb.hist_len;
+    const int s0 = D - sb.pc - 1;
+    float2 *z = smem + warp * kModBuf;
+    float2 *hc = smem + kModWarps * kModBuf;
+    const int gb = max(1, kModTaps / (pg * L));  // groups whose taps are held at a time
+
+    // The warp's 32 outputs of a tile: column m, phase p is sample a0 + m*D - p.
+    // Columns m0 .. m1-1 lie inside the block, with a sample to spare on each side.
+    struct Part {
+        int jw, nv, a0, m0, m1, cols;
+    };
+    auto part = [&](int tile) {
+        Part t;
+        t.jw = tile * kDenseOT + 32 * warp;
+        t.nv = min(32, sb.n_out - t.jw);
+        t.cols = t.nv + L - 1;
+        t.a0 = s0 + (t.jw - (L - 1)) * D;
+        t.m0 = t.a0 >= P ? 0 : min(t.cols, (P - t.a0 + D - 1) / D);
+        t.m1 = t.a0 + (t.cols - 1) * D + 1 < n ? t.cols : max(t.m0, t.cols - 1);
+        return t;
+    };
+    // chunk of phases p0 .. p0+np-1: phase p in position kModKC-1-(p-p0) + par of
+    // its column, par such that pairs of positions are aligned pairs of samples
+    const bool wide = (D & 1) == 0;
+    const int xal = (int)((reinterpret_cast<uintptr_t>(x) >> 3) & 1);
+    const int fc = lane >> 4, fq = 2 * (lane & 15);  // this lane's column and pair of a 16-byte copy
+    const int64_t fstep = 2 * (int64_t)D;
+    auto stage = [&](const Part &t, int p0, int np) {
+        const int ab = t.a0 - p0 - (kModKC - 1);
+        const int par = wide ? (ab + xal) & 1 : 0;
+        if (wide) {
+            if (fq + 1 >= kModKC - np + par) {
+                const float2 *src = x + ((int64_t)(ab - par + fq) + (int64_t)fc * D);
+                float2 *dst = z + fc * kModPitch + fq;
+                constexpr int full = (32 + L - 1) / 2, rest = (32 + L - 1) % 2;
+                if (t.m0 == 0 && t.m1 == 32 + L - 1) {
 #pragma unroll
-    for (int tt = 0; tt < R + L - 1; ++tt) {
-        const int c = lane * R + tt;
-        win[tt] = zrow[c + (c >> 3)];
-    }
-    float2 h[L];
-#pragma unroll
-    for (int u = 0; u < L; ++u) h[u] = hrow[u];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-#pragma unroll
-        for (int u = 0; u < L; ++u) {
-            const float2 z = win[r + L - 1 - u];
-            // (packed multiply-adds spill at three CTAs per SM: 1955 -> 2051 us)
-            acc[r].x = fmaf(h[u].x, z.x, fmaf(-h[u].y, z.y, acc[r].x));
-            acc[r].y = fmaf(h[u].x, z.y, fmaf(h[u].y, z.x, acc[r].y));
+                    for (int i = 0; i < full; ++i, src += fstep)
+                        copy_async<16>(dst + 2 * i * kModPitch + (i >> 2) * 8, src);
+                    if (fc < rest) copy_async<16>(dst + 2 * full * kModPitch + (full >> 2) * 8, src);
+                } else {
+                    for (int m = fc; m < t.m1; m += 2, src += fstep)
+                        if (m >= t.m0) copy_async<16>(z + m * kModPitch + (m >> 3) * 8 + fq, src);
+                }
+            }
+            if (par)
+                for (int m = t.m0 + lane; m < t.m1; m += 32)
+                    copy_async<16>(z + m * kModPitch + (m >> 3) * 8 + kModKC,
+                                   x + ((int64_t)(ab - 1 + kModKC) + (int64_t)m * D));
         }
+        // by 8 bytes: odd D, and the columns at the block's ends
+        if (lane >= kModKC - np) {
+            if (!wide) {
+                const float2 *src = x + ((int64_t)(ab + lane) + (int64_t)t.m0 * D);
+#pragma unroll 4
+                for (int m = t.m0; m < t.m1; ++m, src += D)
+                    copy_async<8>(z + m * kModPitch + (m >> 3) * 8 + lane, src);
+            }
+            auto edge = [&](int m) {
+                const int i = ab + lane + m * D;
+                float2 *dst = z + m * kModPitch + (m >> 3) * 8 + lane + par;
+                if (i >= 0 && i < n) {
+                    copy_async<8>(dst, x + i);
+                } else {
+                    float2 v = make_float2(0.f, 0.f);
+                    if (i < 0 && H + i >= 0)  // a carried sample is shifted already: undo its rotation
+                        v = cmulf(hist[H + i], q64_phasor((uint64_t)0 - (u0 + (uint64_t)(int64_t)i * inc)));
+                    *dst = v;
+                }
+            };
+            for (int m = 0; m < t.m0; ++m) edge(m);
+            for (int m = t.m1; m < t.cols; ++m) edge(m);
+        }
+        return par;
+    };
+
+    const int tile0 = w.y & kModTileMask, tiles = w.y >> kModTileBits;
+    for (int tile = tile0; tile < tile0 + tiles; ++tile) {
+        const Part t = part(tile);
+        const int jw = t.jw, nv = t.nv;
+        const bool live = nv > 0;
+        // this lane's output and its rotation exp(j phi(n_j)), taken by every group's share
+        const float2 ph = q64_phasor(u0 + (uint64_t)(int64_t)(s0 + (jw + lane) * D) * inc);
+        double2 acc64 = make_double2(0.0, 0.0);
+        float2 acc32 = make_float2(0.f, 0.f);
+
+        for (int g = 0, gt = 0; g < ng; ++g) {
+            const int p_lo = g * pg, Pc = min(pg, P - p_lo);
+            if (g == gt) {
+                gt += gb;
+                if (tile == tile0 || gb < ng) {
+                    if (g || tile != tile0) __syncthreads();  // every warp is done with the last groups' taps
+                    for (int i = threadIdx.x, e = (min(P, gt * pg) - p_lo) * L; i < e; i += kDenseThreads) {
+                        const int p = p_lo + i / L, u = i % L;
+                        const float h = tg[p * L + u];
+                        const float2 rot = q64_phasor((uint64_t)0 - (uint64_t)(p + u * D) * inc);
+                        hc[i] = make_float2(h * rot.x, h * rot.y);
+                    }
+                    __syncthreads();
+                }
+            }
+            if (live) {
+                const float2 *h2 = hc + (p_lo - (gt - gb) * pg) * L;
+                float2 acc[R];
+                double2 d[PREC ? R : 1];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    acc[r] = make_float2(0.f, 0.f);
+                    if constexpr (PREC) d[r] = make_double2(0.0, 0.0);
+                }
+                for (int c0 = 0; c0 < Pc; c0 += kModKC) {
+                    const int np = min(kModKC, Pc - c0);
+                    const int par = stage(t, p_lo + c0, np);
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    __syncwarp();
+                    const float2 *zc = z + og * (8 * kModPitch + 8) + (kModKC - 1) + par;
+#pragma unroll 1
+                    for (int s = 0; s < kModKC / 8; ++s) {
+                        const int pl = 8 * s + chain;
+                        if (pl < np) {
+                            float2 win[R + L - 1], h[L];
+#pragma unroll
+                            for (int t = 0; t < R + L - 1; ++t) win[t] = zc[t * kModPitch + (t >> 3) * 8 - pl];
+#pragma unroll
+                            for (int u = 0; u < L; ++u) h[u] = h2[(c0 + pl) * L + u];
+                            if constexpr (PREC) {
+#pragma unroll
+                                for (int r = 0; r < R; ++r) acc[r] = make_float2(0.f, 0.f);
+                            }
+#pragma unroll
+                            for (int r = 0; r < R; ++r) {
+#pragma unroll
+                                for (int u = 0; u < L; ++u) {
+                                    const float2 v = win[r + L - 1 - u];
+                                    acc[r].x = fmaf(h[u].x, v.x, fmaf(-h[u].y, v.y, acc[r].x));
+                                    acc[r].y = fmaf(h[u].x, v.y, fmaf(h[u].y, v.x, acc[r].y));
+                                }
+                            }
+                            if constexpr (PREC) {
+#pragma unroll
+                                for (int r = 0; r < R; ++r) {
+                                    d[r].x += (double)acc[r].x;
+                                    d[r].y += (double)acc[r].y;
+                                }
+                            }
+                        }
+                    }
+                    __syncwarp();
+                }
+                // the group's chains, in order, through the chunk just consumed
+                if constexpr (PREC) {
+                    double2 *z64 = reinterpret_cast<double2 *>(z);
+#pragma unroll
+                    for (int r = 0; r < R; ++r) z64[chain * kModRed + og * R + r] = d[r];
+                    __syncwarp();
+                    double2 v = make_double2(0.0, 0.0);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const double2 e = z64[k * kModRed + lane];
+                        v.x += e.x;
+                        v.y += e.y;
+                    }
+                    acc64.x += v.x * (double)ph.x - v.y * (double)ph.y;
+                    acc64.y += v.x * (double)ph.y + v.y * (double)ph.x;
+                } else {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) z[chain * kModRed + og * R + r] = acc[r];
+                    __syncwarp();
+                    float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const float2 e = z[k * kModRed + lane];
+                        v.x += e.x;
+                        v.y += e.y;
+                    }
+                    const float2 y = cmulf(v, ph);
+                    acc32.x += y.x;
+                    acc32.y += y.y;
+                }
+                __syncwarp();
+            }
+        }
+        if (lane < nv) ext[sb.ext_off + jw + lane] = PREC ? make_float2((float)acc64.x, (float)acc64.y) : acc32;
     }
 }
 
-__global__ void __launch_bounds__(kDenseThreads, 3)
+__global__ void __launch_bounds__(kDenseThreads, 2)
 k_extract_mod(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
               const ChanState *__restrict__ st, const float2 *__restrict__ x, int n,
               const float2 *__restrict__ hist_arena, const float *__restrict__ taps_arena,
@@ -1002,79 +1219,20 @@ k_extract_mod(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, 
     extern __shared__ float4 smemm4[];
     const int2 w = work[blockIdx.x];
     const SlotBlock sb = sbt[w.x];
+    if ((w.y & kModTileMask) * kDenseOT >= sb.n_out) return;
     const ChanParams &cp = prm[sb.slot];
-    const int j0 = w.y * kDenseOT;
-    if (j0 >= sb.n_out) return;
-    const int L = cp.plen, D = cp.decim;
-    const int M = kDenseOT + L - 1;
-    const int Mp = dense_row_stride(L);
-    int zb = (sb.pg * Mp * 8 + 15) & ~15;
-    if (zb < kRedBytes) zb = kRedBytes;
-    float2 *Z = reinterpret_cast<float2 *>(smemm4);
-    float2 *hc = reinterpret_cast<float2 *>(reinterpret_cast<char *>(smemm4) + zb);
-    const uint64_t u0 = st[sb.slot].nco_q;
-    const uint64_t inc = cp.inc_q;
-    const float *tg = taps_arena + cp.taps_off;
-    const int s0 = D - sb.pc - 1;
-    const float2 *hist = hist_arena + cp.hist_off + sb.hist_sel * cp.hcap;
-    const int H = sb.hist_len;
-    auto row = [&](int pp, int lane, float2 *acc) {
-        const float2 *zrow = Z + pp * Mp;
-        const float2 *hrow = hc + pp * L;
-        switch (L) {
-        case 1: mod_row<1>(zrow, hrow, lane, acc); break;
-        case 2: mod_row<2>(zrow, hrow, lane, acc); break;
-        case 3: mod_row<3>(zrow, hrow, lane, acc); break;
-        default: mod_row<4>(zrow, hrow, lane, acc); break;
-        }
-    };
-    const int nv = sb.n_out - j0;
-    const int o = (int)threadIdx.x;  // this thread's output of the tile
-    // its rotation exp(j phi(n_j)), taken by every group's share
-    const float2 ph = q64_phasor(u0 + (uint64_t)(int64_t)(s0 + (j0 + o) * D) * inc);
-    double2 acc64 = make_double2(0.0, 0.0);
-    float2 acc = make_float2(0.f, 0.f);
-    for (int g = 0; g < sb.ng; ++g) {
-        const int p_lo = g * sb.pg;
-        const int Pc = min(sb.pg, cp.nphase - p_lo);
-        if (g) __syncthreads();  // the last group's reduction has read Z and its rows hc
-        for (int i = threadIdx.x; i < Pc * L; i += kDenseThreads) {
-            const int pp = i / L, u = i - pp * L;
-            const int k = p_lo + pp + u * D;
-            const float h = tg[(p_lo + pp) * L + u];
-            const float2 t = q64_phasor((uint64_t)0 - (uint64_t)k * inc);
-            hc[i] = make_float2(h * t.x, h * t.y);
-        }
-        // raw samples: Z[pp][m] = x(cb0 + m*D + r), pp = Pc-1-r
-        const int cb0 = s0 + (j0 - (L - 1)) * D - p_lo - Pc + 1;
-        const bool interior = cb0 >= 0 && cb0 + (M - 1) * D + Pc <= n;
-        if (interior) {
-            stage_columns(Pc, M, Mp, D, cb0, Z, [&](int i, int, int) { return __ldg(x + i); });
-        } else {
-            stage_columns(Pc, M, Mp, D, cb0, Z, [&](int i, int, int) {
-                if (i >= n) return make_float2(0.f, 0.f);
-                if (i >= 0) return __ldg(x + i);
-                const int hi = H + i;
-                // a carried sample is shifted already: undo its rotation
-                return hi >= 0 ? cmulf(hist[hi], q64_phasor((uint64_t)0 - (u0 + (uint64_t)(int64_t)i * inc)))
-                               : make_float2(0.f, 0.f);
-            });
-        }
-        __syncthreads();
-        if (cp.precise_sum) {
-            tile_sum<true>(Pc, row, Z, [&](int, double2 v) {
-                acc64.x += v.x * (double)ph.x - v.y * (double)ph.y;
-                acc64.y += v.x * (double)ph.y + v.y * (double)ph.x;
-            });
-        } else {
-            tile_sum<false>(Pc, row, Z, [&](int, float2 v) {
-                const float2 y = cmulf(v, ph);
-                acc.x += y.x;
-                acc.y += y.y;
-            });
-        }
+    float2 *smem = reinterpret_cast<float2 *>(smemm4);
+#define GPUD_MOD(LL)                                                                                      \
+    if (cp.precise_sum) mod_tile<LL, true>(w, sb, cp, st, x, n, hist_arena, taps_arena, ext, smem);       \
+    else mod_tile<LL, false>(w, sb, cp, st, x, n, hist_arena, taps_arena, ext, smem);                     \
+    break;
+    switch (cp.plen) {  // uniform per CTA
+    case 1: GPUD_MOD(1)
+    case 2: GPUD_MOD(2)
+    case 3: GPUD_MOD(3)
+    default: GPUD_MOD(4)
     }
-    if (o < nv) ext[sb.ext_off + j0 + o] = cp.precise_sum ? make_float2((float)acc64.x, (float)acc64.y) : acc;
+#undef GPUD_MOD
 }
 
 // ===========================================================================
