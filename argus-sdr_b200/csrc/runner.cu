@@ -114,10 +114,14 @@ int wide_smem_bytes_host(int T);
 int group_smem_bytes_host(int Pc, int L);
 int mod_smem_bytes_host(int Pc, int L);
 int mod_launch_bytes_host(int P, int Pc, int L);
+int rot_launch_bytes_host(int P, int pg, int L);
 int mod_item(int tile, int tiles);
 cudaError_t launch_extract_group(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
                                  const ChanParams *prm, const ChanState *st, const float2 *x, int n,
                                  const float2 *hist, const float *taps, float2 *ext);
+cudaError_t launch_extract_rot(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
+                               const ChanParams *prm, const ChanState *st, const float2 *x, int n,
+                               const float2 *hist, const float *taps, float2 *ext);
 cudaError_t launch_extract_mod(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
                                const ChanParams *prm, const ChanState *st, const float2 *x, int n,
                                const float2 *hist, const float *taps, float2 *ext);
@@ -153,6 +157,7 @@ constexpr int kWideTile = 32;                 // outputs per work item of the wa
 constexpr int kGroupSmemTarget = 100 * 1024;  // two CTAs per SM
 constexpr int kModSmemTarget = 72 * 1024;     // three CTAs per SM
 constexpr int kModMaxL = 4;
+constexpr int kRotMaxL = 16;  // longest arm of the phase groups whose warps work alone (k_extract_rot)
 constexpr int kPllMaxIters = 64;
 #ifndef GPUD_FRAMES
 #define GPUD_FRAMES 3
@@ -281,9 +286,11 @@ struct BlockPlan {
     int bank_max_total = 0;               // largest T x cpad of a bank
     std::vector<int2> w_wide;
     int wide_smem = 0;
-    std::vector<int2> w_group;  // (entry, 256-output tile): one CTA takes the tile's phase groups in turn
+    std::vector<int2> w_group;  // (entry, 256-output tile) of long arms: one CTA takes the tile's phase groups in turn
     int group_smem = 0;
-    std::vector<int2> w_mod;    // (entry, 256-output tile) of the modulated short-arm form, likewise
+    std::vector<int2> w_rot;    // (entry, first tile | tiles) of phase groups with arms of up to kRotMaxL taps
+    int rot_smem = 0;
+    std::vector<int2> w_mod;    // (entry, first tile | tiles) of the modulated short-arm form
     int mod_smem = 0;
     std::vector<int2> w_demod, w_am, w_fir, w_out, w_rds;
     int rds_smem = 0;
@@ -1055,6 +1062,8 @@ static void finish_plan(gpud_runner *r, BlockPlan &pl) {
     pl.wide_smem = 0;
     pl.w_group.clear();
     pl.group_smem = 0;
+    pl.w_rot.clear();
+    pl.rot_smem = 0;
     pl.w_mod.clear();
     pl.mod_smem = 0;
     pl.w_demod.clear();
@@ -1068,17 +1077,7 @@ static void finish_plan(gpud_runner *r, BlockPlan &pl) {
     pl.rds_smem = 0;
     std::vector<char> grouped = plan_gemm_groups(r, pl);
     const std::vector<int> banked = plan_bank_groups(r, pl, grouped);
-    // Tiles per work item of the modulated form: the item builds its channel's
-    // T modulated taps once, so with few phases (little to do per tile) it takes
-    // several, unless the block has too few tiles to keep every SM at work.
-    int64_t mod_total = 0;
-    for (int i = 0; i < (int)pl.sbs.size(); ++i)
-        if (r->slots[(size_t)pl.sbs[(size_t)i].slot].ext_kind == 3 && banked[(size_t)i] < 0)
-            mod_total += (pl.sbs[(size_t)i].n_out + dense_tile() - 1) / dense_tile();
-    std::vector<int> mod_rows;
-    auto mod_tiles = [&](const Slot &s) {
-        return mod_total < 16 * (int64_t)r->num_sms ? 1 : std::min(8, std::max(1, 256 / s.P));
-    };
+    std::vector<int> mod_rows, rot_rows;
     for (int i = 0; i < (int)pl.sbs.size(); ++i) {
         const SlotBlock &sb = pl.sbs[(size_t)i];
         Slot &s = r->slots[(size_t)sb.slot];
@@ -1097,7 +1096,10 @@ static void finish_plan(gpud_runner *r, BlockPlan &pl) {
                 pl.dense_smem[s.L] = std::max(pl.dense_smem[s.L], dense_smem_bytes_host(s.P, s.L));
                 pl.dense_pmax[s.L] = std::max(pl.dense_pmax[s.L], s.P);
             } else if (s.ext_kind == 2 || s.ext_kind == 3) {
-                if (s.ext_kind == 2) {
+                if (s.ext_kind == 2 && s.L <= kRotMaxL) {
+                    rot_rows.push_back(i);
+                    pl.rot_smem = std::max(pl.rot_smem, rot_launch_bytes_host(s.P, s.pg, s.L));
+                } else if (s.ext_kind == 2) {
                     for (int t = 0; t * dense_tile() < sb.n_out; ++t) pl.w_group.push_back(make_int2(i, t));
                     pl.group_smem = std::max(pl.group_smem, group_smem_bytes_host(s.pg, s.L));
                 } else {
@@ -1141,18 +1143,28 @@ static void finish_plan(gpud_runner *r, BlockPlan &pl) {
         });
     };
     longest_first(pl.w_group);
-    // the modulated form's rows by code path (the CTAs of an SM share its
-    // instruction cache), the longest first
-    auto mod_key = [&](int row) {
-        const Slot &s = r->slots[(size_t)pl.sbs[(size_t)row].slot];
-        return std::make_tuple(-s.L, precise_sum(s.spec), -(int64_t)s.P);
+    // The forms in which every warp works by itself: rows by code path (the CTAs of
+    // an SM share its instruction cache), the longest first.  A work item prepares
+    // its channel's T taps once, so with few phases (little to do per tile) it takes
+    // several tiles, unless the block has too few to keep every SM at work.
+    auto warp_items = [&](std::vector<int> &rows, std::vector<int2> &wl) {
+        auto slot = [&](int row) -> const Slot & { return r->slots[(size_t)pl.sbs[(size_t)row].slot]; };
+        auto tiles = [&](int row) { return (pl.sbs[(size_t)row].n_out + dense_tile() - 1) / dense_tile(); };
+        auto key = [&](int row) {
+            const Slot &s = slot(row);
+            return std::make_tuple(-s.L, precise_sum(s.spec), -s.P);
+        };
+        std::stable_sort(rows.begin(), rows.end(), [&](int a, int b) { return key(a) < key(b); });
+        int64_t total = 0;
+        for (int row : rows) total += tiles(row);
+        for (int row : rows) {
+            const int k = total < 16 * (int64_t)r->num_sms ? 1 : std::min(8, std::max(1, 256 / slot(row).P));
+            for (int t = 0, nt = tiles(row); t < nt; t += k)
+                wl.push_back(make_int2(row, mod_item(t, std::min(k, nt - t))));
+        }
     };
-    std::stable_sort(mod_rows.begin(), mod_rows.end(), [&](int a, int b) { return mod_key(a) < mod_key(b); });
-    for (int row : mod_rows) {
-        const int nt = (pl.sbs[(size_t)row].n_out + dense_tile() - 1) / dense_tile();
-        const int k = mod_tiles(r->slots[(size_t)pl.sbs[(size_t)row].slot]);
-        for (int t = 0; t < nt; t += k) pl.w_mod.push_back(make_int2(row, mod_item(t, std::min(k, nt - t))));
-    }
+    warp_items(rot_rows, pl.w_rot);
+    warp_items(mod_rows, pl.w_mod);
 }
 
 static int ensure_frame(gpud_runner *r, Frame &f, const BlockPlan &pl) {
@@ -1199,7 +1211,7 @@ static int ensure_frame(gpud_runner *r, Frame &f, const BlockPlan &pl) {
     for (int L = 0; L <= kDenseMaxL; ++L) nw += pl.w_dense[L].size();
     nw += pl.w_wide.size() + pl.w_demod.size() + pl.w_am.size() + pl.w_fir.size() + pl.w_out.size() +
           pl.w_rds.size() + pl.w_aud.size() + pl.w_dec.size() + pl.w_group.size() +
-          pl.w_mod.size() + pl.w_free.size() + pl.w_gemm.size() + pl.w_bank.size();
+          pl.w_rot.size() + pl.w_mod.size() + pl.w_free.size() + pl.w_gemm.size() + pl.w_bank.size();
     size_t dneed = align256(pl.sbs.size() * sizeof(SlotBlock)) + align256(nw * sizeof(int2)) +
                    align256(pl.pll_list.size() * 4) + align256(pl.aud_list.size() * 4) +
                    align256(pl.groups.size() * sizeof(GemmGroup)) + align256(pl.gmembers.size() * 4) +
@@ -1355,7 +1367,7 @@ static int enqueue_block(gpud_runner *r, Frame &f, const Frame *prev, BlockPlan 
     };
     size_t o_wide = put(pl.w_wide), o_dem = put(pl.w_demod), o_am = put(pl.w_am), o_fir = put(pl.w_fir),
            o_out = put(pl.w_out), o_rds = put(pl.w_rds), o_waud = put(pl.w_aud), o_wdec = put(pl.w_dec),
-           o_grp = put(pl.w_group), o_mod = put(pl.w_mod), o_free = put(pl.w_free),
+           o_grp = put(pl.w_group), o_rot = put(pl.w_rot), o_mod = put(pl.w_mod), o_free = put(pl.w_free),
            o_gemm = put(pl.w_gemm), o_bank = put(pl.w_bank);
     size_t o_pll = o_w + align256(cnt * sizeof(int2));
     std::memcpy(hd + o_pll, pl.pll_list.data(), pl.pll_list.size() * 4);
@@ -1483,8 +1495,13 @@ static int enqueue_block(gpud_runner *r, Frame &f, const Frame *prev, BlockPlan 
                                x_dev, f.d_bank, d_ext));
         nl++;
     }
+    if (!pl.w_group.empty() || !pl.w_rot.empty()) prof_mark(r, f, "extract_group");
+    if (!pl.w_rot.empty()) {
+        CK(launch_extract_rot((int)pl.w_rot.size(), pl.rot_smem, f.s, d_w + o_rot, d_sb, r->d_prm, r->d_st, x_dev,
+                              n, r->d_hist, r->d_taps, d_ext));
+        nl++;
+    }
     if (!pl.w_group.empty()) {
-        prof_mark(r, f, "extract_group");
         CK(launch_extract_group((int)pl.w_group.size(), pl.group_smem, f.s, d_w + o_grp, d_sb, r->d_prm, r->d_st,
                                 x_dev, n, r->d_hist, r->d_taps, d_ext));
         nl++;

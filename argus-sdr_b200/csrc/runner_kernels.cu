@@ -918,14 +918,7 @@ k_extract_group(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt
     auto row = [&](int pp, int lane, float2 *acc) {
         const float2 *zrow = Z + pp * gt.Mp;
         const float *hrow = tsm + pp * gt.Le;
-        switch (L) {
-#define GPUD_ROW(LL) \
-    case LL: group_row<LL>(zrow, hrow, lane, acc); break;
-            GPUD_ROW(1) GPUD_ROW(2) GPUD_ROW(3) GPUD_ROW(4) GPUD_ROW(5) GPUD_ROW(6) GPUD_ROW(7) GPUD_ROW(8)
-            GPUD_ROW(9) GPUD_ROW(10) GPUD_ROW(11) GPUD_ROW(12) GPUD_ROW(13) GPUD_ROW(14) GPUD_ROW(15) GPUD_ROW(16)
-#undef GPUD_ROW
-        default: group_row_long(zrow, hrow, gt.Le, lane, acc); break;
-        }
+        group_row_long(zrow, hrow, gt.Le, lane, acc);
     };
     const int nv = sb.n_out - gt.j0;
     const int o = (int)threadIdx.x;  // this thread's output of the tile
@@ -1011,6 +1004,96 @@ __device__ __forceinline__ void copy_async(float2 *dst, const float2 *src) {
         asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
+// A warp's 32 outputs of a tile: column m (of 32 + L - 1), phase p is sample
+// a0 + m*D - p.  Columns m0 .. m1-1 lie inside the block, with a sample to spare
+// on each side.
+struct WarpPart {
+    int jw, nv, a0, m0, m1, cols;
+};
+
+__device__ __forceinline__ WarpPart warp_part(int tile, int warp, int L, int D, int P, int s0, int n_out, int n) {
+    WarpPart t;
+    t.jw = tile * kDenseOT + 32 * warp;
+    t.nv = min(32, n_out - t.jw);
+    t.cols = t.nv + L - 1;
+    t.a0 = s0 + (t.jw - (L - 1)) * D;
+    t.m0 = t.a0 >= P ? 0 : min(t.cols, (P - t.a0 + D - 1) / D);
+    t.m1 = t.a0 + (t.cols - 1) * D + 1 < n ? t.cols : max(t.m0, t.cols - 1);
+    return t;
+}
+
+// Stage phases p0 .. p0+np-1 (np <= KC) of a part's columns: phase p in position
+// KC-1-(p-p0) + par of its column, par (returned) such that pairs of positions are
+// aligned pairs of samples.  edge(i) is the value of sample i outside the block.
+template <int L, int KC, class Edge>
+__device__ __forceinline__ int stage_part(const WarpPart &t, float2 *z, int p0, int np, int D,
+                                          const float2 *__restrict__ x, int n, const Edge &edge) {
+    constexpr int pitch = KC + 2, per = 64 / KC, C = 32 + L - 1;  // columns per warp-wide 16-byte copy; all
+    const int lane = threadIdx.x & 31;
+    const bool wide = (D & 1) == 0;
+    const int ab = t.a0 - p0 - (KC - 1);
+    const int par = wide ? (ab + (int)(reinterpret_cast<uintptr_t>(x) >> 3)) & 1 : 0;
+    if (wide) {
+        const int fc = lane / (KC / 2), fq = 2 * (lane % (KC / 2));
+        const int64_t step = per * (int64_t)D;
+        if (fq + 1 >= KC - np + par) {
+            const float2 *src = x + ((int64_t)(ab - par + fq) + (int64_t)fc * D);
+            float2 *dst = z + fc * pitch + fq;
+            constexpr int full = C / per, rest = C % per;
+            if (t.m0 == 0 && t.m1 == C) {
+#pragma unroll
+                for (int i = 0; i < full; ++i, src += step)
+                    copy_async<16>(dst + per * i * pitch + (per * i >> 3) * 8, src);
+                if (fc < rest) copy_async<16>(dst + per * full * pitch + (per * full >> 3) * 8, src);
+            } else {
+                for (int m = fc; m < t.m1; m += per, src += step)
+                    if (m >= t.m0) copy_async<16>(z + m * pitch + (m >> 3) * 8 + fq, src);
+            }
+        }
+        if (par)
+            for (int m = t.m0 + lane; m < t.m1; m += 32)
+                copy_async<16>(z + m * pitch + (m >> 3) * 8 + KC, x + ((int64_t)(ab - 1 + KC) + (int64_t)m * D));
+    }
+    // by 8 bytes: odd D, and the columns at the block's ends
+    const int q = lane % KC, c = lane / KC;
+    if (q >= KC - np) {
+        if (!wide) {
+            const float2 *src = x + ((int64_t)(ab + q) + (int64_t)(t.m0 + c) * D);
+#pragma unroll 4
+            for (int m = t.m0 + c; m < t.m1; m += 32 / KC, src += 32 / KC * D)
+                copy_async<8>(z + m * pitch + (m >> 3) * 8 + q, src);
+        }
+        auto end = [&](int m) {
+            const int i = ab + q + m * D;
+            float2 *dst = z + m * pitch + (m >> 3) * 8 + q + par;
+            if (i >= 0 && i < n) copy_async<8>(dst, x + i);
+            else *dst = edge(i);
+        };
+        for (int m = c; m < t.m0; m += 32 / KC) end(m);
+        for (int m = t.m1 + c; m < t.cols; m += 32 / KC) end(m);
+    }
+    return par;
+}
+
+// Sum of the eight chains of this lane's output, in order; lane chain + 8 og holds
+// the outputs 8 og .. 8 og + 7 of its chain.  red: the consumed chunk.
+template <class V>
+__device__ __forceinline__ V chain_sum(V *red, const V (&part)[kModR], int chain, int og, int lane) {
+#pragma unroll
+    for (int r = 0; r < kModR; ++r) red[chain * kModRed + og * kModR + r] = part[r];
+    __syncwarp();
+    V v;
+    v.x = v.y = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const V e = red[k * kModRed + lane];
+        v.x += e.x;
+        v.y += e.y;
+    }
+    __syncwarp();
+    return v;
+}
+
 template <int L, bool PREC>
 __device__ __forceinline__ void mod_tile(const int2 w, const SlotBlock &sb, const ChanParams &cp,
                                          const ChanState *__restrict__ st, const float2 *__restrict__ x, int n,
@@ -1030,79 +1113,14 @@ __device__ __forceinline__ void mod_tile(const int2 w, const SlotBlock &sb, cons
     float2 *hc = smem + kModWarps * kModBuf;
     const int gb = max(1, kModTaps / (pg * L));  // groups whose taps are held at a time
 
-    // The warp's 32 outputs of a tile: column m, phase p is sample a0 + m*D - p.
-    // Columns m0 .. m1-1 lie inside the block, with a sample to spare on each side.
-    struct Part {
-        int jw, nv, a0, m0, m1, cols;
-    };
-    auto part = [&](int tile) {
-        Part t;
-        t.jw = tile * kDenseOT + 32 * warp;
-        t.nv = min(32, sb.n_out - t.jw);
-        t.cols = t.nv + L - 1;
-        t.a0 = s0 + (t.jw - (L - 1)) * D;
-        t.m0 = t.a0 >= P ? 0 : min(t.cols, (P - t.a0 + D - 1) / D);
-        t.m1 = t.a0 + (t.cols - 1) * D + 1 < n ? t.cols : max(t.m0, t.cols - 1);
-        return t;
-    };
-    // chunk of phases p0 .. p0+np-1: phase p in position kModKC-1-(p-p0) + par of
-    // its column, par such that pairs of positions are aligned pairs of samples
-    const bool wide = (D & 1) == 0;
-    const int xal = (int)((reinterpret_cast<uintptr_t>(x) >> 3) & 1);
-    const int fc = lane >> 4, fq = 2 * (lane & 15);  // this lane's column and pair of a 16-byte copy
-    const int64_t fstep = 2 * (int64_t)D;
-    auto stage = [&](const Part &t, int p0, int np) {
-        const int ab = t.a0 - p0 - (kModKC - 1);
-        const int par = wide ? (ab + xal) & 1 : 0;
-        if (wide) {
-            if (fq + 1 >= kModKC - np + par) {
-                const float2 *src = x + ((int64_t)(ab - par + fq) + (int64_t)fc * D);
-                float2 *dst = z + fc * kModPitch + fq;
-                constexpr int full = (32 + L - 1) / 2, rest = (32 + L - 1) % 2;
-                if (t.m0 == 0 && t.m1 == 32 + L - 1) {
-#pragma unroll
-                    for (int i = 0; i < full; ++i, src += fstep)
-                        copy_async<16>(dst + 2 * i * kModPitch + (i >> 2) * 8, src);
-                    if (fc < rest) copy_async<16>(dst + 2 * full * kModPitch + (full >> 2) * 8, src);
-                } else {
-                    for (int m = fc; m < t.m1; m += 2, src += fstep)
-                        if (m >= t.m0) copy_async<16>(z + m * kModPitch + (m >> 3) * 8 + fq, src);
-                }
-            }
-            if (par)
-                for (int m = t.m0 + lane; m < t.m1; m += 32)
-                    copy_async<16>(z + m * kModPitch + (m >> 3) * 8 + kModKC,
-                                   x + ((int64_t)(ab - 1 + kModKC) + (int64_t)m * D));
-        }
-        // by 8 bytes: odd D, and the columns at the block's ends
-        if (lane >= kModKC - np) {
-            if (!wide) {
-                const float2 *src = x + ((int64_t)(ab + lane) + (int64_t)t.m0 * D);
-#pragma unroll 4
-                for (int m = t.m0; m < t.m1; ++m, src += D)
-                    copy_async<8>(z + m * kModPitch + (m >> 3) * 8 + lane, src);
-            }
-            auto edge = [&](int m) {
-                const int i = ab + lane + m * D;
-                float2 *dst = z + m * kModPitch + (m >> 3) * 8 + lane + par;
-                if (i >= 0 && i < n) {
-                    copy_async<8>(dst, x + i);
-                } else {
-                    float2 v = make_float2(0.f, 0.f);
-                    if (i < 0 && H + i >= 0)  // a carried sample is shifted already: undo its rotation
-                        v = cmulf(hist[H + i], q64_phasor((uint64_t)0 - (u0 + (uint64_t)(int64_t)i * inc)));
-                    *dst = v;
-                }
-            };
-            for (int m = 0; m < t.m0; ++m) edge(m);
-            for (int m = t.m1; m < t.cols; ++m) edge(m);
-        }
-        return par;
+    auto edge = [&](int i) {  // a carried sample is shifted already: undo its rotation
+        return i < 0 && H + i >= 0 ? cmulf(hist[H + i], q64_phasor((uint64_t)0 - (u0 + (uint64_t)(int64_t)i * inc)))
+                                   : make_float2(0.f, 0.f);
     };
 
     const int tile0 = w.y & kModTileMask, tiles = w.y >> kModTileBits;
     for (int tile = tile0; tile < tile0 + tiles; ++tile) {
-        const Part t = part(tile);
+        const WarpPart t = warp_part(tile, warp, L, D, P, s0, sb.n_out, n);
         const int jw = t.jw, nv = t.nv;
         const bool live = nv > 0;
         // this lane's output and its rotation exp(j phi(n_j)), taken by every group's share
@@ -1136,7 +1154,7 @@ __device__ __forceinline__ void mod_tile(const int2 w, const SlotBlock &sb, cons
                 }
                 for (int c0 = 0; c0 < Pc; c0 += kModKC) {
                     const int np = min(kModKC, Pc - c0);
-                    const int par = stage(t, p_lo + c0, np);
+                    const int par = stage_part<L, kModKC>(t, z, p_lo + c0, np, D, x, n, edge);
                     asm volatile("cp.async.wait_all;" ::: "memory");
                     __syncwarp();
                     const float2 *zc = z + og * (8 * kModPitch + 8) + (kModKC - 1) + par;
@@ -1173,37 +1191,15 @@ __device__ __forceinline__ void mod_tile(const int2 w, const SlotBlock &sb, cons
                     }
                     __syncwarp();
                 }
-                // the group's chains, in order, through the chunk just consumed
                 if constexpr (PREC) {
-                    double2 *z64 = reinterpret_cast<double2 *>(z);
-#pragma unroll
-                    for (int r = 0; r < R; ++r) z64[chain * kModRed + og * R + r] = d[r];
-                    __syncwarp();
-                    double2 v = make_double2(0.0, 0.0);
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const double2 e = z64[k * kModRed + lane];
-                        v.x += e.x;
-                        v.y += e.y;
-                    }
+                    const double2 v = chain_sum(reinterpret_cast<double2 *>(z), d, chain, og, lane);
                     acc64.x += v.x * (double)ph.x - v.y * (double)ph.y;
                     acc64.y += v.x * (double)ph.y + v.y * (double)ph.x;
                 } else {
-#pragma unroll
-                    for (int r = 0; r < R; ++r) z[chain * kModRed + og * R + r] = acc[r];
-                    __syncwarp();
-                    float2 v = make_float2(0.f, 0.f);
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const float2 e = z[k * kModRed + lane];
-                        v.x += e.x;
-                        v.y += e.y;
-                    }
-                    const float2 y = cmulf(v, ph);
+                    const float2 y = cmulf(chain_sum(z, acc, chain, og, lane), ph);
                     acc32.x += y.x;
                     acc32.y += y.y;
                 }
-                __syncwarp();
             }
         }
         if (lane < nv) ext[sb.ext_off + jw + lane] = PREC ? make_float2((float)acc64.x, (float)acc64.y) : acc32;
@@ -1233,6 +1229,184 @@ k_extract_mod(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, 
     default: GPUD_MOD(4)
     }
 #undef GPUD_MOD
+}
+
+// Phase groups of arms up to 16 taps with the warp layout of the modulated form:
+// the copied samples are rotated in place (sample r of column m by A[m] B[r],
+// the phase group's two exact phasors), then each lane runs its chain of rows.
+// Chunks hold 32 phases, 16 for arms above 8 taps (whose windows have more
+// columns), so two CTAs fit on an SM.  Arms above 16 taps stay with the whole CTA
+// on one tile: a warp's 32 + L - 1 columns would be staged for 32 outputs.
+// 480 phase-grouped channels among 2048 (300 with arms of 5..11 taps): 2057 us
+// with every tile staged by its whole CTA through registers, 679 + 1182 us (the
+// long arms) now.
+__host__ __device__ constexpr int rot_kc(int L) { return L > 8 ? 16 : 32; }
+__host__ __device__ constexpr int rot_buf(int L) {  // float2 entries of a warp's chunk
+    return (32 + L - 1) * (rot_kc(L) + 2) + ((32 + L - 2) >> 3) * 8;
+}
+constexpr int kRotMaxL = 16;
+constexpr int kRotCols = 32 + kRotMaxL;  // column phasors of a warp
+constexpr int kRotTaps = 1024;           // taps held at a time
+static_assert(rot_buf(9) >= 2 * 8 * kModRed && rot_buf(1) >= 2 * 8 * kModRed, "float64 sums of eight chains");
+
+int rot_launch_bytes_host(int P, int pg, int L) {
+    return (kModWarps * (rot_buf(L) + kRotCols) + pg) * 8 + std::max(pg * L, std::min(P * L, kRotTaps)) * 4;
+}
+
+template <int L, bool PREC>
+__device__ __forceinline__ void rot_tile(const int2 w, const SlotBlock &sb, const ChanParams &cp,
+                                         const ChanState *__restrict__ st, const float2 *__restrict__ x, int n,
+                                         const float2 *__restrict__ hist_arena, const float *__restrict__ taps_arena,
+                                         float2 *__restrict__ ext, float2 *smem) {
+    constexpr int R = kModR, KC = rot_kc(L), pitch = KC + 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int chain = lane & 7, og = lane >> 3;
+    const int D = cp.decim, P = cp.nphase, pg = sb.pg, ng = sb.ng;
+    const uint64_t u0 = st[sb.slot].nco_q;
+    const uint64_t inc = cp.inc_q;
+    const float *tg = taps_arena + cp.taps_off;
+    const float2 *hist = hist_arena + cp.hist_off + sb.hist_sel * cp.hcap;
+    const int H = sb.hist_len;
+    const int s0 = D - sb.pc - 1;
+    float2 *z = smem + warp * rot_buf(L);
+    float2 *A = smem + kModWarps * rot_buf(L) + warp * kRotCols;
+    float2 *B = smem + kModWarps * (rot_buf(L) + kRotCols);
+    float *hs = reinterpret_cast<float *>(B + pg);
+    const int gb = max(1, kRotTaps / (pg * L));  // groups whose taps are held at a time
+    auto edge = [&](int i) { return i < 0 && H + i >= 0 ? hist[H + i] : make_float2(0.f, 0.f); };  // shifted already
+
+    for (int r = threadIdx.x; r < pg; r += kDenseThreads) B[r] = q64_phasor((uint64_t)r * inc);
+    const int tile0 = w.y & kModTileMask, tiles = w.y >> kModTileBits;
+    for (int tile = tile0; tile < tile0 + tiles; ++tile) {
+        const WarpPart t = warp_part(tile, warp, L, D, P, s0, sb.n_out, n);
+        const bool live = t.nv > 0;
+        double2 acc64 = make_double2(0.0, 0.0);
+        float2 acc32 = make_float2(0.f, 0.f);
+        for (int g = 0, gt = 0; g < ng; ++g) {
+            const int p_lo = g * pg, Pc = min(pg, P - p_lo);
+            if (g == gt) {
+                gt += gb;
+                if (tile == tile0 || gb < ng) {
+                    if (g || tile != tile0) __syncthreads();  // every warp is done with the last groups' taps
+                    for (int i = threadIdx.x, e = (min(P, gt * pg) - p_lo) * L; i < e; i += kDenseThreads)
+                        hs[i] = tg[p_lo * L + i];
+                    __syncthreads();
+                }
+            }
+            if (live) {
+                const float *h2 = hs + (p_lo - (gt - gb) * pg) * L;
+                for (int m = lane; m < t.cols; m += 32)
+                    A[m] = q64_phasor(u0 + (uint64_t)(int64_t)(t.a0 - (p_lo + Pc - 1) + m * D) * inc);
+                float2 acc[R];
+                double2 d[PREC ? R : 1];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    acc[r] = make_float2(0.f, 0.f);
+                    if constexpr (PREC) d[r] = make_double2(0.0, 0.0);
+                }
+                for (int c0 = 0; c0 < Pc; c0 += KC) {
+                    const int np = min(KC, Pc - c0);
+                    const int par = stage_part<L, KC>(t, z, p_lo + c0, np, D, x, n, edge);
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    __syncwarp();
+                    {
+                        // the rotation: this lane's position of every (32/KC)-th column
+                        constexpr int S = 32 / KC, U = 4;
+                        const int q = lane % KC, c = lane / KC;
+                        if (q >= KC - np) {
+                            const float2 b = B[Pc - 1 - (c0 + KC - 1 - q)];
+                            float2 *zq = z + q + par;
+                            int m = c;
+                            for (; m < t.m0; m += S) {  // carried samples stay
+                                float2 &v = zq[m * pitch + (m >> 3) * 8];
+                                if (t.a0 - (p_lo + c0 + KC - 1) + q + m * D >= 0) v = cmulf(v, cmulf(A[m], b));
+                            }
+                            for (; m < t.cols; m += S * U) {
+                                float2 v[U];
+#pragma unroll
+                                for (int u = 0; u < U; ++u) {
+                                    const int mu = m + S * u;
+                                    if (mu < t.cols) v[u] = cmulf(zq[mu * pitch + (mu >> 3) * 8], cmulf(A[mu], b));
+                                }
+#pragma unroll
+                                for (int u = 0; u < U; ++u) {
+                                    const int mu = m + S * u;
+                                    if (mu < t.cols) zq[mu * pitch + (mu >> 3) * 8] = v[u];
+                                }
+                            }
+                        }
+                        __syncwarp();
+                    }
+                    const float2 *zc = z + og * (8 * pitch + 8) + (KC - 1) + par;
+#pragma unroll 1
+                    for (int k = 0; k < KC / 8; ++k) {
+                        const int pl = 8 * k + chain;
+                        if (pl < np) {
+                            float2 win[R + L - 1];
+                            float h[L];
+#pragma unroll
+                            for (int i = 0; i < R + L - 1; ++i) win[i] = zc[i * pitch + (i >> 3) * 8 - pl];
+#pragma unroll
+                            for (int u = 0; u < L; ++u) h[u] = h2[(c0 + pl) * L + u];
+                            if constexpr (PREC) {
+#pragma unroll
+                                for (int r = 0; r < R; ++r) acc[r] = make_float2(0.f, 0.f);
+                            }
+#pragma unroll
+                            for (int r = 0; r < R; ++r) {
+#pragma unroll
+                                for (int u = 0; u < L; ++u)
+                                    acc[r] = ffma2(make_float2(h[u], h[u]), win[r + L - 1 - u], acc[r]);
+                            }
+                            if constexpr (PREC) {
+#pragma unroll
+                                for (int r = 0; r < R; ++r) {
+                                    d[r].x += (double)acc[r].x;
+                                    d[r].y += (double)acc[r].y;
+                                }
+                            }
+                        }
+                    }
+                    __syncwarp();
+                }
+                if constexpr (PREC) {
+                    const double2 v = chain_sum(reinterpret_cast<double2 *>(z), d, chain, og, lane);
+                    acc64.x += v.x;
+                    acc64.y += v.y;
+                } else {
+                    const float2 v = chain_sum(z, acc, chain, og, lane);
+                    acc32.x += v.x;
+                    acc32.y += v.y;
+                }
+            }
+        }
+        if (lane < t.nv) ext[sb.ext_off + t.jw + lane] = PREC ? make_float2((float)acc64.x, (float)acc64.y) : acc32;
+    }
+}
+
+__global__ void __launch_bounds__(kDenseThreads, 2)
+k_extract_rot(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
+              const ChanState *__restrict__ st, const float2 *__restrict__ x, int n,
+              const float2 *__restrict__ hist_arena, const float *__restrict__ taps_arena,
+              float2 *__restrict__ ext) {
+    dependency_wait();
+    extern __shared__ float4 smemr4[];
+    const int2 w = work[blockIdx.x];
+    const SlotBlock sb = sbt[w.x];
+    if ((w.y & kModTileMask) * kDenseOT >= sb.n_out) return;
+    const ChanParams &cp = prm[sb.slot];
+    float2 *smem = reinterpret_cast<float2 *>(smemr4);
+    switch (cp.plen) {  // uniform per CTA
+#define GPUD_ROT(LL)                                                                                          \
+    case LL:                                                                                                  \
+        if (cp.precise_sum) rot_tile<LL, true>(w, sb, cp, st, x, n, hist_arena, taps_arena, ext, smem);       \
+        else rot_tile<LL, false>(w, sb, cp, st, x, n, hist_arena, taps_arena, ext, smem);                     \
+        break;
+        GPUD_ROT(1) GPUD_ROT(2) GPUD_ROT(3) GPUD_ROT(4) GPUD_ROT(5) GPUD_ROT(6) GPUD_ROT(7) GPUD_ROT(8)
+        GPUD_ROT(9) GPUD_ROT(10) GPUD_ROT(11) GPUD_ROT(12) GPUD_ROT(13) GPUD_ROT(14) GPUD_ROT(15) GPUD_ROT(16)
+#undef GPUD_ROT
+    default: break;
+    }
 }
 
 // ===========================================================================
@@ -3188,6 +3362,16 @@ cudaError_t launch_extract_group(int grid, int smem, cudaStream_t sm, const int2
     cudaError_t e = smem_optin_once(optin, (const void *)k_extract_group, 220 * 1024);
     if (e != cudaSuccess) return e;
     return launch_dependent(k_extract_group, dim3((unsigned)grid), kDenseThreads, (size_t)smem, sm, work, sbt, prm,
+                            st, x, n, hist, taps, ext);
+}
+
+cudaError_t launch_extract_rot(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
+                               const ChanParams *prm, const ChanState *st, const float2 *x, int n,
+                               const float2 *hist, const float *taps, float2 *ext) {
+    static std::atomic<uint64_t> optin{0};
+    cudaError_t e = smem_optin_once(optin, (const void *)k_extract_rot, 220 * 1024);
+    if (e != cudaSuccess) return e;
+    return launch_dependent(k_extract_rot, dim3((unsigned)grid), kDenseThreads, (size_t)smem, sm, work, sbt, prm,
                             st, x, n, hist, taps, ext);
 }
 
