@@ -115,13 +115,14 @@ int group_smem_bytes_host(int Pc, int L);
 int mod_smem_bytes_host(int Pc, int L);
 int mod_launch_bytes_host(int P, int Pc, int L);
 int rot_launch_bytes_host(int P, int pg, int L);
+int rot_dense_bytes_host(int P, int L);
 int mod_item(int tile, int tiles);
 cudaError_t launch_extract_group(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
                                  const ChanParams *prm, const ChanState *st, const float2 *x, int n,
                                  const float2 *hist, const float *taps, float2 *ext);
-cudaError_t launch_extract_rot(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
-                               const ChanParams *prm, const ChanState *st, const float2 *x, int n,
-                               const float2 *hist, const float *taps, float2 *ext);
+cudaError_t launch_extract_rot(bool dense, int grid, int smem, cudaStream_t sm, const int2 *work,
+                               const SlotBlock *sbt, const ChanParams *prm, const ChanState *st, const float2 *x,
+                               int n, const float2 *hist, const float *taps, float2 *ext);
 cudaError_t launch_extract_mod(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
                                const ChanParams *prm, const ChanState *st, const float2 *x, int n,
                                const float2 *hist, const float *taps, float2 *ext);
@@ -994,6 +995,10 @@ static std::vector<int> plan_bank_groups(gpud_runner *r, BlockPlan &pl, const st
     return first;
 }
 
+// Tiles that a work item of the warp-private forms takes when the block has
+// many: with few phases there is little to do per tile.
+static int warp_tiles_per_item(int phases) { return std::min(8, std::max(1, 256 / phases)); }
+
 static void finish_plan(gpud_runner *r, BlockPlan &pl) {
     int64_t ext = 0;
     pl.tot_emit_ext = 0;
@@ -1158,7 +1163,7 @@ static void finish_plan(gpud_runner *r, BlockPlan &pl) {
         int64_t total = 0;
         for (int row : rows) total += tiles(row);
         for (int row : rows) {
-            const int k = total < 16 * (int64_t)r->num_sms ? 1 : std::min(8, std::max(1, 256 / slot(row).P));
+            const int k = total < 16 * (int64_t)r->num_sms ? 1 : warp_tiles_per_item(slot(row).P);
             for (int t = 0, nt = tiles(row); t < nt; t += k)
                 wl.push_back(make_int2(row, mod_item(t, std::min(k, nt - t))));
         }
@@ -1320,7 +1325,10 @@ static int enqueue_block(gpud_runner *r, Frame &f, const Frame *prev, BlockPlan 
     // run one tile per CTA.  Such classes whose shared memory is within 2x of
     // each other go out as one launch (their tiles laid out contiguously,
     // largest footprint first), so that a dozen small classes fill the GPU
-    // together instead of one after another.
+    // together instead of one after another; with two tiles per SM in them all
+    // (too much shared memory for the pipelined kernel, or a misaligned block),
+    // their warps work alone (224 channels among 2048: 1077 us with
+    // k_extract_dense_any, 840 with k_extract_rot; the sums keep their order).
     bool dense_pipe[kDenseMaxL + 1] = {};
     int dense_ng[kDenseMaxL + 1] = {};
     std::vector<int> tile_classes;
@@ -1335,8 +1343,13 @@ static int enqueue_block(gpud_runner *r, Frame &f, const Frame *prev, BlockPlan 
                      [&](int a, int b) { return pl.dense_smem[a] > pl.dense_smem[b]; });
     struct DenseBatch {
         size_t off = 0, items = 0;
-        int smem = 0, classes = 0, L = 0;
+        int smem = 0, classes = 0, L = 0, warp_smem = 0;
     };
+    size_t warp_tiles = 0;
+    for (int L : tile_classes) warp_tiles += pl.w_dense[L].size();
+    const bool warp_form = warp_tiles >= 2 * (size_t)r->num_sms;
+    auto dense_phases = [&](int row) { return r->slots[(size_t)pl.sbs[(size_t)row].slot].P; };
+
     std::vector<DenseBatch> batches;
     size_t w_dense_off[kDenseMaxL + 1] = {};
     for (int L : tile_classes) {
@@ -1347,11 +1360,18 @@ static int enqueue_block(gpud_runner *r, Frame &f, const Frame *prev, BlockPlan 
             batches.back().L = L;
         }
         DenseBatch &bt = batches.back();
+        const std::vector<int2> &wl = pl.w_dense[L];
         w_dense_off[L] = cnt;
-        std::memcpy(hw + cnt, pl.w_dense[L].data(), pl.w_dense[L].size() * sizeof(int2));
-        cnt += pl.w_dense[L].size();
-        bt.items += pl.w_dense[L].size();
+        for (size_t i = 0; i < wl.size();) {
+            const int k = warp_tiles < 16 * (size_t)r->num_sms ? 1 : warp_tiles_per_item(dense_phases(wl[i].x));
+            size_t e = i + 1;
+            while (e < wl.size() && (int)(e - i) < k && wl[e].x == wl[i].x) ++e;
+            hw[cnt++] = warp_form ? make_int2(wl[i].x, mod_item(wl[i].y, (int)(e - i))) : wl[i];
+            i = e;
+        }
+        bt.items = cnt - bt.off;
         bt.classes++;
+        bt.warp_smem = std::max(bt.warp_smem, rot_dense_bytes_host(pl.dense_pmax[L], L));
     }
     for (int L = 0; L <= kDenseMaxL; ++L) {
         if (pl.w_dense[L].empty() || !dense_pipe[L]) continue;
@@ -1425,7 +1445,10 @@ static int enqueue_block(gpud_runner *r, Frame &f, const Frame *prev, BlockPlan 
     for (const DenseBatch &bt : batches) {
         // one tile per CTA; the smaller CTAs share SMs with the other blocks in flight
         if (!side) prof_mark(r, f, bt.classes > 1 ? "extract_dense" : dense_name(bt.L).c_str());
-        if (bt.classes > 1)
+        if (warp_form)
+            CK(launch_extract_rot(true, (int)bt.items, bt.warp_smem, ds, d_w + bt.off, d_sb, r->d_prm, r->d_st, x_dev,
+                                  n, r->d_hist, r->d_taps, d_ext));
+        else if (bt.classes > 1)
             CK(launch_extract_dense_any((int)bt.items, bt.smem, ds, d_w + bt.off, d_sb, r->d_prm, r->d_st, x_dev, n,
                                         r->d_hist, r->d_taps, d_ext));
         else
@@ -1497,7 +1520,7 @@ static int enqueue_block(gpud_runner *r, Frame &f, const Frame *prev, BlockPlan 
     }
     if (!pl.w_group.empty() || !pl.w_rot.empty()) prof_mark(r, f, "extract_group");
     if (!pl.w_rot.empty()) {
-        CK(launch_extract_rot((int)pl.w_rot.size(), pl.rot_smem, f.s, d_w + o_rot, d_sb, r->d_prm, r->d_st, x_dev,
+        CK(launch_extract_rot(false, (int)pl.w_rot.size(), pl.rot_smem, f.s, d_w + o_rot, d_sb, r->d_prm, r->d_st, x_dev,
                               n, r->d_hist, r->d_taps, d_ext));
         nl++;
     }

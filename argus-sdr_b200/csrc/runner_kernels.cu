@@ -1253,7 +1253,16 @@ int rot_launch_bytes_host(int P, int pg, int L) {
     return (kModWarps * (rot_buf(L) + kRotCols) + pg) * 8 + std::max(pg * L, std::min(P * L, kRotTaps)) * 4;
 }
 
-template <int L, bool PREC>
+int rot_dense_bytes_host(int P, int L) {
+    return (kModWarps * rot_buf(L) + kDenseThreads + dense_rounds(P, L)) * 8 + P * L * 4;
+}
+
+// DENSE: one group of all D phases with the dense form's rotation, sample i' of
+// the tile by T1[i' % 256] T2[i' / 256].
+// For many tiles whose classes need too much shared memory for the pipelined
+// kernel: k_extract_dense_any then fits one CTA on an SM (224 channels among 2048:
+// 1077 us there, 903 here with one tile per item, 840 with several).
+template <int L, bool PREC, bool DENSE>
 __device__ __forceinline__ void rot_tile(const int2 w, const SlotBlock &sb, const ChanParams &cp,
                                          const ChanState *__restrict__ st, const float2 *__restrict__ x, int n,
                                          const float2 *__restrict__ hist_arena, const float *__restrict__ taps_arena,
@@ -1261,7 +1270,7 @@ __device__ __forceinline__ void rot_tile(const int2 w, const SlotBlock &sb, cons
     constexpr int R = kModR, KC = rot_kc(L), pitch = KC + 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int chain = lane & 7, og = lane >> 3;
-    const int D = cp.decim, P = cp.nphase, pg = sb.pg, ng = sb.ng;
+    const int D = cp.decim, P = cp.nphase, pg = DENSE ? P : sb.pg, ng = DENSE ? 1 : sb.ng;
     const uint64_t u0 = st[sb.slot].nco_q;
     const uint64_t inc = cp.inc_q;
     const float *tg = taps_arena + cp.taps_off;
@@ -1269,24 +1278,33 @@ __device__ __forceinline__ void rot_tile(const int2 w, const SlotBlock &sb, cons
     const int H = sb.hist_len;
     const int s0 = D - sb.pc - 1;
     float2 *z = smem + warp * rot_buf(L);
-    float2 *A = smem + kModWarps * rot_buf(L) + warp * kRotCols;
-    float2 *B = smem + kModWarps * (rot_buf(L) + kRotCols);
-    float *hs = reinterpret_cast<float *>(B + pg);
+    // column and row phasors; DENSE: T1 and T2
+    const int nk = DENSE ? dense_rounds(P, L) : pg;
+    float2 *A = smem + kModWarps * rot_buf(L) + (DENSE ? 0 : warp * kRotCols);
+    float2 *B = smem + kModWarps * (rot_buf(L) + (DENSE ? 0 : kRotCols)) + (DENSE ? kDenseThreads : 0);
+    float *hs = reinterpret_cast<float *>(B + nk);
     const int gb = max(1, kRotTaps / (pg * L));  // groups whose taps are held at a time
     auto edge = [&](int i) { return i < 0 && H + i >= 0 ? hist[H + i] : make_float2(0.f, 0.f); };  // shifted already
 
-    for (int r = threadIdx.x; r < pg; r += kDenseThreads) B[r] = q64_phasor((uint64_t)r * inc);
+    for (int r = threadIdx.x; r < nk; r += kDenseThreads)
+        B[r] = q64_phasor((uint64_t)r * (uint64_t)(DENSE ? kDenseThreads : 1) * inc);
     const int tile0 = w.y & kModTileMask, tiles = w.y >> kModTileBits;
     for (int tile = tile0; tile < tile0 + tiles; ++tile) {
         const WarpPart t = warp_part(tile, warp, L, D, P, s0, sb.n_out, n);
         const bool live = t.nv > 0;
         double2 acc64 = make_double2(0.0, 0.0);
         float2 acc32 = make_float2(0.f, 0.f);
+        if constexpr (DENSE) {
+            const int ibase = s0 + (tile * kDenseOT - (L - 1)) * D - (D - 1);
+            if (tile != tile0) __syncthreads();  // every warp is done with the last tile's T1
+            A[threadIdx.x] = q64_phasor(u0 + (uint64_t)(int64_t)(ibase + (int)threadIdx.x) * inc);
+            if (tile != tile0) __syncthreads();  // (the first tile's: with the taps)
+        }
         for (int g = 0, gt = 0; g < ng; ++g) {
             const int p_lo = g * pg, Pc = min(pg, P - p_lo);
             if (g == gt) {
                 gt += gb;
-                if (tile == tile0 || gb < ng) {
+                if (tile == tile0 || (!DENSE && gb < ng)) {
                     if (g || tile != tile0) __syncthreads();  // every warp is done with the last groups' taps
                     for (int i = threadIdx.x, e = (min(P, gt * pg) - p_lo) * L; i < e; i += kDenseThreads)
                         hs[i] = tg[p_lo * L + i];
@@ -1295,8 +1313,9 @@ __device__ __forceinline__ void rot_tile(const int2 w, const SlotBlock &sb, cons
             }
             if (live) {
                 const float *h2 = hs + (p_lo - (gt - gb) * pg) * L;
-                for (int m = lane; m < t.cols; m += 32)
-                    A[m] = q64_phasor(u0 + (uint64_t)(int64_t)(t.a0 - (p_lo + Pc - 1) + m * D) * inc);
+                if constexpr (!DENSE)
+                    for (int m = lane; m < t.cols; m += 32)
+                        A[m] = q64_phasor(u0 + (uint64_t)(int64_t)(t.a0 - (p_lo + Pc - 1) + m * D) * inc);
                 float2 acc[R];
                 double2 d[PREC ? R : 1];
 #pragma unroll
@@ -1314,19 +1333,28 @@ __device__ __forceinline__ void rot_tile(const int2 w, const SlotBlock &sb, cons
                         constexpr int S = 32 / KC, U = 4;
                         const int q = lane % KC, c = lane / KC;
                         if (q >= KC - np) {
-                            const float2 b = B[Pc - 1 - (c0 + KC - 1 - q)];
+                            const int r = Pc - 1 - (c0 + KC - 1 - q);  // of the column's samples, oldest first
+                            const float2 b = B[DENSE ? 0 : r];
+                            auto rotate = [&](float2 v, int m) {
+                                if constexpr (DENSE) {
+                                    const int i = (32 * warp + m) * D + r;
+                                    return cmulf(v, cmulf(A[i & (kDenseThreads - 1)], B[i / kDenseThreads]));
+                                } else {
+                                    return cmulf(v, cmulf(A[m], b));
+                                }
+                            };
                             float2 *zq = z + q + par;
                             int m = c;
                             for (; m < t.m0; m += S) {  // carried samples stay
                                 float2 &v = zq[m * pitch + (m >> 3) * 8];
-                                if (t.a0 - (p_lo + c0 + KC - 1) + q + m * D >= 0) v = cmulf(v, cmulf(A[m], b));
+                                if (t.a0 - (p_lo + c0 + KC - 1) + q + m * D >= 0) v = rotate(v, m);
                             }
                             for (; m < t.cols; m += S * U) {
                                 float2 v[U];
 #pragma unroll
                                 for (int u = 0; u < U; ++u) {
                                     const int mu = m + S * u;
-                                    if (mu < t.cols) v[u] = cmulf(zq[mu * pitch + (mu >> 3) * 8], cmulf(A[mu], b));
+                                    if (mu < t.cols) v[u] = rotate(zq[mu * pitch + (mu >> 3) * 8], mu);
                                 }
 #pragma unroll
                                 for (int u = 0; u < U; ++u) {
@@ -1371,12 +1399,10 @@ __device__ __forceinline__ void rot_tile(const int2 w, const SlotBlock &sb, cons
                 }
                 if constexpr (PREC) {
                     const double2 v = chain_sum(reinterpret_cast<double2 *>(z), d, chain, og, lane);
-                    acc64.x += v.x;
-                    acc64.y += v.y;
+                    acc64 = DENSE ? v : make_double2(acc64.x + v.x, acc64.y + v.y);
                 } else {
                     const float2 v = chain_sum(z, acc, chain, og, lane);
-                    acc32.x += v.x;
-                    acc32.y += v.y;
+                    acc32 = DENSE ? v : make_float2(acc32.x + v.x, acc32.y + v.y);
                 }
             }
         }
@@ -1384,6 +1410,7 @@ __device__ __forceinline__ void rot_tile(const int2 w, const SlotBlock &sb, cons
     }
 }
 
+template <bool DENSE>
 __global__ void __launch_bounds__(kDenseThreads, 2)
 k_extract_rot(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
               const ChanState *__restrict__ st, const float2 *__restrict__ x, int n,
@@ -1399,8 +1426,8 @@ k_extract_rot(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, 
     switch (cp.plen) {  // uniform per CTA
 #define GPUD_ROT(LL)                                                                                          \
     case LL:                                                                                                  \
-        if (cp.precise_sum) rot_tile<LL, true>(w, sb, cp, st, x, n, hist_arena, taps_arena, ext, smem);       \
-        else rot_tile<LL, false>(w, sb, cp, st, x, n, hist_arena, taps_arena, ext, smem);                     \
+        if (cp.precise_sum) rot_tile<LL, true, DENSE>(w, sb, cp, st, x, n, hist_arena, taps_arena, ext, smem);       \
+        else rot_tile<LL, false, DENSE>(w, sb, cp, st, x, n, hist_arena, taps_arena, ext, smem);                     \
         break;
         GPUD_ROT(1) GPUD_ROT(2) GPUD_ROT(3) GPUD_ROT(4) GPUD_ROT(5) GPUD_ROT(6) GPUD_ROT(7) GPUD_ROT(8)
         GPUD_ROT(9) GPUD_ROT(10) GPUD_ROT(11) GPUD_ROT(12) GPUD_ROT(13) GPUD_ROT(14) GPUD_ROT(15) GPUD_ROT(16)
@@ -3365,14 +3392,22 @@ cudaError_t launch_extract_group(int grid, int smem, cudaStream_t sm, const int2
                             st, x, n, hist, taps, ext);
 }
 
-cudaError_t launch_extract_rot(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
-                               const ChanParams *prm, const ChanState *st, const float2 *x, int n,
-                               const float2 *hist, const float *taps, float2 *ext) {
+template <bool DENSE>
+static cudaError_t launch_rot(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
+                              const ChanParams *prm, const ChanState *st, const float2 *x, int n,
+                              const float2 *hist, const float *taps, float2 *ext) {
     static std::atomic<uint64_t> optin{0};
-    cudaError_t e = smem_optin_once(optin, (const void *)k_extract_rot, 220 * 1024);
+    cudaError_t e = smem_optin_once(optin, (const void *)k_extract_rot<DENSE>, 220 * 1024);
     if (e != cudaSuccess) return e;
-    return launch_dependent(k_extract_rot, dim3((unsigned)grid), kDenseThreads, (size_t)smem, sm, work, sbt, prm,
-                            st, x, n, hist, taps, ext);
+    return launch_dependent(k_extract_rot<DENSE>, dim3((unsigned)grid), kDenseThreads, (size_t)smem, sm, work, sbt,
+                            prm, st, x, n, hist, taps, ext);
+}
+
+cudaError_t launch_extract_rot(bool dense, int grid, int smem, cudaStream_t sm, const int2 *work,
+                               const SlotBlock *sbt, const ChanParams *prm, const ChanState *st, const float2 *x,
+                               int n, const float2 *hist, const float *taps, float2 *ext) {
+    return dense ? launch_rot<true>(grid, smem, sm, work, sbt, prm, st, x, n, hist, taps, ext)
+                 : launch_rot<false>(grid, smem, sm, work, sbt, prm, st, x, n, hist, taps, ext);
 }
 
 cudaError_t launch_extract_mod(int grid, int smem, cudaStream_t sm, const int2 *work, const SlotBlock *sbt,
