@@ -1082,7 +1082,7 @@ static void finish_plan(gpud_runner *r, BlockPlan &pl) {
     pl.rds_smem = 0;
     std::vector<char> grouped = plan_gemm_groups(r, pl);
     const std::vector<int> banked = plan_bank_groups(r, pl, grouped);
-    std::vector<int> mod_rows, rot_rows;
+    std::vector<int> mod_rows, rot_rows, long_rows;
     for (int i = 0; i < (int)pl.sbs.size(); ++i) {
         const SlotBlock &sb = pl.sbs[(size_t)i];
         Slot &s = r->slots[(size_t)sb.slot];
@@ -1105,7 +1105,7 @@ static void finish_plan(gpud_runner *r, BlockPlan &pl) {
                     rot_rows.push_back(i);
                     pl.rot_smem = std::max(pl.rot_smem, rot_launch_bytes_host(s.P, s.pg, s.L));
                 } else if (s.ext_kind == 2) {
-                    for (int t = 0; t * dense_tile() < sb.n_out; ++t) pl.w_group.push_back(make_int2(i, t));
+                    long_rows.push_back(i);
                     pl.group_smem = std::max(pl.group_smem, group_smem_bytes_host(s.pg, s.L));
                 } else {
                     mod_rows.push_back(i);
@@ -1139,15 +1139,15 @@ static void finish_plan(gpud_runner *r, BlockPlan &pl) {
             pl.rds_smem = std::max(pl.rds_smem, rds_smem_bytes(std::max(1, demod_rate(s) / 19000)));
         }
     }
-    // a phase-grouped tile costs its channel's phases x arm length: the
-    // longest go first, so that the short ones fill in behind them
-    auto longest_first = [&](std::vector<int2> &wl) {
-        std::stable_sort(wl.begin(), wl.end(), [&](int2 a, int2 b) {
-            const Slot &sa = r->slots[(size_t)pl.sbs[(size_t)a.x].slot], &sb = r->slots[(size_t)pl.sbs[(size_t)b.x].slot];
-            return (int64_t)sa.P * sa.L > (int64_t)sb.P * sb.L;
-        });
-    };
-    longest_first(pl.w_group);
+    // A long arm's tile costs its channel's phases x arm length: the longest go
+    // first, so that the short ones fill in behind them.  Rows are sorted, not
+    // their tiles (17000 among 2048 channels: 0.6 ms of the host's time).
+    std::stable_sort(long_rows.begin(), long_rows.end(), [&](int a, int b) {
+        const Slot &sa = r->slots[(size_t)pl.sbs[(size_t)a].slot], &sb = r->slots[(size_t)pl.sbs[(size_t)b].slot];
+        return (int64_t)sa.P * sa.L > (int64_t)sb.P * sb.L;
+    });
+    for (int row : long_rows)
+        for (int t = 0; t * dense_tile() < pl.sbs[(size_t)row].n_out; ++t) pl.w_group.push_back(make_int2(row, t));
     // The forms in which every warp works by itself: rows by code path (the CTAs of
     // an SM share its instruction cache), the longest first.  A work item prepares
     // its channel's T taps once, so with few phases (little to do per tile) it takes

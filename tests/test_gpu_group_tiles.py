@@ -65,6 +65,10 @@ def _run(chans, fs, lens, shift, group_phases=0):
     (400, 50, 0, True),      # float64 row sums
     (350, 27, 0, True),
     (272, 16, 0, False),     # L 17: tiles of the whole CTA
+    (513, 27, 17, False),    # L 19, odd D, two groups
+    (640, 20, 20, False),    # L 32: no padding
+    (1000, 25, 25, True),    # L 40, float64 row sums, odd D
+    (4000, 10, 0, False),    # L 400
 ])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_group_tiles_match_oracle(cuda, taps, decim, group_phases, over, shift):
@@ -75,5 +79,5 @@ def test_group_tiles_match_oracle(cuda, taps, decim, group_phases, over, shift):
 def test_several_tiles_per_item_match_oracle(cuda):
     """Enough tiles that a work item takes several: few phases, two blocks."""
     fs = 1_600_000
-    chans = [(1_000.0 * k - 40_000.0, t, 16, k == 1) for k, t in enumerate((80, 150, 96, 256))]
-    _run(chans, fs, [16 * 160_003 + 5, 16 * 256 * 620], 0)
+    chans = [(1_000.0 * k - 40_000.0, t, 16, k == 1) for k, t in enumerate((80, 150, 96, 256, 300, 401))]
+    _run(chans, fs, [16 * 256 * 1_250 + 5, 16 * 256 * 1_220], 0)
