@@ -785,7 +785,8 @@ k_extract_wide(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt,
 // ===========================================================================
 // Phase-grouped polyphase form: channels whose D phases of a 256-output tile
 // do not fit in shared memory (large D), channels with one tap per phase
-// (T <= D), and long arms (L > 16).  A work item is (tile, phase group g):
+// (T <= D), and long arms (L > 16).  Arms of up to 16 taps run on
+// k_extract_rot (below), whose warps work alone; here, for longer arms,
 // the CTA stages the rotated samples of phases p_lo .. p_lo+Pc-1 only,
 //     Z[pp][m] = s(s0 + (m_base + m)*D - (p_lo + pp)),
 // -- for each column m a contiguous run of Pc samples -- and computes the
