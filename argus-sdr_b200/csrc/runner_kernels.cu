@@ -2266,6 +2266,10 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
     const SlotBlock sb = sbt[list[idx]];
     const int n = sb.n_disc;
     if (n <= 0) return;  // uniform per cluster
+    // Another CTA's shared memory may be touched once that CTA is known to run:
+    // every CTA of the cluster arrives here and waits before the first scan, so
+    // the staging and the coarse sums hide the barrier.
+    cl.barrier_arrive();
     const ChanParams &cp = prm[sb.slot];
     ChanState &s = st[sb.slot];
     const float *pil = wk + 3 * W + sb.comp_off;
@@ -2336,6 +2340,7 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
         if (tid == kNewtonThreads - 1)
             sh.next = SegState{start.dphi + (double)(t1 - c0) * start.df, start.df, start.I, start.Q};
         const int ncoarse = locked ? kPllCoarse : kPllCoarseFree;
+        if (c0 == 0) cl.barrier_wait();  // the arrive above
         for (int it = 0; it < ncoarse; ++it) {
             if (lane == 0) sh.first[warp] = x0;
             __syncthreads();
