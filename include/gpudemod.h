@@ -110,7 +110,9 @@ GPUD_API int GPUD_CALL gpud_launch_streaming_polyphase_prepare_cuda(
 /* exports.cu:533-631 -- production stateful streaming extractor for one
  * signal.  history_len_io, phase_count_state, phase_state and n_out are host
  * pointers read before and written after the launches; everything else is
- * device memory.  Codes -10..-16 as the reference.  Taps follow the CPU
+ * device memory.  After a call that returns 0 shifted_new_tmp holds the block
+ * times exp(j*(phase + i*phase_inc)) and history_scratch the new history, as
+ * after the reference's.  Codes -10..-16 as the reference.  Taps follow the CPU
  * oracle: the layout stride is polyphase_len/decim and taps with
  * p + k*decim >= num_taps are not applied (gpudemod/streaming_host_core.go). */
 GPUD_API int GPUD_CALL gpud_launch_streaming_polyphase_stateful_cuda(
