@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include "gpud_internal.cuh"
+#include "pll_step.cuh"
 
 #ifndef GPUD_DENSE_STAGE_U
 #define GPUD_DENSE_STAGE_U 4
@@ -1642,133 +1643,6 @@ k_wfm_fir(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, cons
     }
 }
 
-constexpr int kPllSeg = 16;  // steps per segment of the parallel solver; the float32 angle restarts as often
-
-struct PllK {
-    double alpha, beta;
-    float lpa;
-    double dfmin, dfmax;  // frequency clamp as deviations from the block-start frequency
-    uint64_t q0, qf;      // block-start phase and frequency in Q0.64 turns
-};
-
-// One loop step (recorder/streamer.go:1588-1613) in deviation form: the phase
-// is phase0 + t*freq0 + dphi, the frequency freq0 + df (dphi, df float64); the
-// ramp phase0 + t*freq0 is exact in Q0.64 turns, so the sin/cos argument needs
-// no float64 range reduction.  The I/Q lowpass states are float32.  The serial
-// loop and the Newton solver both use this step, so they iterate the same map.
-//
-// A trajectory is one chain of dependent operations, so a step costs its
-// latency.  The chain runs through float32 only: the angle above the ramp is
-// the float64 phase at the last pll_begin (the start of a 16-step segment),
-// rounded once, plus the advance since then in float32 -- below 1 rad, of an
-// angle that is rounded to float32 anyway -- while the float64 phase and
-// frequency are carried beside it.  (430 cycles a step through atan2f and the
-// float64 state.)
-struct PllRun {
-    double dphi, df;
-    float I, Q;
-    float base, off, adv;  // the next step's angle above the ramp: base + off + adv
-    float dff;             // df in float32
-};
-
-struct PllEval {
-    float e;
-    float ja, jb, jc, jd;   // phase row: d/dphase, d/dfreq, d/dI, d/dQ
-    float ka, kb, kc, kd;   // freq row
-    float iphi, qphi;       // I/Q rows' d/dphase (diagonals are 1 - lpa)
-};
-
-// The phase deviation of an unlocked loop grows to hundreds of radians: it is
-// reduced to one turn in float64 before it is rounded, else the rounding of the
-// angle (4e-6 rad at 50 rad) keeps the parallel solver above its tolerance.
-__device__ __forceinline__ PllRun pll_begin(double dphi, double df, float I, float Q) {
-    const double turns = rint(dphi * (1.0 / (2.0 * GPUD_PI)));
-    return PllRun{dphi, df, I, Q, (float)fma(turns, -2.0 * GPUD_PI, dphi), 0.f, 0.f, (float)df};
-}
-
-__device__ __forceinline__ float pll_rcp(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
-// atan2 in float32 (within 1.8 ulp; atan2f: 2.0): the quotient t of the smaller
-// by the larger magnitude from an approximate reciprocal and one residual
-// correction, then t + t u P(u), u = t^2, P fitted to atan on [0, 1] by
-// reweighted least squares (relative error 1.7e-8) and evaluated as short
-// chains; octant and signs enter as a factor of t and an offset, both ready
-// before the quotient is.  The scaling keeps the reciprocal's argument normal
-// as I and Q die out (and above zero).
-__device__ __forceinline__ float pll_atan2(float y, float x) {
-    const float ax = fabsf(x), ay = fabsf(y);
-    const float hi = fmaf(fmaxf(ax, ay), 1.8446744e19f, 1e-30f), lo = fminf(ax, ay) * 1.8446744e19f;
-    const bool swap = ay > ax, neg = x < 0.f;
-    // angle of (ax, ay): r or pi/2 - r; of (x, ay): that or pi minus it
-    const float sg = copysignf(1.f, y), st = swap != neg ? -sg : sg;
-    const float oh = swap ? 1.57079637f : neg ? 3.14159274f : 0.f;
-    const float ol = swap ? -4.371139e-8f : neg ? -8.742278e-8f : 0.f;
-    const float sh = sg * oh, sl = sg * ol;
-    const float rc = pll_rcp(hi);
-    float t = lo * rc;
-    t = fmaf(fmaf(-hi, t, lo), rc, t);
-    const float u = t * t, u2 = u * u, u4 = u2 * u2;
-    const float p01 = fmaf(u, 0.19993773f, -0.33333153f), p23 = fmaf(u, 0.10666005f, -0.14211056f);
-    const float p45 = fmaf(u, 0.04321186f, -0.07552214f), p67 = fmaf(u, 0.00292069f, -0.01636793f);
-    const float pp = fmaf(u4, fmaf(u2, p67, p45), fmaf(u2, p23, p01));
-    const float ts = t * st;
-    return (fmaf(ts * u, pp, ts) + sl) + sh;
-}
-
-// q: the ramp phase phase0 + t*freq0 of step t in Q0.64 turns (callers carry
-// it by adding k.qf per step: the same integer as k.q0 + t*k.qf); radians.
-__device__ __forceinline__ float pll_ramp(uint64_t q) { return (float)(int32_t)(q >> 32) * 1.46291808e-9f; }
-
-template <bool kJac>
-__device__ __forceinline__ void pll_step(uint64_t q, PllRun &s, float p, const PllK &k, PllEval &o) {
-    float sn, cs;
-    __sincosf((pll_ramp(q) + s.base + s.off) + s.adv, &sn, &cs);  // |angle| <= pi + |dphi|
-    s.off += s.adv;
-    const float I1 = fmaf(k.lpa, fmaf(p, cs, -s.I), s.I);
-    const float Q1 = fmaf(k.lpa, fmaf(p, -sn, -s.Q), s.Q);
-    const float e = pll_atan2(Q1, I1);
-    o.e = e;
-    const float df1 = fminf(fmaxf(fmaf((float)k.beta, e, s.dff), (float)k.dfmin), (float)k.dfmax);
-    s.adv = fmaf((float)k.alpha, e, df1);
-    s.dff = df1;
-    const double ed = (double)e;
-    double d = fma(k.beta, ed, s.df);
-    const bool clamped = d < k.dfmin || d > k.dfmax;
-    d = d < k.dfmin ? k.dfmin : (d > k.dfmax ? k.dfmax : d);
-    s.dphi = fma(k.alpha, ed, s.dphi) + d;
-    s.df = d;
-    s.I = I1;
-    s.Q = Q1;
-    if (kJac) {
-        // the Jacobian sets the convergence rate only, not the fixed point:
-        // an approximate reciprocal is enough
-        const float r2 = fmaf(I1, I1, Q1 * Q1);
-        const float inv = r2 > 0.f ? __fdividef(1.f, r2) : 0.f;
-        const float gI = -Q1 * inv, gQ = I1 * inv;
-        const float dIphi = -k.lpa * p * sn;  // d/dphase of lpa*p*cos(phase)
-        const float dQphi = -k.lpa * p * cs;  // d/dphase of -lpa*p*sin(phase)
-        const float ePhi = fmaf(gI, dIphi, gQ * dQphi);
-        const float om = 1.f - k.lpa;
-        const float eI = gI * om, eQ = gQ * om;
-        const float g = clamped ? 0.f : (float)k.beta, h = clamped ? 0.f : 1.f;
-        const float ga = g + (float)k.alpha;
-        o.ka = g * ePhi;
-        o.kb = h;
-        o.kc = g * eI;
-        o.kd = g * eQ;
-        o.ja = 1.f + ga * ePhi;
-        o.jb = h;
-        o.jc = ga * eI;
-        o.jd = ga * eQ;
-        o.iphi = dIphi;
-        o.qphi = dQphi;
-    }
-}
-
 __device__ __forceinline__ PllK pll_consts(const ChanParams &cp, const ChanState &s) {
     PllK k;
     k.alpha = cp.pll_alpha;
@@ -1787,13 +1661,6 @@ __device__ __forceinline__ double pll_phase_at(const PllK &k, int t, double dphi
     double ph = (double)q * (2.0 * GPUD_PI / 18446744073709551616.0) + dphi;
     ph -= (2.0 * GPUD_PI) * floor(ph * (1.0 / (2.0 * GPUD_PI)));
     return ph;
-}
-
-// Twice the loop phase in half-turns, float32 (lr = bpf * 2 sin(pi h)); q is
-// the ramp phase of the same step in Q0.64 turns.
-__device__ __forceinline__ float pll_twice(uint64_t q, double dphi) {
-    const uint64_t q2 = 2 * q;
-    return (float)(int32_t)(q2 >> 32) * 4.656612873077393e-10f + (float)(dphi * (2.0 / GPUD_PI));
 }
 
 // End of one stereoDecodeStateful call: store the loop state, update errAvg
@@ -1889,11 +1756,11 @@ k_pll(const int *__restrict__ list, int count, const SlotBlock *__restrict__ sbt
                 uint64_t qr = k.q0 + (uint64_t)base * k.qf;
                 for (int q = 0; q < len; ++q) {
                     PllEval o;
-                    if (q % kPllSeg == 0) x = pll_begin(x.dphi, x.df, x.I, x.Q);
+                    if (q % kPllSeg == 0) x = pll_begin(x.dphi(), x.df, x.I, x.Q);
                     pll_step<false>(qr, x, sp[q], k, o);
                     qr += k.qf;
                     es += fabs((double)o.e);
-                    th[q] = pll_twice(qr, x.dphi);
+                    th[q] = pll_twice(qr, x);
                 }
             }
         } else {
@@ -1925,7 +1792,7 @@ k_pll(const int *__restrict__ list, int count, const SlotBlock *__restrict__ sbt
     }
     __syncthreads();
     if (threadIdx.x != 0) return;
-    pll_finish(s, cp, n, pll_phase_at(k, n, x.dphi), s.pll_freq + x.df, (double)x.I, (double)x.Q, es, s_red[0]);
+    pll_finish(s, cp, n, pll_phase_at(k, n, x.dphi()), s.pll_freq + x.df, (double)x.I, (double)x.Q, es, s_red[0]);
     s.pll_path = 2;
 }
 
@@ -2410,7 +2277,7 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
                         pll_put_matrix(sh.aff[tid], a);
                     }
                 }
-                pll_put_gap(sh.aff[tid], SegState{x.dphi, x.df, x.I, x.Q}, nx, has_next);
+                pll_put_gap(sh.aff[tid], SegState{x.dphi(), x.df, x.I, x.Q}, nx, has_next);
             } else {
                 pll_put_identity(sh.aff[tid]);
             }
@@ -2448,7 +2315,10 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
                 converged = true;
             // Or when the corrections no longer shrink and are below the rounding of
             // a step's angle: unlocked loops, where I and Q pass near zero, stay
-            // there (2e-8 to 2e-7 rad) and would take every iteration allowed.
+            // there (2e-8 to 2e-7 rad) and would take every iteration allowed.  What
+            // is left is no more than the step's own distance to float64 on noise
+            // (1.1e-7 to 1.4e-7 rad rms, 1e-6 at most; 2e-6 to 7e-6 rms where the
+            // turns of the phase deviation stayed in the angle).
             if (!converged && mx.x <= kTolAngle && mx.x > 0.25f * prev_m0 && mx.y <= 1e-10f && mx.z <= 1e-6f &&
                 mx.w <= 1e-6f)
                 converged = true;
@@ -2494,7 +2364,7 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
                     pll_step<false>(qr, x, p, k, o);
                     qr += k.qf;
                     es += fabs((double)o.e);
-                    sh.seg[t - t0][tid] = pll_twice(qr, x.dphi);  // this thread's own cell, already read
+                    sh.seg[t - t0][tid] = pll_twice(qr, x);  // this thread's own cell, already read
                     p = pn;
                 }
             }
@@ -2528,7 +2398,7 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
             // never waits on a load), and lane i keeps step i's L-R product for
             // one coalesced store per 32 steps.
             const int ol = owner & 31;
-            PllRun xs = pll_begin(__shfl_sync(0xffffffffu, x.dphi, ol), __shfl_sync(0xffffffffu, x.df, ol),
+            PllRun xs = pll_begin(__shfl_sync(0xffffffffu, x.dphi(), ol), __shfl_sync(0xffffffffu, x.df, ol),
                                   __shfl_sync(0xffffffffu, x.I, ol), __shfl_sync(0xffffffffu, x.Q, ol));
             const int ts = __shfl_sync(0xffffffffu, t0, ol), te = c0 + nc;
             double es_w = __shfl_sync(0xffffffffu, es, ol);
@@ -2545,11 +2415,11 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
                 for (int i = 0; i < cnt; ++i) {
                     const float pt = __shfl_sync(0xffffffffu, pcur, i);
                     PllEval o;
-                    if (i % kPllSeg == 0) xs = pll_begin(xs.dphi, xs.df, xs.I, xs.Q);
+                    if (i % kPllSeg == 0) xs = pll_begin(xs.dphi(), xs.df, xs.I, xs.Q);
                     pll_step<false>(qr, xs, pt, k, o);
                     qr += k.qf;
                     es_w += fabs((double)o.e);
-                    const float th = pll_twice(qr, xs.dphi);
+                    const float th = pll_twice(qr, xs);
                     if (lane == i) mine = th;
                 }
                 if (lane < cnt) lr[s0 + lane] = bcur * (2.0f * sinpif(mine));
@@ -2562,7 +2432,7 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
             }
         }
         if (g == owner)
-            for (int r = 0; r < csize; ++r) *cl.map_shared_rank(&sh.end, r) = SegState{x.dphi, x.df, x.I, x.Q};
+            for (int r = 0; r < csize; ++r) *cl.map_shared_rank(&sh.end, r) = SegState{x.dphi(), x.df, x.I, x.Q};
         all_converged = all_converged && converged;
         locked = converged && it <= kPllOnce;
         if (c0 + kPllChunkSteps < n) {
