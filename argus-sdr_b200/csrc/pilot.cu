@@ -28,7 +28,8 @@
 // was as fast but doubled the error, 6e-15 -> 1e-14); periods beyond the table
 // take a sincospi per term.  (One CTA per station and bin, each thread walking
 // its own run of y: 1045 us.)  k_pilot_decide adds the CTAs' shares in
-// order and takes the max / median decision.
+// order and takes the max / median decision.  The shares of one full pass are
+// kept at a time; a call with more stations decides as it goes.
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
@@ -330,7 +331,8 @@ cudaError_t launch_pilot_bins(const PilotPass &ps, cudaStream_t s, const PilotJo
 struct gpud_pilot {
     int max_jobs = 0, max_samples = 0, num_sms = 148;
     double *d_y = nullptr;
-    double2 *d_part = nullptr;  // partial sums: num_sms x 201 per job
+    double2 *d_part = nullptr;  // partial sums [share][column][bin] of the passes between two decisions
+    int64_t part_cap = 0;       // its entries: one full pass (passes of one call take turns in it)
     double2 *d_tab = nullptr;   // roots of unity of the last pass's period
     int tab_period = 0;
     PilotJob *d_jobs = nullptr;
@@ -347,6 +349,11 @@ extern "C" {
 // window's samples; an even number, so that the pairs are aligned.
 static int64_t pilot_row(int max_samples) { return ((int64_t)max_samples + 3) & ~(int64_t)1; }
 
+// Shares of a pass: CTAs that split its terms.
+static int pilot_shares(const gpud_pilot *p, int folded) {
+    return std::max(1, std::min(p->num_sms, folded / (2 * kChunk)));
+}
+
 GPUD_API int GPUD_CALL gpud_pilot_create(int max_jobs, int max_samples, gpud_pilot **out) {
     if (!out || max_jobs <= 0 || max_samples <= 1) return GPUD_E_ARG;
     auto *p = new gpud_pilot();
@@ -356,9 +363,10 @@ GPUD_API int GPUD_CALL gpud_pilot_create(int max_jobs, int max_samples, gpud_pil
     if (cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0)
         p->num_sms = sms;
+    // a pass has at most kMaxSt columns and no more terms than a window has samples
+    p->part_cap = (int64_t)std::min(max_jobs, kMaxSt) * kBins * pilot_shares(p, max_samples);
     bool ok = cudaMalloc((void **)&p->d_y, sizeof(double) * (size_t)max_jobs * (size_t)pilot_row(max_samples)) == cudaSuccess &&
-              cudaMalloc((void **)&p->d_part, sizeof(double2) * (size_t)max_jobs * kBins * (size_t)p->num_sms) ==
-                  cudaSuccess &&
+              cudaMalloc((void **)&p->d_part, sizeof(double2) * (size_t)p->part_cap) == cudaSuccess &&
               cudaMalloc((void **)&p->d_tab, sizeof(double2) * (size_t)kMaxTable) == cudaSuccess &&
               cudaMalloc((void **)&p->d_jobs, sizeof(PilotJob) * (size_t)max_jobs) == cudaSuccess &&
               cudaMalloc((void **)&p->d_res, sizeof(gpud_pilot_result) * (size_t)max_jobs) == cudaSuccess;
@@ -434,6 +442,8 @@ GPUD_API int GPUD_CALL gpud_pilot_run(gpud_pilot *p, const gpud_pilot_job *jobs,
         sorted[(size_t)k] = p->jobs[(size_t)order[(size_t)k]];
         at[(size_t)order[(size_t)k]] = k;
     }
+    // Partial sums stand side by side while they fit the workspace; a pass that
+    // finds no room starts a new round, after the decisions on the one before.
     p->passes.clear();
     int64_t part = 0;
     for (int k = 0; k < nj;) {
@@ -450,7 +460,9 @@ GPUD_API int GPUD_CALL gpud_pilot_run(gpud_pilot *p, const gpud_pilot_job *jobs,
             ++k;
         }
         ps.spt = (ps.count + kStGroups - 1) / kStGroups;
-        ps.nshare = std::max(1, std::min(p->num_sms, ps.folded / (2 * kChunk)));
+        ps.nshare = pilot_shares(p, ps.folded);
+        const int64_t need = (int64_t)ps.nshare * kBins * ps.count;
+        if (part + need > p->part_cap) part = 0;
         ps.part_off = part;
         for (int c = 0; c < ps.count; ++c) {
             PilotJob &jb = sorted[(size_t)(ps.first + c)];
@@ -459,7 +471,7 @@ GPUD_API int GPUD_CALL gpud_pilot_run(gpud_pilot *p, const gpud_pilot_job *jobs,
             jb.ncol = ps.count;
             jb.part_off = part;
         }
-        part += (int64_t)ps.nshare * kBins * ps.count;
+        part += need;
         p->passes.push_back(ps);
     }
     if (cudaMemcpyAsync(p->d_jobs, sorted.data(), sizeof(PilotJob) * (size_t)nj, cudaMemcpyHostToDevice, s) !=
@@ -469,19 +481,27 @@ GPUD_API int GPUD_CALL gpud_pilot_run(gpud_pilot *p, const gpud_pilot_job *jobs,
     for (auto &jb : sorted) maxf = std::max(maxf, jb.folded);
     dim3 gf((unsigned)std::min(1024, (maxf + kPilotThreads - 1) / kPilotThreads), (unsigned)nj);
     k_pilot_fold<<<gf, kPilotThreads, 0, s>>>(p->d_jobs, p->d_y);
-    for (const PilotPass &ps : p->passes) {
+    int decided = 0, launches = 1;  // jobs decided; kernels
+    for (size_t k = 0; k < p->passes.size(); ++k) {
+        const PilotPass &ps = p->passes[k];
         const bool table = ps.period <= kMaxTable;
         if (table && ps.period != p->tab_period) {  // the pass before has read the old one (stream order)
             k_pilot_table<<<std::min(1024, (ps.period + 255) / 256), 256, 0, s>>>(ps.period, p->d_tab);
-            gpud_count_launch(1);
+            launches++;
             p->tab_period = ps.period;
         }
         if (launch_pilot_bins(ps, s, p->d_jobs, p->d_y, table ? p->d_tab : nullptr, p->d_part) != cudaSuccess)
             return GPUD_E_CUDA;
+        launches++;
+        if (k + 1 < p->passes.size() && p->passes[k + 1].part_off != 0) continue;
+        const int end = ps.first + ps.count;
+        k_pilot_decide<<<end - decided, kDecideParts * kPilotThreads, 0, s>>>(p->d_jobs + decided, p->d_part, threshold,
+                                                                              p->d_res + decided);
+        launches++;
+        decided = end;
     }
-    k_pilot_decide<<<nj, kDecideParts * kPilotThreads, 0, s>>>(p->d_jobs, p->d_part, threshold, p->d_res);
     if (cudaGetLastError() != cudaSuccess) return GPUD_E_CUDA;
-    gpud_count_launch(2 + (int)p->passes.size());
+    gpud_count_launch(launches);
     std::vector<gpud_pilot_result> tmp((size_t)nj);
     if (cudaMemcpyAsync(tmp.data(), p->d_res, sizeof(gpud_pilot_result) * (size_t)nj, cudaMemcpyDeviceToHost, s) !=
             cudaSuccess ||
