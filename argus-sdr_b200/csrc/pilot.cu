@@ -23,7 +23,7 @@
 // gives every CTA a contiguous share of m for all bins and up to 40 stations:
 // a thread keeps 7 bins x (cos, sin) x SPT stations in registers and reads 7
 // twiddles and SPT samples from shared memory for 14 SPT multiply-adds.  The
-// CTA copies its operands 16 m's ahead with asynchronous copies, the twiddles
+// CTA copies its operands 16 (8 with many stations) m's ahead with asynchronous copies, the twiddles
 // from a table of the P-th roots of unity (rotating 16 from one sincospi instead
 // was as fast but doubled the error, 6e-15 -> 1e-14); periods beyond the table
 // take a sincospi per term.  (One CTA per station and bin, each thread walking
@@ -49,11 +49,22 @@ namespace {
 constexpr int kBins = 201;
 constexpr int kPilotThreads = 256;
 constexpr int64_t kMaxTable = 1 << 20;  // roots-of-unity table entries (16 MiB)
-constexpr int kChunk = 16;        // m's per staged chunk
 constexpr int kBinsPT = 7;        // bins per thread: 4 warps x 8 lanes x 7 >= 201
 constexpr int kStGroups = 8;      // station groups of a CTA: 2 warp rows x 4 lane groups
 constexpr int kMaxSpt = 5;        // stations per thread
 constexpr int kMaxSt = kStGroups * kMaxSpt;  // stations per pass
+// The longer a chain of sums, the more of the station's programme, far above a
+// bin, is rounded into it, so a thread's sums are taken into second ones every
+// kChain terms.  With one chain per CTA the error was 1.04 (312.5 kS/s x 156250
+// samples) and 1.7 times (320 kS/s x 30000) that of 256 chains per bin; now it is
+// 0.5 times in both.  Up to three stations per thread the second sums are in
+// registers, above in shared memory, with smaller chunks to make room; the order
+// of sums is the same, so a station's result does not depend on how many others
+// there are.
+constexpr int kChain = 32;
+__host__ __device__ constexpr bool second_in_registers(int spt) { return spt <= 3; }
+__host__ __device__ constexpr int chunk_of(int spt) { return second_in_registers(spt) ? 16 : 8; }  // m's staged at a time
+constexpr int kShareMin = 32;  // fewest terms of a CTA's share
 
 struct PilotJob {
     const float2 *iq;  // first sample of the analysed window
@@ -105,10 +116,18 @@ k_pilot_fold(const PilotJob *__restrict__ jobs, double *__restrict__ y) {
 }
 
 // Shared memory of a CTA, both halves of a double buffer: twiddles | samples.
+template <int CH>
 struct PilotStage {
-    double2 w[2][kChunk][32 * kBinsPT];
-    double2 y[2][kChunk][kMaxSt];  // (s, d); the first alone where not paired
+    double2 w[2][CH][32 * kBinsPT];
+    double2 y[2][CH][kMaxSt];  // (s, d); the first alone where not paired
 };
+
+template <int SPT>
+constexpr int pilot_smem() {
+    return (int)sizeof(PilotStage<chunk_of(SPT)>) +
+           (second_in_registers(SPT) ? 0 : kBinsPT * SPT * kPilotThreads * (int)sizeof(double2));
+}
+static_assert(pilot_smem<kMaxSpt>() <= 227 * 1024, "shared memory of a CTA");
 
 // tab[a] = exp(j 2 pi a / P), a < P
 __global__ void k_pilot_table(int P, double2 *__restrict__ tab) {
@@ -137,21 +156,44 @@ template <int SPT, bool PAIRED>
 __global__ void __launch_bounds__(kPilotThreads)
 k_pilot_bins(const PilotJob *__restrict__ jobs, int count, int P, int folded, int fstep, const double *__restrict__ y,
              const double2 *__restrict__ tab, double2 *__restrict__ part) {
-    constexpr int NS = kStGroups * SPT;
+    constexpr int NS = kStGroups * SPT, kChunk = chunk_of(SPT);
     constexpr int NL = (kChunk * NS + kPilotThreads - 1) / kPilotThreads;  // samples a thread fetches
     extern __shared__ __align__(16) unsigned char psm[];
-    PilotStage &sm = *reinterpret_cast<PilotStage *>(psm);
+    PilotStage<kChunk> &sm = *reinterpret_cast<PilotStage<kChunk> *>(psm);
     const int t = (int)threadIdx.x, lane = t & 31, warp = t >> 5;
     // a warp takes 8 bins x 4 station groups at a time: both operands are
     // broadcast to the lanes that share them
     const int bin0 = (warp & 3) * (8 * kBinsPT) + (lane & 7), grp = (warp >> 2) * 4 + (lane >> 3);
     const int m0 = (int)((int64_t)folded * blockIdx.x / gridDim.x);
     const int m1 = (int)((int64_t)folded * (blockIdx.x + 1) / gridDim.x);
+    // the chain under way, and the sums of the chains before it
+    constexpr bool kRegs = second_in_registers(SPT);
     double re[kBinsPT][SPT], im[kBinsPT][SPT];
+    double2 own[kRegs ? kBinsPT : 1][SPT];
+    double2 *far = reinterpret_cast<double2 *>(psm + sizeof(PilotStage<kChunk>)) + t;
+    auto second = [&](int b, int s) -> double2 & {
+        if constexpr (kRegs) return own[b][s];
+        else return far[(b * SPT + s) * kPilotThreads];
+    };
 #pragma unroll
     for (int b = 0; b < kBinsPT; ++b)
 #pragma unroll
-        for (int s = 0; s < SPT; ++s) re[b][s] = im[b][s] = 0.0;
+        for (int s = 0; s < SPT; ++s) {
+            re[b][s] = im[b][s] = 0.0;
+            second(b, s) = make_double2(0.0, 0.0);
+        }
+    auto chain_end = [&]() {
+#pragma unroll
+        for (int b = 0; b < kBinsPT; ++b)
+#pragma unroll
+            for (int s = 0; s < SPT; ++s) {
+                double2 v = second(b, s);
+                v.x += re[b][s];
+                v.y += im[b][s];
+                second(b, s) = v;
+                re[b][s] = im[b][s] = 0.0;
+            }
+    };
     // thread t's twiddles: bin t; f / gcd(fs, 10) = (1800 + bin) * fstep
     const int64_t fq = ((int64_t)(1800 + t) * fstep) % P;
     // its samples of a chunk: consecutive threads on consecutive samples of a station
@@ -195,6 +237,7 @@ k_pilot_bins(const PilotJob *__restrict__ jobs, int count, int P, int folded, in
     __syncthreads();
     int buf = 0;
     for (int mc = m0; mc < m1; mc += kChunk, buf ^= 1) {
+        if (mc != m0 && (mc - m0) % kChain == 0) chain_end();
         if (mc + kChunk < m1) stage(buf ^ 1, mc + kChunk);
         for (int i = 0; i < kChunk; ++i) {  // samples past the share are zero
             double2 v[SPT];
@@ -216,6 +259,7 @@ k_pilot_bins(const PilotJob *__restrict__ jobs, int count, int P, int folded, in
         copies_wait();
         __syncthreads();
     }
+    chain_end();
     double2 *out = part + (int64_t)blockIdx.x * kBins * count;
 #pragma unroll
     for (int b = 0; b < kBinsPT; ++b) {
@@ -223,7 +267,7 @@ k_pilot_bins(const PilotJob *__restrict__ jobs, int count, int P, int folded, in
 #pragma unroll
         for (int s = 0; s < SPT; ++s) {
             const int st = grp * SPT + s;
-            if (bin < kBins && st < count) out[st * kBins + bin] = make_double2(re[b][s], im[b][s]);
+            if (bin < kBins && st < count) out[st * kBins + bin] = second(b, s);
         }
     }
 }
@@ -307,9 +351,9 @@ template <int SPT, bool PAIRED>
 cudaError_t launch_pilot_bins_as(const PilotPass &ps, cudaStream_t s, const PilotJob *jobs, const double *y,
                                  const double2 *tab, double2 *part) {
     static std::atomic<uint64_t> optin{0};
-    cudaError_t e = gpud::smem_optin_once(optin, (const void *)k_pilot_bins<SPT, PAIRED>, (int)sizeof(PilotStage));
+    cudaError_t e = gpud::smem_optin_once(optin, (const void *)k_pilot_bins<SPT, PAIRED>, pilot_smem<SPT>());
     if (e != cudaSuccess) return e;
-    k_pilot_bins<SPT, PAIRED><<<ps.nshare, kPilotThreads, sizeof(PilotStage), s>>>(
+    k_pilot_bins<SPT, PAIRED><<<ps.nshare, kPilotThreads, pilot_smem<SPT>(), s>>>(
         jobs + ps.first, ps.count, ps.period, ps.folded, ps.fstep, y, tab, part + ps.part_off);
     return cudaGetLastError();
 }
@@ -351,7 +395,7 @@ static int64_t pilot_row(int max_samples) { return ((int64_t)max_samples + 3) & 
 
 // Shares of a pass: CTAs that split its terms.
 static int pilot_shares(const gpud_pilot *p, int folded) {
-    return std::max(1, std::min(p->num_sms, folded / (2 * kChunk)));
+    return std::max(1, std::min(p->num_sms, folded / kShareMin));
 }
 
 GPUD_API int GPUD_CALL gpud_pilot_create(int max_jobs, int max_samples, gpud_pilot **out) {
