@@ -1869,14 +1869,25 @@ static int run_plain(gpud_runner *r, const gpud_float2 *iq, int n, int on_device
     return finish_frame(r, 0, -1);
 }
 
+// A block that was not enqueued whole (a copy or a launch was refused) leaves
+// work behind on the frame's two streams and the input stream, joined by no
+// event: it is waited for, so that the caller may free the block and the next
+// one may use the frame.
+static void settle_frame(gpud_runner *r, Frame &f) {
+    for (cudaStream_t s : {r->in_s, f.s2, f.s})
+        if (s) cudaStreamSynchronize(s);
+}
+
 static int run_block(gpud_runner *r, const gpud_float2 *iq, int n, int on_device, bool wait, uint64_t *ticket) {
     if (n < 0 || n > r->max_block) return set_err(r, GPUD_E_BLOCK, "block larger than max_block");
     int rc;
     if (r->schedule == GPUD_SCHED_PLAIN) {
         rc = run_plain(r, iq, n, on_device);
+        if (rc) settle_frame(r, r->fr[0]);
     } else {
         rc = submit_batched(r, iq, n, on_device);
-        if (!rc && wait) rc = drain(r);  // oldest first: the results are this block's
+        if (rc) settle_frame(r, r->fr[r->nxt]);  // nxt moves on with a whole block only
+        else if (wait) rc = drain(r);            // oldest first: the results are this block's
     }
     if (ticket) *ticket = r->submitted;
     return rc;
