@@ -1826,10 +1826,10 @@ k_pll(const int *__restrict__ list, int count, const SlotBlock *__restrict__ sbt
 // Jacobians.
 //
 // Measured (kernel alone; before: Newton with F's Jacobians from the
-// free-running ramp and scans by shuffles): 40 channels x 32768 steps 78 -> 52
-// us (3-5 -> 2 iterations), one channel of 7680 steps 48 -> 28 us, 154 channels
-// of 8192 steps of which half on noise 360-495 -> 119 us (up to 64 iterations
-// and a serial rest -> 12).  What bounds it: the latency of 16 dependent steps
+// free-running ramp and scans by shuffles): 40 channels x 32768 steps 78 -> 53
+// us (3-5 -> 2 iterations), one channel of 7680 steps 48 -> 31 us, 154 channels
+// of 8192 steps of which half on noise 360-495 -> 122 us (up to 64 iterations
+// and a serial rest -> 11).  What bounds it: the latency of 16 dependent steps
 // (~250 cycles each) and of a scan (~4500 cycles) per iteration.
 //
 // A block not converged after max_iters iterations keeps its consistent
@@ -2870,7 +2870,7 @@ __host__ __device__ inline AudTile aud_tile(int L, int M, int K, int C) {
         int ot = kAudThreads * r / unit * unit;
         while (ot > 0 && aud_window(ot, L, M, K) > kAudWin) ot -= unit;
         if (ot < kAudLive * r) continue;
-        return {r, ot, (((L * K + 1) & ~1) + C * aud_window(ot, L, M, K)) * 8};
+        return {r, ot, ((L * K + 1) & ~1) * 8 + C * aud_window(ot, L, M, K) * 4};
     }
     return {0, kAudOT, 0};
 }
@@ -2925,9 +2925,10 @@ __device__ __forceinline__ void aud_outputs(const SlotBlock &sb, int oa, int ob,
 // arms a quarter as often, load a coefficient once for four products, keep four
 // chains in flight and fit 120 narrow channels in about one wave of CTAs.
 // Measured, one output per thread before and now: 120 mono channels 20.9 ->
-// 12.8 us, 512 channels of all modes 26.0 -> 20.5, 40 stereo ones (r = 1) 14.0
-// both.  (A window staged in float64 spares 33 conversions per output but strides
-// of M/L doubles conflict in the banks: 40 stereo channels 21.7 us.)
+// 12.8 us, 512 channels of all modes 26.0 -> 19.6, 40 stereo ones (r = 1) 14.0 ->
+// 13.6 (the two last with 8 bytes reserved for a float of the window: 20.5, 14.0).
+// (A window staged in float64 spares 33 conversions per output but strides of M/L
+// doubles conflict in the banks: 40 stereo channels 21.7 us.)
 __global__ void __launch_bounds__(kAudThreads)
 k_audio48_rs(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt, const ChanParams *__restrict__ prm,
              const RsBank *__restrict__ banks, const AudState *__restrict__ aud, const float *__restrict__ audio,
@@ -3408,7 +3409,7 @@ cudaError_t launch_audio48(int grid_rs, int rs_smem, int count, cudaStream_t sm,
                            const SlotBlock *sbt, const ChanParams *prm, const RsBank *banks, AudState *aud,
                            const float *audio, float *rs_buf, int16_t *pcm) {
     static std::atomic<uint64_t> optin{0};  // more than 48 KiB of dynamic shared memory needs the opt-in
-    cudaError_t e = smem_optin_once(optin, (const void *)k_audio48_rs, (kAudBank + 2 * kAudWin) * 8);
+    cudaError_t e = smem_optin_once(optin, (const void *)k_audio48_rs, kAudBank * 8 + 2 * kAudWin * 4);
     if (e != cudaSuccess) return e;
     if (grid_rs > 0)
         e = launch_dependent(k_audio48_rs, dim3((unsigned)grid_rs), kAudThreads, (size_t)rs_smem, sm, work, sbt, prm, banks,
