@@ -121,6 +121,10 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
     return d;
 }
 
+// Longest arm (taps per phase) of the phase groups and large dense classes whose
+// warps work alone (k_extract_rot); longer arms run on k_extract_group.
+constexpr int kRotMaxL = 16;
+
 // ---------------------------------------------------------------------------
 // Per-slot constants
 // ---------------------------------------------------------------------------

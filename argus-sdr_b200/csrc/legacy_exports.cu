@@ -387,6 +387,18 @@ __global__ void __launch_bounds__(kPolyThreads) lk_poly_tile(PolyArgs a, const f
     out[j] = make_float2(ar, ai);
 }
 
+// SMs of the current device (asked once per device).
+static int device_sms() {
+    static std::atomic<int> known[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    n = known[dev].load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+    known[dev].store(n, std::memory_order_relaxed);
+    return n;
+}
+
 // Outputs of the concatenation a: the tile kernel where its rows fit in shared
 // memory (decimations up to ~800) and most samples of the span meet a tap, the
 // gather kernel beyond.
@@ -395,7 +407,7 @@ static cudaError_t launch_poly(const PolyArgs &a, const float *taps, int D, int 
     const int Lu = (num_taps + D - 1) / D, P = num_taps < D ? num_taps : D;
     for (int OT : {256, 64, 32}) {
         if (D > 4 * P) break;  // few taps far apart: most of the span would be walked for nothing
-        if (OT == 256 && n_out < 2 * 148 * 256) continue;
+        if (OT == 256 && n_out < 2 * 256 * device_sms()) continue;  // too few tiles of 256 for two per SM
         const int Mp = (OT + Lu - 1) | 1;
         const long long smem = (long long)P * Mp * sizeof(float2) + (long long)P * Lu * sizeof(float);
         if (smem > (OT == 32 ? 220 : 100) * 1024) continue;

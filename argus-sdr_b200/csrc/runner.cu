@@ -155,10 +155,12 @@ constexpr int kWideTile = 32;                 // outputs per work item of the wa
 #ifndef GPUD_DENSE_PIPE
 #define GPUD_DENSE_PIPE 2  // most consumer groups of the pipelined dense kernel (0: one-tile-per-CTA kernel only)
 #endif
-constexpr int kGroupSmemTarget = 100 * 1024;  // two CTAs per SM
-constexpr int kModSmemTarget = 72 * 1024;     // three CTAs per SM
+// What a channel's phase groups are sized by.  The groups order its sums, so
+// these stay as they were set, when every form staged a group by its whole CTA:
+// two CTAs per SM (k_extract_group still does) and three.
+constexpr int kGroupSmemTarget = 100 * 1024;
+constexpr int kModSmemTarget = 72 * 1024;
 constexpr int kModMaxL = 4;
-constexpr int kRotMaxL = 16;  // longest arm of the phase groups whose warps work alone (k_extract_rot)
 constexpr int kPllMaxIters = 64;
 #ifndef GPUD_FRAMES
 #define GPUD_FRAMES 3
@@ -2132,11 +2134,14 @@ static void choose_extraction(gpud_runner *r, Slot &s) {
     s.ext_kind = mod ? 3 : 2;
     s.ng = (s.P + pmax - 1) / pmax;
     s.pg = (s.P + s.ng - 1) / s.ng;
-    // The staging puts a group's phases on lanes (one pass per 32) and its
-    // rows on the 8 warps: groups of at most a multiple of 32 phases can keep
-    // the lanes full (100 phases as 4 x 25 rather than 3 x 34, whose second
-    // lane pass holds 2 of 32) at the price of more groups; take that split
-    // when the instructions per thread it needs are fewer.
+    // The cost model is that of a group staged by its whole CTA, its phases on
+    // lanes (one pass per 32) and its rows on the 8 warps, as k_extract_group
+    // does: groups of at most a multiple of 32 phases can keep the lanes full
+    // (100 phases as 4 x 25 rather than 3 x 34, whose second lane pass holds 2 of
+    // 32) at the price of more groups; that split is taken when the instructions
+    // per thread it needs are fewer.  The forms whose warps work alone (arms of up
+    // to kRotMaxL taps) need no such split; they keep it because the groups order
+    // a channel's sums.
     if (pmax >= 64 || (pmax >= 32 && pmax % 32 != 0)) {
         const int q = pmax / 32 * 32;
         const int ng = (s.P + q - 1) / q, pg = (s.P + ng - 1) / ng;

@@ -799,7 +799,9 @@ k_extract_wide(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt,
 // The rotation of sample cb(m) + r is A[m] * B[r], A[m] = exp(j phi(cb(m))),
 // B[r] = exp(j r inc), both exact from the Q0.64 phase.
 // ===========================================================================
-__host__ __device__ inline int group_Le(int L) { return L > 16 ? (L + 7) & ~7 : L; }
+// Arm length as k_extract_group runs it (whole chunks of 8 taps).  Shorter arms
+// run elsewhere, but their groups are sized by the same rule.
+__host__ __device__ inline int group_Le(int L) { return L > kRotMaxL ? (L + 7) & ~7 : L; }
 
 __host__ __device__ inline int group_smem_bytes(int Pc, int L) {
     const int Le = group_Le(L);
@@ -1246,7 +1248,6 @@ __host__ __device__ constexpr int rot_kc(int L) { return L > 8 ? 16 : 32; }
 __host__ __device__ constexpr int rot_buf(int L) {  // float2 entries of a warp's chunk
     return (32 + L - 1) * (rot_kc(L) + 2) + ((32 + L - 2) >> 3) * 8;
 }
-constexpr int kRotMaxL = 16;
 constexpr int kRotCols = 32 + kRotMaxL;  // column phasors of a warp
 constexpr int kRotTaps = 1024;           // taps held at a time
 static_assert(rot_buf(9) >= 2 * 8 * kModRed && rot_buf(1) >= 2 * 8 * kModRed, "float64 sums of eight chains");
