@@ -326,14 +326,16 @@ __global__ void __launch_bounds__(256) lk_poly_accum(PolyArgs a, const float *__
 // adds its taps in the order of lk_poly_accum (bit-identical).  lk_poly_accum
 // waited on one global load a tap (257 taps, 10240 outputs: 40 us; now 10); the
 // 256 threads stage with four loads in flight each, and the chain of
-// multiply-adds of the OT output threads is the bound.  OT = 64 spreads the
+// multiply-adds of the OT output threads is the bound; shifted (may be null)
+// takes the rotated samples beside it.  OT = 64 spreads the
 // few outputs of a call over the SMs; calls that fill them anyway take 256 and
 // stage fewer samples twice.
 constexpr int kPolyThreads = 256;
 
 __global__ void __launch_bounds__(kPolyThreads) lk_poly_tile(PolyArgs a, const float *__restrict__ taps, int D, int L,
                                                              int Lu, int P, int num_taps, int start_idx, int n_out,
-                                                             int OT, int Mp, float2 *__restrict__ out) {
+                                                             int OT, int Mp, float2 *__restrict__ shifted,
+                                                             float2 *__restrict__ out) {
     extern __shared__ float2 Z[];  // P rows of pitch Mp, then the taps P x Lu
     float *st = reinterpret_cast<float *>(Z + P * Mp);
     const int t = threadIdx.x;
@@ -359,8 +361,13 @@ __global__ void __launch_bounds__(kPolyThreads) lk_poly_tile(PolyArgs a, const f
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int e = e0 + u * kPolyThreads, q = base + e - a.H, p = D - 1 - r;
-            if (e < M * D && p < P)
-                Z[p * Mp + c] = a.rotate && q >= 0 ? cmulf(v[u], q64_phasor(a.u0 + (uint64_t)q * a.inc)) : v[u];
+            // the columns of this tile's outputs are its own (the ones before them belong to the last tile)
+            const bool own = shifted && c >= Lu - 1 && j0 + c - (Lu - 1) < n_out && q >= 0;
+            if (e < M * D && (p < P || own)) {
+                const float2 s = a.rotate && q >= 0 ? cmulf(v[u], q64_phasor(a.u0 + (uint64_t)q * a.inc)) : v[u];
+                if (p < P) Z[p * Mp + c] = s;
+                if (own) shifted[q] = s;
+            }
             c += dc;
             r += dr;
             if (r >= D) {
@@ -401,9 +408,10 @@ static int device_sms() {
 
 // Outputs of the concatenation a: the tile kernel where its rows fit in shared
 // memory (decimations up to ~800) and most samples of the span meet a tap, the
-// gather kernel beyond.
+// gather kernel beyond.  With `shifted` the block's samples up to the newest
+// that an output takes, rotated, go there too on the tile path: *covered of them.
 static cudaError_t launch_poly(const PolyArgs &a, const float *taps, int D, int L, int num_taps, int start_idx,
-                               int n_out, float2 *out) {
+                               int n_out, float2 *out, float2 *shifted = nullptr, int *covered = nullptr) {
     const int Lu = (num_taps + D - 1) / D, P = num_taps < D ? num_taps : D;
     for (int OT : {256, 64, 32}) {
         if (D > 4 * P) break;  // few taps far apart: most of the span would be walked for nothing
@@ -415,25 +423,26 @@ static cudaError_t launch_poly(const PolyArgs &a, const float *taps, int D, int 
         cudaError_t e = smem_optin_once(optin, (const void *)lk_poly_tile, 220 * 1024);
         if (e != cudaSuccess) return e;
         lk_poly_tile<<<(n_out + OT - 1) / OT, kPolyThreads, (size_t)smem>>>(a, taps, D, L, Lu, P, num_taps, start_idx,
-                                                                          n_out, OT, Mp, out);
+                                                                          n_out, OT, Mp, shifted, out);
+        if (covered) *covered = start_idx + (n_out - 1) * D + 1;
         return cudaGetLastError();
     }
     lk_poly_accum<<<(n_out + 255) / 256, 256>>>(a, taps, D, L, num_taps, start_idx, n_out, out);
     return cudaGetLastError();
 }
 
-// The state after a block in one pass: sample q of the block, rotated, goes to
-// shifted[q], and the last `keep` samples of the concatenation to dst and, where
-// given, to dst2 (the history itself: allowed when keep <= n_new, so that no
+// The state after a block in one pass: sample q >= q0 of the block, rotated, goes
+// to shifted[q], and the last `keep` samples of the concatenation to dst and,
+// where given, to dst2 (the history itself: allowed when keep <= n_new, so that no
 // sample of the old history is read).  shifted may be null.
-__global__ void __launch_bounds__(256) lk_block_state(PolyArgs a, int keep, float2 *__restrict__ shifted,
+__global__ void __launch_bounds__(256) lk_block_state(PolyArgs a, int keep, float2 *__restrict__ shifted, int q0,
                                                       float2 *__restrict__ dst, float2 *__restrict__ dst2) {
     const int total = a.H + a.n_new;
-    const int first = shifted ? min(a.H, total - keep) : total - keep;
+    const int first = shifted ? min(a.H + q0, total - keep) : total - keep;
     const int i = first + (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= total) return;
     const float2 v = poly_sample(a, i);
-    if (shifted && i >= a.H) shifted[i - a.H] = v;
+    if (shifted && i >= a.H + q0) shifted[i - a.H] = v;
     const int h = i - (total - keep);
     if (h < 0) return;
     dst[h] = v;
@@ -467,7 +476,7 @@ extern "C" GPUD_API int GPUD_CALL gpud_launch_streaming_polyphase_prepare_cuda(
     if (history_out && keep > 0) {
         int nh = H + n_new < keep ? H + n_new : keep;
         if (nh > 0) {
-            lk_block_state<<<(nh + 255) / 256, 256>>>(a, nh, nullptr, (float2 *)history_out, nullptr);
+            lk_block_state<<<(nh + 255) / 256, 256>>>(a, nh, nullptr, 0, (float2 *)history_out, nullptr);
             gpud_count_launch(1);
             cudaError_t e = cudaGetLastError();
             if (e != cudaSuccess) return (int)e;
@@ -524,14 +533,13 @@ static int polyphase_stateful(const gpud_float2 *in_new, int n_new, gpud_float2 
     }
     const int total = pc + n_new;
     const int out_count = total / decim;
-    // The samples are rotated as they are read, and the state after the block is
-    // written in one pass: no copy of the block between the kernels, no staging of
-    // a history that lies whole in the new block.  That changes what is read after
-    // what is written, so it is for buffers that have nothing in common: where any
-    // two of them overlap, and where an error is returned, the steps are separate
-    // (the block is copied, shifted, before anything else is written).  Measured
-    // with 204800 samples, 257 taps, decimation 20: separate steps 19.4 us, this 16.4
-    // (without the caller's two temporaries 14.3).
+    // The samples are rotated as they are read, the shifted block is written by the
+    // kernel that has it in hand, and a history that lies whole in the new block
+    // without staging.  That changes what is read after what is written, so it is
+    // for buffers that have nothing in common: where any two of them overlap, and
+    // where an error is returned, the steps are separate (the block is copied,
+    // shifted, before anything else is written).  Measured with 204800 samples, 257
+    // taps, decimation 20: separate steps 19.4 us, this 14.4.
     const bool fused = out_count <= out_cap && (out_count == 0 || out) &&
                        (newH == 0 || (history_state && history_scratch)) &&
                        poly_apart({{in_new, n_new}, {shifted_new_tmp, n_new}, {out, out_count},
@@ -546,20 +554,23 @@ static int polyphase_stateful(const gpud_float2 *in_new, int n_new, gpud_float2 
     if (out_count > out_cap) return -14;
     const PolyArgs a{(const float2 *)history_state, H, (const float2 *)(fused ? in_new : shifted_new_tmp), n_new, fused,
                      u0, inc};
+    float2 *const shifted = fused && keep_temps && n_new > 0 ? (float2 *)shifted_new_tmp : nullptr;
+    int q0 = 0;  // samples of the shifted block that the outputs' kernel writes
     if (out_count > 0) {
         if (!out) return -15;
-        cudaError_t e = launch_poly(a, polyphase_taps, decim, L, num_taps, decim - pc - 1, out_count, (float2 *)out);
+        cudaError_t e = launch_poly(a, polyphase_taps, decim, L, num_taps, decim - pc - 1, out_count, (float2 *)out,
+                                    shifted, &q0);
         gpud_count_launch(1);
         if (e != cudaSuccess) return (int)e;
     }
     if (newH > 0 && (!history_state || !history_scratch)) return -16;
     const bool in_place = fused && n_new >= newH;  // no sample of the old history is kept
-    float2 *const shifted = fused && keep_temps && n_new > 0 ? (float2 *)shifted_new_tmp : nullptr;
     float2 *const state = (float2 *)history_state, *const scratch = (float2 *)history_scratch;
-    if (newH > 0 || shifted) {
-        const int count = shifted ? std::max(n_new, newH) : newH;
+    const int rest = shifted ? n_new - q0 : 0;  // samples of the shifted block that are not written yet
+    if (newH > 0 || rest > 0) {
+        const int count = std::max(rest, newH);
         const bool direct = in_place && !keep_temps;
-        lk_block_state<<<(count + 255) / 256, 256>>>(a, newH, shifted, direct ? state : scratch,
+        lk_block_state<<<(count + 255) / 256, 256>>>(a, newH, shifted, q0, direct ? state : scratch,
                                                      in_place && !direct ? state : nullptr);
         gpud_count_launch(1);
         cudaError_t e = cudaGetLastError();

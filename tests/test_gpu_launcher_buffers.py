@@ -86,3 +86,30 @@ def test_shifted_block_without_history(cuda, n):
     assert nout.value == n and hl.value == 0
     assert max_abs(d_sh.cpu().numpy()[:n], want) <= 1e-5
     assert max_abs(d_out.cpu().numpy()[:n], want) <= 1e-5
+
+
+@pytest.mark.parametrize("taps,decim,n", [
+    (101, 4, 4_001), (512, 2, 160_003), (65, 64, 64 * 33 + 5), (300, 400, 12_345), (512, 500, 499), (1, 7, 700),
+    (33, 200, 8_130), (512, 1000, 33_333),  # few taps far apart, rows too large: the gather kernel
+])
+def test_shifted_block_of_every_route(cuda, taps, decim, n):
+    """Every sample of the shifted block: those an output's tile has in hand, the
+    rest behind the newest output, and all of them where no tile runs."""
+    import torch
+    poly = O.build_polyphase_taps_phase_major(O.base_taps_f32(200_000, FS, max(taps, 2)), decim)
+    cap = max(1, taps - 1)
+    x = make_tone_noise_iq(n, 0.03)
+    d_in, d_taps = torch.from_numpy(x).cuda(), torch.from_numpy(poly).cuda()
+    d_sh, d_hist, d_scr = (torch.full((m,), float("nan"), dtype=torch.complex64, device="cuda") for m in (n, cap, cap))
+    d_out = torch.zeros(n // decim + 2, dtype=torch.complex64, device="cuda")
+    hl, pc, ph, nout = C.c_int(0), C.c_int(decim // 3), C.c_double(0.2), C.c_int()
+    torch.cuda.synchronize()
+    assert lib.gpud_launch_streaming_polyphase_stateful_cuda(
+        d_in.data_ptr(), n, d_sh.data_ptr(), d_taps.data_ptr(), poly.size, decim, taps, d_hist.data_ptr(),
+        d_scr.data_ptr(), cap, C.byref(hl), C.byref(pc), C.byref(ph), INC, d_out.data_ptr(), d_out.numel(),
+        C.byref(nout)) == 0
+    assert lib.gpud_stream_sync(None) == 0
+    want = x * np.exp(1j * (0.2 + INC * np.arange(n)))
+    assert max_abs(d_sh.cpu().numpy(), want.astype(np.complex64)) <= 1e-5
+    assert max_abs(d_hist[:hl.value].cpu().numpy(), want[n - hl.value:].astype(np.complex64)) <= 1e-5
+    assert max_abs(d_scr[:hl.value].cpu().numpy(), want[n - hl.value:].astype(np.complex64)) <= 1e-5
