@@ -19,7 +19,8 @@
 //
 // The bins of all stations of one rate are a matrix product, (201 x 2) x P/2
 // twiddles times P/2 x stations samples, and float64 multiply-adds are its bound
-// (40 stations at 312.5 kS/s: 0.25 G, 14 us at the chip's rate).  k_pilot_bins
+// (40 stations at 312.5 kS/s: 0.25 G, 14 us at the chip's rate; 61 us measured,
+// the staging and barriers of 8-term chunks and the prologue the rest).  k_pilot_bins
 // gives every CTA a contiguous share of m for all bins and up to 40 stations:
 // a thread keeps 7 bins x (cos, sin) x SPT stations in registers and reads 7
 // twiddles and SPT samples from shared memory for 14 SPT multiply-adds.  The

@@ -968,8 +968,10 @@ k_extract_group(const int2 *__restrict__ work, const SlotBlock *__restrict__ sbt
 // even), else 8.  Eight columns are followed by a pad of 64 bytes, so the window
 // loads of two output groups fall on the two halves of the banks.  Nothing waits
 // for another warp but the taps, which are built once per work item.
-// Bound by instruction issue (multiply-adds 42 % of the instructions, staging
-// addresses and window loads the rest; 16 warps per SM).  1344 such channels of
+// Bound by the instructions of four warps a scheduler (two CTAs per SM by shared
+// memory): issue slots 51 % busy, multiply-adds 38 % of the instructions, staging
+// addresses and window loads the rest, waits for fixed latencies the largest
+// stall (profiles/extraction_headroom_512.md).  1344 such channels of
 // 64..768 taps among 2048: 1954 us with a tile's samples staged by the whole CTA
 // through registers, 1288 now.  Chunks of 16 with the next one in flight: 1643
 // (per-chunk work weighs more than the latency that 16 warps hide); rows of a

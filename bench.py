@@ -425,13 +425,14 @@ def stage_key(name):
 # the kernel on the same workload (cold cache, serialised); None where no
 # capture exists.
 NCU_TRAFFIC = {("fm_band", "extract_gemm"): 8.73e6,
-               ("fm_band", "pll"): 10.58e6,
+               ("fm_band", "pll"): 10.93e6,
                }
 # Headroom stress, captured at 512 channels (the 2048-channel launch was not
-# captured): the phase-group kernels read the L2-resident block once and write
+# captured): the extraction kernels read the L2-resident block once and write
 # nothing to DRAM during the launch, so their traffic does not grow with the
-# channel count and is reported as measured, not scaled.
-NCU_TRAFFIC_HEADROOM_512 = {"extract_mod": 10.23e6, "extract_group": 9.70e6}
+# channel count and is reported as measured, not scaled.  The phase-group stage
+# is two launches (arms of up to 16 taps, longer ones): their sum.
+NCU_TRAFFIC_HEADROOM_512 = {"extract_mod": 10.35e6, "extract_group": 9.46e6 + 8.92e6, "extract_dense": 9.28e6}
 
 
 def kernel_roofline(name, ms, work, fp32, hbm_peak, peak_kind, wl, tf32=None):
