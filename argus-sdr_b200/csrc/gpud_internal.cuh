@@ -50,6 +50,13 @@ inline cudaError_t smem_optin_once(std::atomic<uint64_t> &done, const void *fn, 
 // 585.  Letting the next kernel's CTAs start while this one still runs was
 // slower: 126, 326, 218, 605 -- they hold shared memory while they wait.)
 // ---------------------------------------------------------------------------
+// A refused launch is reported by its return value: taken out of the thread's last
+// error too, where the next launch that is checked there would find it.
+inline cudaError_t launch_status(cudaError_t e) {
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e;
+}
+
 __device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class... P, class... A>
@@ -64,7 +71,18 @@ inline cudaError_t launch_dependent(void (*fn)(P...), dim3 grid, int threads, si
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
+    return launch_status(cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...));
+}
+
+// A launch on its own whose error, if any, is its own.
+template <class... P, class... A>
+inline cudaError_t launch_alone(void (*fn)(P...), dim3 grid, int threads, size_t smem, cudaStream_t sm, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = sm;
+    return launch_status(cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...));
 }
 
 // ---------------------------------------------------------------------------

@@ -436,6 +436,7 @@ struct gpud_runner {
 
 static int set_err(gpud_runner *r, int code, const char *what, cudaError_t e = cudaSuccess) {
     char buf[256];
+    if (e != cudaSuccess) (void)cudaGetLastError();  // reported here: not the next call's
     if (e != cudaSuccess)
         std::snprintf(buf, sizeof buf, "%s: %s", what, cudaGetErrorString(e));
     else

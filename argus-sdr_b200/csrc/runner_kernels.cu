@@ -3374,7 +3374,7 @@ cudaError_t launch_pll_newton(int count, int cluster, cudaStream_t sm, const int
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, k_pll_newton, list, count, sbt, prm, st, wk, W, max_iters);
+    return launch_status(cudaLaunchKernelEx(&cfg, k_pll_newton, list, count, sbt, prm, st, wk, W, max_iters));
 }
 
 int pll_newton_threads() { return kNewtonThreads; }
@@ -3462,8 +3462,7 @@ __global__ void __launch_bounds__(256) k_rs_bank(int L, int M, int K, double *__
 }
 
 cudaError_t launch_rs_bank(cudaStream_t sm, int L, int M, int K, double *arm) {
-    k_rs_bank<<<(L * K + 255) / 256, 256, 0, sm>>>(L, M, K, arm);
-    return cudaGetLastError();
+    return launch_alone(k_rs_bank, dim3((unsigned)((L * K + 255) / 256)), 256, 0, sm, L, M, K, arm);
 }
 
 cudaError_t launch_post_extract(int grid, cudaStream_t sm, const SlotBlock *sbt, const ChanParams *prm, ChanState *st,

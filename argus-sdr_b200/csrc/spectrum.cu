@@ -156,9 +156,9 @@ GPUD_API int GPUD_CALL gpud_spectrum_create(int max_fft, int max_segments, gpud_
         gpud_spectrum_destroy(s);
         return GPUD_E_CUDA;
     }
-    k_spectrum_twiddles<<<kMaxFft / 2 / 256, 256>>>(s->d_tab);
+    const cudaError_t e = gpud::launch_alone(k_spectrum_twiddles, dim3(kMaxFft / 2 / 256), 256, 0, nullptr, s->d_tab);
     gpud_count_launch(1);
-    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess) {
+    if (e != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess) {
         gpud_spectrum_destroy(s);
         return GPUD_E_CUDA;
     }
