@@ -58,7 +58,7 @@ __global__ void k_loop(const float *pilot, int n, Loop c, int rounded, double *p
 
 __global__ void k_atan2(const float *y, const float *x, int n, int plain, float *out) {
     const int i = blockIdx.x * blockDim.x + (int)threadIdx.x;
-    if (i < n) out[i] = plain ? atan2f(y[i], x[i]) : pll_atan2(y[i], x[i]);
+    if (i < n) out[i] = plain ? atan2f(y[i], x[i]) : pll_atan2(y[i], x[i], pll_scale(fmaxf(fabsf(y[i]), fabsf(x[i]))));
 }
 
 }  // namespace

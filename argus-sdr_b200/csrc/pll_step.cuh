@@ -70,11 +70,14 @@ __device__ __forceinline__ float pll_rcp(float x) {
 // correction, then t + t u P(u), u = t^2, P fitted to atan on [0, 1] by
 // reweighted least squares (relative error 1.7e-8) and evaluated as short
 // chains; octant and signs enter as a factor of t and an offset, both ready
-// before the quotient is.  The scaling keeps the reciprocal's argument normal
-// as I and Q die out (and above zero).
-__device__ __forceinline__ float pll_atan2(float y, float x) {
+// before the quotient is.  `scale` keeps the reciprocal's argument normal: 2^64
+// as I and Q die out (and the offset above zero), 2^-64 above 2^60, so that all of
+// float32's range is covered, as by atan2f.  It may come from any bound on the two.
+__device__ __forceinline__ float pll_scale(float bound) { return bound > 1.1529215e18f ? 5.4210109e-20f : 1.8446744e19f; }
+
+__device__ __forceinline__ float pll_atan2(float y, float x, float scale) {
     const float ax = fabsf(x), ay = fabsf(y);
-    const float hi = fmaf(fmaxf(ax, ay), 1.8446744e19f, 1e-30f), lo = fminf(ax, ay) * 1.8446744e19f;
+    const float hi = fmaf(fmaxf(ax, ay), scale, 1e-30f), lo = fminf(ax, ay) * scale;
     const bool swap = ay > ax, neg = x < 0.f;
     // angle of (ax, ay): r or pi/2 - r; of (x, ay): that or pi minus it
     const float sg = copysignf(1.f, y), st = swap != neg ? -sg : sg;
@@ -110,7 +113,7 @@ __device__ __forceinline__ void pll_step(uint64_t q, PllRun &s, float p, const P
     __sincosf(fmaf(h, 3.14159265358979f, s.adv), &sn, &cs);  // |angle| <= 2 pi and a step
     const float I1 = fmaf(k.lpa, fmaf(p, cs, -s.I), s.I);
     const float Q1 = fmaf(k.lpa, fmaf(p, -sn, -s.Q), s.Q);
-    const float e = pll_atan2(Q1, I1);
+    const float e = pll_atan2(Q1, I1, pll_scale(fmaxf(fmaxf(fabsf(s.I), fabsf(s.Q)), fabsf(p))));  // known before I1, Q1
     o.e = e;
     const float df1 = fminf(fmaxf(fmaf((float)k.beta, e, (float)s.df), (float)k.dfmin), (float)k.dfmax);
     s.adv = fmaf((float)k.alpha, e, df1);

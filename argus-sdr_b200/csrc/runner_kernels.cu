@@ -1837,7 +1837,7 @@ k_pll(const int *__restrict__ list, int count, const SlotBlock *__restrict__ sbt
 //
 // A block not converged after max_iters iterations keeps its consistent
 // prefix (a segment whose start is exact is exact after one more iteration)
-// and one warp runs the serial loop over the rest.  Blocks longer than one
+// and one warp runs the serial loop from its last segment on.  Blocks longer than one
 // segment per thread of the largest cluster (32768 steps) are solved chunk by
 // chunk, each from the end state of the one before.
 #ifndef GPUD_PLL_CLUSTER
@@ -2109,7 +2109,11 @@ __device__ __forceinline__ void pll_put_gap(AffCols &m, const SegState &x, const
 // pi beta, so a start t steps on cannot be further off.  (An iterate that
 // overshoots on noise would run into the frequency clamp, where the map forgets
 // its start, and only the consistent prefix would grow, a segment an iteration.)
+// A correction that overflowed or is not a number moves nothing: in a start it
+// would stay for good (the residuals of a NaN start are NaN), while a finite guess
+// gets its exact value once the segments before it have theirs.
 __device__ __forceinline__ void pll_move(SegState &x, const float4 &d, double f0, double reach) {
+    if (!(fabsf(d.x) + fabsf(d.y) + fabsf(d.z) + fabsf(d.w) < 1e38f)) return;
     x.dphi += (double)d.x;
     x.df = fmin(fmax(x.df + (double)d.y, f0 - reach), f0 + reach);
     x.I += d.z;
@@ -2209,7 +2213,11 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
         const double pi_beta = GPUD_PI * k.beta, reach = (double)(t0 - c0) * pi_beta;
         if (tid == kNewtonThreads - 1)
             sh.next = SegState{start.dphi + (double)(t1 - c0) * start.df, start.df, start.I, start.Q};
-        const int ncoarse = locked ? kPllCoarse : kPllCoarseFree;
+        // A loop that a non-finite sample has gone through stays not a number, here
+        // as in the serial loop: there is nothing to solve.
+        const bool dead = !(isfinite(start.dphi) && isfinite(start.df) && isfinite(start.I) && isfinite(start.Q) &&
+                            isfinite(s.pll_phase) && isfinite(s.pll_freq));
+        const int ncoarse = dead ? 0 : locked ? kPllCoarse : kPllCoarseFree;
         if (c0 == 0) cl.barrier_wait();  // the arrive above
         for (int it = 0; it < ncoarse; ++it) {
             if (lane == 0) sh.first[warp] = x0;
@@ -2239,7 +2247,7 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
         if (tid == 0 && crank > 0) *cl.map_shared_rank(&sh.next, crank - 1) = x0;
         cl.sync();
         // ---- Newton on the loop -------------------------------------------
-        bool converged = false, bad = true;
+        bool converged = dead, bad = true;
         bool quasi = true;      // the coarse map's Jacobian (uniform in the cluster)
         int sweeps = 0;         // of F with its own Jacobian
         float prev_m0 = 1e30f;  // last iteration's largest phase correction (uniform in the cluster)
@@ -2331,9 +2339,9 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
         iters = max(iters, it);
         // ---- not converged: the longest consistent prefix is kept ----------
         // Segments before the first one whose start still moved by more than the
-        // tolerance form a consistent trajectory from the chunk start, and that
-        // segment's updated start is its exact start; one warp continues the
-        // serial loop from there to the chunk end.
+        // tolerance form a consistent trajectory from the chunk start; one warp
+        // continues the serial loop from the start of the last of them to the chunk
+        // end.
         int gstar = INT_MAX;
         if (!converged) {
             int v = bad ? g : INT_MAX;
@@ -2348,7 +2356,7 @@ k_pll_newton(const int *__restrict__ list, int count, const SlotBlock *__restric
             }
             cl.sync();
             for (int r = 0; r < csize; ++r) gstar = min(gstar, *cl.map_shared_rank(&sh.cbad, r));
-            if (gstar == INT_MAX) gstar = 0;  // no start moved past the tolerance in the last iteration
+            gstar = gstar == INT_MAX ? 0 : max(gstar - 1, 0);  // INT_MAX: none moved past the tolerance in the last iteration
         }
         // ---- outputs: each converged segment again from its start ----------
         PllRun x = pll_begin(x0.dphi, x0.df, x0.I, x0.Q);
