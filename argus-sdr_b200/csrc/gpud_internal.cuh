@@ -379,6 +379,7 @@ std::vector<double> lowpass_fir(double cutoff_hz, int sample_rate, int taps);
 int build_binade_table(double inc, BinadeTable *t);
 
 constexpr int kWfmTaps = 101;      // stereo / RDS filter length (streamer.go:1531-1545, fm.go:155)
+constexpr int kWfmTapsBytes = 2480;  // one rate's filters in the table that the host writes and the kernels read
 constexpr int kWfmHist = 100;
 constexpr int kD1Taps = 101;       // pre-demod decimating FIR (streamer.go:1124)
 

@@ -128,10 +128,13 @@ cudaError_t launch_extract_mod(int grid, int smem, cudaStream_t sm, const int2 *
                                const float2 *hist, const float *taps, float2 *ext);
 
 constexpr int kWfmTapsPadH = 104;
-struct WfmTapsHost {
+// A rate's filters as the kernels read them (WfmTaps): float4 alignment, so the
+// same stride from one rate to the next.
+struct alignas(16) WfmTapsHost {
     float t[kWfmTapsPadH][4];
     double rds[kWfmTaps];
 };
+static_assert(sizeof(WfmTapsHost) == kWfmTapsBytes, "the rates' stride of the kernels");
 constexpr int kAudioDlStrideH = kWfmHist + 4;
 constexpr int kMaxWfmClasses = 16;
 constexpr int kDenseMaxL = 16;

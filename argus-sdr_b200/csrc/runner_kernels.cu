@@ -1556,6 +1556,7 @@ struct WfmTaps {
     float4 t[kWfmTapsPad];
     double rds[kWfmTaps];
 };
+static_assert(sizeof(WfmTaps) == kWfmTapsBytes, "the rates' stride of the host");
 
 // Composite-rate work arrays (all float, same offsets comp_off):
 //   work + 0*W comp (discriminator output), 1*W lpr, 2*W bpf, 3*W pilot, 4*W lr
