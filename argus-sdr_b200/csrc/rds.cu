@@ -19,8 +19,10 @@
 // samples from shared memory and leaves its symbols there, the loop thread
 // takes the last round's symbols, and the other warps fetch the next window.
 // What is left is the longer of the two chains (the Costas loop's float64 sine
-// and cosine, ~490 cycles a symbol): 40 stations x 4750 symbols 4325 -> 1217 us
-// against one thread that did both from global memory.  The expensive part of
+// and cosine, ~490 cycles a symbol): 40 stations x 4750 symbols 4325 -> 1202 us
+// against one thread that did both from global memory; one station x 94 symbols,
+// too few to decode, 30 -> 23 (55 with the first window read from global memory
+// and the Costas loop run for nothing).  The expensive part of
 // the search -- decoding a 104-bit group at every start offset, each block with
 // up to 26 trial flips -- runs over all offsets in parallel into a table (the
 // syndrome is linear: a flip adds its own), and the flywheel walk, by one warp,
@@ -209,6 +211,7 @@ __device__ void rds_table(const uint8_t *bits, int nbits, bool inv, uint8_t *ok,
 
 constexpr int kWin = 2048;  // samples per window
 constexpr int kSyms = 256;  // most symbols per round
+constexpr int kMinSyms = 104;  // one group: fewer symbols are not decoded
 
 __global__ void __launch_bounds__(kRdsThreads)
 k_rds_decode(const RdsJobDev *__restrict__ jobs, RdsState *__restrict__ states, uint8_t *__restrict__ bits_s,
@@ -231,7 +234,8 @@ k_rds_decode(const RdsJobDev *__restrict__ jobs, RdsState *__restrict__ states, 
         s_go = 0;
         s_nb = 0;
         s_cnt[0] = s_cnt[1] = 0;
-        s_at[0] = s_at[1] = -1;
+        s_at[0] = run ? 0 : -1;  // the first window is fetched here
+        s_at[1] = -1;
         s_idx = 0;
         s_done = run ? 0 : 1;
         if (run) {
@@ -244,6 +248,8 @@ k_rds_decode(const RdsJobDev *__restrict__ jobs, RdsState *__restrict__ states, 
             d.last_sample_rate = fs;
         }
     }
+    if (run)
+        for (int i = tid; i <= kWin && i < n; i += kRdsThreads) s_win[0][i] = jb.s[i];
     __syncthreads();
     // Mueller-Muller timing (rds.go:109-160), thread 0
     const double sps = (double)fs / 1187.5;
@@ -309,7 +315,8 @@ k_rds_decode(const RdsJobDev *__restrict__ jobs, RdsState *__restrict__ states, 
         } else if (tid == 0) {
             s_cnt[half] = 0;
         } else if (tid == 32) {
-            const int cnt = s_cnt[half ^ 1];
+            // too few symbols in all leave the loop as it was: nothing to run it for
+            const int got = s_cnt[half ^ 1], cnt = ended && nsym + got < kMinSyms ? 0 : got;
             for (int i = 0; i < cnt; ++i) {
                 double sd, cd;
                 sincos(phase, &sd, &cd);  // the values of sin and cos (equal on 6e8 arguments)
@@ -364,7 +371,7 @@ k_rds_decode(const RdsJobDev *__restrict__ jobs, RdsState *__restrict__ states, 
         d.sync_prev_dec = prev_dec;
         d.sync_has_prev = have_prev;
     }
-    if (tid == 32 && run && nsym >= 104) {  // fewer symbols leave the loop as it was
+    if (tid == 32 && run && nsym >= kMinSyms) {
         d.costas_phase = phase;
         d.costas_freq = freq;
         d.last_hard_bit = last;
