@@ -76,6 +76,8 @@ struct PilotJob {
     int32_t nshare;    // CTAs of its pass
     int32_t column;    // its column in the pass
     int32_t ncol;      // columns of the pass
+    int32_t fstep;     // 10 / gcd(fs, 10)
+    int32_t span;      // terms of its pass: the longest folded of its stations
     int64_t part_off;  // its pass's partial sums
     int64_t y_off;     // offset of this job's folded vector
 };
@@ -85,6 +87,7 @@ struct PilotPass {
     int first, count, period, folded, paired, fstep, spt;
     int64_t part_off;  // double2 offset of its partial sums [share][column][bin]
     int nshare;
+    bool each;         // few terms: k_pilot_bins_each
 };
 
 // fmDemod (pll.go:170-183): float64 products of the float32 samples, atan2.
@@ -271,6 +274,44 @@ k_pilot_bins(const PilotJob *__restrict__ jobs, int count, int P, int folded, in
             if (bin < kBins && st < count) out[st * kBins + bin] = second(b, s);
         }
     }
+}
+
+// The sums of short windows: one CTA per (share, station), a thread per bin, any
+// rates together, twiddles computed where they are used.  The shares, the chains and
+// so the bits are those of k_pilot_bins, which takes 14 us whatever it is given (its
+// 100 KB and more of shared memory, a launch and a table a rate).  Up to kEachTerms
+// station-terms a rate this takes 9 to 20 us; the products of many stations
+// belong there (40 stations of 100000 samples: 95 us; 0.8 ms one by one).
+constexpr int kEachTerms = 8192;
+
+__global__ void __launch_bounds__(kPilotThreads)
+k_pilot_bins_each(const PilotJob *__restrict__ jobs, const double *__restrict__ y, double2 *__restrict__ part) {
+    const PilotJob jb = jobs[blockIdx.y];
+    const int share = blockIdx.x, bin = (int)threadIdx.x, P = jb.period;
+    if (share >= jb.nshare || bin >= kBins) return;
+    const int64_t fq = ((int64_t)(1800 + bin) * jb.fstep) % P;
+    const int m0 = (int)((int64_t)jb.span * share / jb.nshare);
+    const int m1 = min(jb.folded, (int)((int64_t)jb.span * (share + 1) / jb.nshare));
+    const double *ym = y + jb.y_off;
+    double2 all = make_double2(0.0, 0.0);
+    const unsigned up = (unsigned)P, uf = (unsigned)fq;  // both below 2^31
+    unsigned a = (unsigned)((fq * (int64_t)m0) % P);
+    for (int mc = m0; mc < m1; mc += kChain) {
+        const int me = min(m1, mc + kChain);
+        double2 v = make_double2(0.0, 0.0);
+#pragma unroll 4
+        for (int m = mc; m < me; ++m) {
+            double s, c;
+            sincospi(2.0 * (double)a / (double)P, &s, &c);
+            v.x = fma(ym[jb.paired ? 2 * m : m], c, v.x);
+            v.y = fma(ym[jb.paired ? 2 * m + 1 : m], s, v.y);
+            a += uf;
+            if (a >= up) a -= up;
+        }
+        all.x += v.x;
+        all.y += v.y;
+    }
+    part[jb.part_off + ((int64_t)share * jb.ncol + jb.column) * kBins + bin] = all;
 }
 
 // max (first occurrence, as the reference's strict '>' scan from 0) and the
@@ -465,6 +506,7 @@ GPUD_API int GPUD_CALL gpud_pilot_run(gpud_pilot *p, const gpud_pilot_job *jobs,
         jb.period = q.sample_rate / g;
         jb.paired = jb.nd >= jb.period ? 1 : 0;
         jb.folded = jb.paired ? jb.period / 2 + 1 : jb.nd;
+        jb.fstep = 10 / g;
         jb.y_off = (int64_t)p->jobs.size() * pilot_row(p->max_samples);
         p->job_of[(size_t)j] = (int)p->jobs.size();
         p->jobs.push_back(jb);
@@ -505,6 +547,7 @@ GPUD_API int GPUD_CALL gpud_pilot_run(gpud_pilot *p, const gpud_pilot_job *jobs,
             ++k;
         }
         ps.spt = (ps.count + kStGroups - 1) / kStGroups;
+        ps.each = (int64_t)ps.count * ps.folded <= kEachTerms;
         ps.nshare = pilot_shares(p, ps.folded);
         const int64_t need = (int64_t)ps.nshare * kBins * ps.count;
         if (part + need > p->part_cap) part = 0;
@@ -512,6 +555,7 @@ GPUD_API int GPUD_CALL gpud_pilot_run(gpud_pilot *p, const gpud_pilot_job *jobs,
         for (int c = 0; c < ps.count; ++c) {
             PilotJob &jb = sorted[(size_t)(ps.first + c)];
             jb.nshare = ps.nshare;
+            jb.span = ps.folded;
             jb.column = c;
             jb.ncol = ps.count;
             jb.part_off = part;
@@ -528,14 +572,23 @@ GPUD_API int GPUD_CALL gpud_pilot_run(gpud_pilot *p, const gpud_pilot_job *jobs,
     k_pilot_fold<<<gf, kPilotThreads, 0, s>>>(p->d_jobs, p->d_y);
     int decided = 0, launches = 1;  // jobs decided; kernels
     for (size_t k = 0; k < p->passes.size(); ++k) {
-        const PilotPass &ps = p->passes[k];
-        const bool table = ps.period <= kMaxTable;
+        PilotPass ps = p->passes[k];
+        if (ps.each) {  // with the short windows of the next rates
+            for (; k + 1 < p->passes.size() && p->passes[k + 1].each && p->passes[k + 1].part_off != 0; ++k) {
+                ps.count += p->passes[k + 1].count;
+                ps.nshare = std::max(ps.nshare, p->passes[k + 1].nshare);
+            }
+            k_pilot_bins_each<<<dim3((unsigned)ps.nshare, (unsigned)ps.count), kPilotThreads, 0, s>>>(
+                p->d_jobs + ps.first, p->d_y, p->d_part);
+        }
+        const bool table = !ps.each && ps.period <= kMaxTable;
         if (table && ps.period != p->tab_period) {  // the pass before has read the old one (stream order)
             k_pilot_table<<<std::min(1024, (ps.period + 255) / 256), 256, 0, s>>>(ps.period, p->d_tab);
             launches++;
             p->tab_period = ps.period;
         }
-        if (launch_pilot_bins(ps, s, p->d_jobs, p->d_y, table ? p->d_tab : nullptr, p->d_part) != cudaSuccess)
+        if (!ps.each &&
+            launch_pilot_bins(ps, s, p->d_jobs, p->d_y, table ? p->d_tab : nullptr, p->d_part) != cudaSuccess)
             return GPUD_E_CUDA;
         launches++;
         if (k + 1 < p->passes.size() && p->passes[k + 1].part_off != 0) continue;
