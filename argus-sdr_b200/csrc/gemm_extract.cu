@@ -234,9 +234,11 @@ k_extract_gemm(const int2 *__restrict__ work, const GemmGroup *__restrict__ grou
     const int rows = kGemmM + L - 1;
     const int i0 = -g.pc + (j0 - L + 1) * D;
     const int total = rows * D;
-    const int a0 = i0 & ~1;
+    // bulk copies start and end on 16 bytes: at an even sample of a block that
+    // does, at an odd one of a block on an odd multiple of 8 bytes
+    const int a0 = i0 - (int)(((unsigned)i0 + (unsigned)(reinterpret_cast<uintptr_t>(x) >> 3)) & 1u);
     const int cnt = (i0 - a0 + total + 1) & ~1;
-    const bool raw = (long long)a0 + cnt <= (long long)n && cnt * 8 <= lo.b_stage;
+    const bool raw = a0 >= 0 && (long long)a0 + cnt <= (long long)n && cnt * 8 <= lo.b_stage;
     const int nb0 = raw ? NS - 1 : NS;  // stages loaded before the staging
     char *rawp = reinterpret_cast<char *>(gsm + lo.o_b + (NS - 1) * lo.b_stage);
     if (tid == 0) {
