@@ -276,16 +276,20 @@ k_pilot_bins(const PilotJob *__restrict__ jobs, int count, int P, int folded, in
     }
 }
 
-// The sums of short windows: one CTA per (share, station), a thread per bin, any
-// rates together, twiddles computed where they are used.  The shares, the chains and
-// so the bits are those of k_pilot_bins, which takes 14 us whatever it is given (its
-// 100 KB and more of shared memory, a launch and a table a rate).  Up to kEachTerms
-// station-terms a rate this takes 9 to 20 us; the products of many stations
-// belong there (40 stations of 100000 samples: 95 us; 0.8 ms one by one).
-constexpr int kEachTerms = 8192;
+// The sums of a few stations: one CTA per (share, station), a thread per bin, any
+// rates together; twiddles from the table for the rate that it holds, else computed.
+// The shares, the chains and so the bits are those of k_pilot_bins, which takes 14 us
+// and about 2.4 for every 16 terms of a share whatever it is given (its 100 KB and
+// more of shared memory, one chunk ahead), and a launch and a table a rate; here a
+// thousand station-terms cost 0.6 us, more than there from the third station on.
+// Calls at 312.5 kS/s, this and that: one station of 23000 samples 68 and 89 us, two
+// 82 and 91, three 97 and 95, five of 4000 75 and 65, eight of 1000 64 and 69.
+constexpr int kEachStations = 2;
+constexpr int kEachTerms = 12288;  // station-terms that more of them may have
 
 __global__ void __launch_bounds__(kPilotThreads)
-k_pilot_bins_each(const PilotJob *__restrict__ jobs, const double *__restrict__ y, double2 *__restrict__ part) {
+k_pilot_bins_each(const PilotJob *__restrict__ jobs, const double *__restrict__ y, const double2 *__restrict__ tab,
+                  int tab_period, double2 *__restrict__ part) {
     const PilotJob jb = jobs[blockIdx.y];
     const int share = blockIdx.x, bin = (int)threadIdx.x, P = jb.period;
     if (share >= jb.nshare || bin >= kBins) return;
@@ -299,14 +303,33 @@ k_pilot_bins_each(const PilotJob *__restrict__ jobs, const double *__restrict__ 
     for (int mc = m0; mc < m1; mc += kChain) {
         const int me = min(m1, mc + kChain);
         double2 v = make_double2(0.0, 0.0);
-#pragma unroll 4
-        for (int m = mc; m < me; ++m) {
-            double s, c;
-            sincospi(2.0 * (double)a / (double)P, &s, &c);
-            v.x = fma(ym[jb.paired ? 2 * m : m], c, v.x);
-            v.y = fma(ym[jb.paired ? 2 * m + 1 : m], s, v.y);
+        auto term = [&](int m, const double2 w) {
+            v.x = fma(ym[jb.paired ? 2 * m : m], w.x, v.x);
+            v.y = fma(ym[jb.paired ? 2 * m + 1 : m], w.y, v.y);
+        };
+        auto next = [&]() {
+            const unsigned at = a;
             a += uf;
             if (a >= up) a -= up;
+            return at;
+        };
+        int m = mc;
+        if (P == tab_period) {
+            for (; m + 8 <= me; m += 8) {  // eight gathers in flight
+                double2 w[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) w[u] = __ldg(tab + next());
+#pragma unroll
+                for (int u = 0; u < 8; ++u) term(m + u, w[u]);
+            }
+            for (; m < me; ++m) term(m, __ldg(tab + next()));
+        } else {
+#pragma unroll 4
+            for (; m < me; ++m) {
+                double s, c;
+                sincospi(2.0 * (double)next() / (double)P, &s, &c);
+                term(m, make_double2(c, s));
+            }
         }
         all.x += v.x;
         all.y += v.y;
@@ -342,11 +365,19 @@ k_pilot_decide(const PilotJob *__restrict__ jobs, const double2 *__restrict__ pa
     if (i < kBins) {
         const double2 *p = part + jb.part_off + (int64_t)jb.column * kBins + i;
         double re = 0.0, im = 0.0, er = 0.0, ei = 0.0;
-#pragma unroll 8
-        for (int k = q; k < jb.nshare; k += kDecideParts) {
-            const double2 v = p[(int64_t)k * kBins * jb.ncol];
-            add_exact(re, er, v.x);
-            add_exact(im, ei, v.y);
+        for (int k0 = q; k0 < jb.nshare; k0 += 8 * kDecideParts) {  // eight loads in flight
+            double2 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int k = k0 + u * kDecideParts;
+                v[u] = k < jb.nshare ? p[(int64_t)k * kBins * jb.ncol] : make_double2(0.0, 0.0);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                if (k0 + u * kDecideParts >= jb.nshare) break;
+                add_exact(re, er, v[u].x);
+                add_exact(im, ei, v[u].y);
+            }
         }
         s_p[q][i] = make_double2(re + er, im + ei);
     }
@@ -547,7 +578,7 @@ GPUD_API int GPUD_CALL gpud_pilot_run(gpud_pilot *p, const gpud_pilot_job *jobs,
             ++k;
         }
         ps.spt = (ps.count + kStGroups - 1) / kStGroups;
-        ps.each = (int64_t)ps.count * ps.folded <= kEachTerms;
+        ps.each = ps.count <= kEachStations || (int64_t)ps.count * ps.folded <= kEachTerms;
         ps.nshare = pilot_shares(p, ps.folded);
         const int64_t need = (int64_t)ps.nshare * kBins * ps.count;
         if (part + need > p->part_cap) part = 0;
@@ -573,22 +604,23 @@ GPUD_API int GPUD_CALL gpud_pilot_run(gpud_pilot *p, const gpud_pilot_job *jobs,
     int decided = 0, launches = 1;  // jobs decided; kernels
     for (size_t k = 0; k < p->passes.size(); ++k) {
         PilotPass ps = p->passes[k];
-        if (ps.each) {  // with the short windows of the next rates
+        bool table = ps.period <= kMaxTable, have = ps.period == p->tab_period;
+        if (ps.each)  // with the next rates of a station or two, or of short windows
             for (; k + 1 < p->passes.size() && p->passes[k + 1].each && p->passes[k + 1].part_off != 0; ++k) {
                 ps.count += p->passes[k + 1].count;
                 ps.nshare = std::max(ps.nshare, p->passes[k + 1].nshare);
+                have = have || p->passes[k + 1].period == p->tab_period;
             }
-            k_pilot_bins_each<<<dim3((unsigned)ps.nshare, (unsigned)ps.count), kPilotThreads, 0, s>>>(
-                p->d_jobs + ps.first, p->d_y, p->d_part);
-        }
-        const bool table = !ps.each && ps.period <= kMaxTable;
-        if (table && ps.period != p->tab_period) {  // the pass before has read the old one (stream order)
+        if (table && !have) {  // the pass before has read the old one (stream order)
             k_pilot_table<<<std::min(1024, (ps.period + 255) / 256), 256, 0, s>>>(ps.period, p->d_tab);
             launches++;
             p->tab_period = ps.period;
         }
-        if (!ps.each &&
-            launch_pilot_bins(ps, s, p->d_jobs, p->d_y, table ? p->d_tab : nullptr, p->d_part) != cudaSuccess)
+        if (ps.each)
+            k_pilot_bins_each<<<dim3((unsigned)ps.nshare, (unsigned)ps.count), kPilotThreads, 0, s>>>(
+                p->d_jobs + ps.first, p->d_y, p->d_tab, p->tab_period, p->d_part);
+        else if (launch_pilot_bins(ps, s, p->d_jobs, p->d_y, table ? p->d_tab : nullptr, p->d_part) !=
+                 cudaSuccess)
             return GPUD_E_CUDA;
         launches++;
         if (k + 1 < p->passes.size() && p->passes[k + 1].part_off != 0) continue;
